@@ -34,6 +34,7 @@ import os
 import statistics
 import subprocess
 import sys
+import tempfile
 import threading
 import time
 
@@ -325,8 +326,15 @@ class CpuSolves:
         if self.F is None:
             # the port has no construction of its own: the reference's factors equal the
             # library's bit for bit (tests/test_host.py), so the port uses those
-            import fiim_b200 as FB
-            self.F = FB.pdfiim_build(self.A, **PDFIIM_PARAMS)
+            # (built in a child process: this one loads no library of the project)
+            with tempfile.TemporaryDirectory() as d:
+                np.savez(os.path.join(d, "A.npz"), *self.A)
+                code = ("import sys, numpy as np; sys.path.insert(0, sys.argv[1]); import fiim_b200 as FB; "
+                        "z = np.load(sys.argv[2] + '/A.npz'); A = tuple(z['arr_%d' % k] for k in range(3)); "
+                        f"np.savez(sys.argv[2] + '/F.npz', **FB.pdfiim_build(A, **{PDFIIM_PARAMS!r}))")
+                subprocess.run([sys.executable, "-c", code, PKG, d], check=True)
+                with np.load(os.path.join(d, "F.npz")) as z:
+                    self.F = {k: z[k] for k in z.files}
         t0 = time.perf_counter()
         x, res, it, info = self.O.bicgstab("pdfiim", self.A, self.b, self.F, tol=1e-8, nmax=self.port_its)
         dt = time.perf_counter() - t0

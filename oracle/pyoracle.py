@@ -29,7 +29,7 @@ _libs: dict[str, C.CDLL] = {}
 def build(ref: bool = True) -> None:
     """Compile the restatement (always) and, when the reference tree exists, oracle/_ref."""
     targets = ["restatement"]
-    if ref and os.path.isdir(REFERENCE):
+    if ref and os.path.isdir(os.path.join(REFERENCE, "AFIIM", "src")):
         targets += ["ref", "REF=" + REFERENCE]
     subprocess.run(["make", "-s", "-C", HERE, *targets], check=True)
 
