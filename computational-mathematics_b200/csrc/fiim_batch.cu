@@ -97,21 +97,24 @@ struct BatchSolver : SolverBase {
     bool host_loop = false;          // FIIM_GRAPH=host: the host relaunches a one-iteration graph
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
+    template <bool SHARED, typename V, typename Epi>
+    cudaError_t spmv_dia(const BMat &B, const double *xx, const Epi &epi) {
+        const DiaView<V> view = dia_view<V>(B.M);
+        auto go = [&](auto kern) {
+            return launch_k(kern, grid_for(kern, kWarps, B.M.nsl), 0, stream, view, B.sflag, xx, epi, bs, partials);
+        };
+        if constexpr (sizeof(V) == 8) {
+            if (B.M.dsh == 64) return go(bt::k_bspmv_dia<V, 2, SHARED, Epi>);
+            return go(bt::k_bspmv_dia<V, 1, SHARED, Epi>);
+        } else {
+            return go(bt::k_bspmv_dia<V, sizeof(V) == 4 ? 2 : 4, SHARED, Epi>);
+        }
+    }
+
     template <typename V, typename Epi>
     cudaError_t spmv(const BMat &B, const V *vals, const double *xx, const Epi &epi) {
         if (B.M.dia) {   // its sliced-diagonal copy (values of V's width: 2 rows a lane for FP32)
-            const DiaView<V> view{B.M.drec, static_cast<const V *>(B.M.dvals), (int)B.M.n, B.M.nsl, B.M.drs};
-            if constexpr (sizeof(V) == 8) {
-                if (B.M.dsh == 64) {
-                    auto k2 = bt::k_bspmv_dia<V, 2, Epi>;
-                    return launch_k(k2, grid_for(k2, kWarps, B.M.nsl), 0, stream, view, B.sflag, xx, epi, bs, partials);
-                }
-                auto k1 = bt::k_bspmv_dia<V, 1, Epi>;
-                return launch_k(k1, grid_for(k1, kWarps, B.M.nsl), 0, stream, view, B.sflag, xx, epi, bs, partials);
-            } else {
-                auto kd = bt::k_bspmv_dia<V, sizeof(V) == 4 ? 2 : 4, Epi>;
-                return launch_k(kd, grid_for(kd, kWarps, B.M.nsl), 0, stream, view, B.sflag, xx, epi, bs, partials);
-            }
+            return B.M.dcls ? spmv_dia<true, V>(B, xx, epi) : spmv_dia<false, V>(B, xx, epi);
         }
         auto kern = bt::k_bspmv<kTile, V, Epi, false>;
         const int g = sgrid(kern, B.M.nblk);
@@ -145,13 +148,11 @@ struct BatchSolver : SolverBase {
         return launch_k(bt::k_bfinish<NR, true, Fin>, g, 0, stream, A.sys_blk, kWarps, nsys, partials, bs, fin);
     }
 
-    // The sliced-diagonal copy of B (fiim_internal.h, build_dia_structure) with slices inside
+    // The sliced-diagonal copy of B (fiim_internal.h, build_dia) with slices inside
     // the systems, its values `vals` (device, the stored width vbytes), its slice flags and the
     // systems' first slices; B keeps its CSR streams when the matrix does not allow it.
     int build_copy(BMat &B, int m, int vbytes, const void *vals) {
-        FIIM_TRY(build_dia_structure(B.M, stream, vbytes, &sys_rows));
-        if (!B.M.dia_mem) return FIIM_OK;
-        FIIM_TRY(place_dia(B.M, vals, stream));
+        FIIM_TRY(build_dia(B.M, stream, vbytes, vals, &sys_rows));
         if (!B.M.dia) return FIIM_OK;
         const size_t bf = Arena::need(sizeof(int) * std::max(B.M.nsl, 1)), bsl = Arena::need(sizeof(int) * (nsys + 1));
         char *mem = nullptr;

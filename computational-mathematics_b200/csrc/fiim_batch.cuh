@@ -383,7 +383,7 @@ k_bspmv(CsrView<V> M, const int *__restrict__ rb, const int *__restrict__ eb, co
 // the system's done flag), and each slice's reductions stored as one partial (lane 0, after
 // the warp's tree) for the per-system finish (qmul = 1). Factor values stored in FP32 or BF16
 // are widened to FP64 at the rounded product, as in k_bspmv.
-template <typename V, int R, typename Epi>
+template <typename V, int R, bool SHARED, typename Epi>
 static __global__ void __launch_bounds__(kThreads)
 k_bspmv_dia(DiaView<V> M, const int *__restrict__ sflag, const double *__restrict__ x, Epi epi, BState bs,
             double *__restrict__ partials) {
@@ -391,18 +391,33 @@ k_bspmv_dia(DiaView<V> M, const int *__restrict__ sflag, const double *__restric
     const int lane = (int)threadIdx.x & 31;
     const int nw = (int)gridDim.x * kWarps;
     int sl = (int)blockIdx.x * kWarps + ((int)threadIdx.x >> 5);
-    int rec = (sl < M.nsl && lane < M.rs) ? __ldg(M.rec + (long)sl * M.rs + lane) : 0;
+    auto load = [&](int s) {   // the record's lane, or the class
+        if (s >= M.nsl) return 0;
+        if constexpr (SHARED) return __ldg(M.cls + s);
+        else return lane < M.rs ? __ldg(M.rec + (long)s * M.rs + lane) : 0;
+    };
+    int rec = load(sl);
+    // a batch of one system has one segment and no position list
+    auto where = [&](int s) {
+        return M.pos ? __ldg(M.pos + s) : make_int2(s * 32 * R, min(32 * R, M.n - s * 32 * R));
+    };
+    int2 at = sl < M.nsl ? where(sl) : make_int2(0, 0);
     for (; sl < M.nsl; sl += nw) {
         const int nxt = sl + nw;
-        const int rec_next = (nxt < M.nsl && lane < M.rs) ? __ldg(M.rec + (long)nxt * M.rs + lane) : 0;
+        const int rec_next = load(nxt);
+        const int2 at_next = nxt < M.nsl ? where(nxt) : make_int2(0, 0);
         if (!(Epi::GATED && sflag[sl])) {   // uniform in the warp
             double red[Epi::NR];
 #pragma unroll
             for (int j = 0; j < Epi::NR; ++j) red[j] = 0.0;
-            dia_slice<V, double, R>(M, x, epi, rec, lane, [&](int row, double s, double opnd) {
+            auto emit = [&](int row, double s, double opnd) {
                 if constexpr (HasPre<Epi>::value) epi.emit_pre(row, s, opnd, red);
                 else epi.emit(row, s, red);
-            });
+            };
+            if constexpr (SHARED)
+                cls_slice<V, double, R>(M, x, epi, rec, at.x, at.y, lane,
+                                        [&](int, int row, double s, double opnd) { emit(row, s, opnd); });
+            else dia_slice<V, double, R>(M, x, epi, rec, at.x, at.y, lane, emit);
             if constexpr (Epi::REDUCES) {
 #pragma unroll
                 for (int j = 0; j < Epi::NR; ++j) red[j] = warp_sum(red[j]);
@@ -412,6 +427,7 @@ k_bspmv_dia(DiaView<V> M, const int *__restrict__ sflag, const double *__restric
             }
         }
         rec = rec_next;
+        at = at_next;
     }
     pdl_release();
 }

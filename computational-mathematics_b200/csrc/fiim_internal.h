@@ -74,12 +74,14 @@ struct DevCsr {
     // Sliced-diagonal copy (kFormDia; fiim_kernels.cuh, k_spmv_dia), in its own allocation.
     int dia = 0;                 // 1: built and current
     int nsl = 0;                 // slices of dsh rows
+    int dncls = 0;               // different slices: records and value blocks held
     int dsh = 0;                 // rows a slice: 32 R, R rows a lane (dia_rows_per_lane)
     int drs = 0;                 // ints per slice record (16 or 32): first diagonal, count, offsets
-    long ndiag = 0;              // diagonals over all slices (dsh slots each)
-    int *drec = nullptr;         // nsl records
-    int *dmap = nullptr;         // nnz: the slot of each entry
-    int *dbad = nullptr;         // device flag of the structure check and value placement
+    long ndiag = 0;              // diagonals over the blocks held (dsh slots each)
+    int *drec = nullptr;         // dncls records
+    int *dcls = nullptr;         // the record of each slice (null: its own)
+    int2 *dpos = nullptr;        // first row and rows of each slice (several segments only)
+    char *dstat = nullptr;       // device counters of the check (fiim_slices.cuh, Stats)
     void *dvals = nullptr;       // dsh * ndiag values of dvbytes bytes each (FP64, FP32 or BF16)
     int dvbytes = 0;
     void *dia_mem = nullptr;
@@ -138,31 +140,27 @@ int upload_csr(DevCsr &M, long nnz_cap, int n, const int *rp, const int *ci, con
 int set_tile(DevCsr &M, int tile, cudaStream_t s);
 // Builds the narrow column stream (cd, cb) of M's row blocks (eb) when every block allows it.
 int build_narrow(DevCsr &M, cudaStream_t s);
-// The sliced-diagonal copy of M (fiim_kernels.cuh, k_spmv_dia). build_dia_structure lays it
-// out (slice records, the slot of every entry; slices never straddle a boundary of
-// `segments`, ascending row starts from 0 to n, one segment when null) for values of vbytes
-// bytes (8, 4 or 2) when
-// M's rows are sorted by column, every slice (32 R rows, R = dia_rows_per_lane) has at most
-// kDiaMaxDiags diagonals and the copy moves fewer bytes than the CSR streams (M.dia_mem
-// stays null otherwise);
-// place_dia moves the nnz values `vals` (device, that width) into it and sets M.dia = 1,
-// unless an entry holds the padding pattern (then the copy is released). dia_fits tells
-// whether M's current columns (same row offsets) still sit in the laid-out slots.
-// build_dia / refresh_dia do this for the FP64 values M.v: refresh_dia, after new values (and
-// possibly new columns) with the same row offsets, re-places the values when the columns
-// still fit and rebuilds otherwise. release_dia frees the copy; dia_wanted is false under
-// FIIM_DIA=0 or FIIM_SPMV=rows / staged / warp.
+// The sliced-diagonal copy of M (fiim_kernels.cuh, k_spmv_dia; fiim_slices.cu). build_dia lays
+// it out for the nnz device values `vals` of vbytes bytes (8, 4 or 2) and sets M.dia = 1 when
+// M's rows are sorted by column, every slice (32 R rows, R = dia_rows_per_lane; slices never
+// straddle a boundary of `segments`, ascending row starts from 0 to n, one segment when null)
+// has at most kDiaMaxDiags diagonals, no entry holds the padding pattern and the copy moves
+// fewer bytes than the CSR streams; otherwise M keeps the CSR streams. Slices with the same
+// diagonals and values share one record and block (FIIM_DIA_SHARE=0: none do).
+// refresh_dia, after new FP64 values M.v (and possibly new columns) with the same row offsets,
+// keeps or re-places the values where the copy allows it and builds it again otherwise.
+// refresh_dia_async enqueues the same on `aux`, after the copies issued on `copy_s` before the
+// call, so it runs while later copies do; once `aux` is done, *h_bad (pinned) is 0 when the
+// copy holds the new values, else they are not to be used and refresh_dia decides again.
+// release_dia frees the copy; dia_wanted is false under FIIM_DIA=0 or FIIM_SPMV=rows / staged /
+// warp.
 bool dia_wanted();
 // Rows a lane of the sliced-diagonal copy for values of vbytes bytes: 2 for FP32, 4 for BF16;
-// for FP64 0, which lets build_dia_structure choose 1 or 2 by the matrix (FIIM_DIA_R=1 or 2
-// forces one).
+// for FP64 0, which lets build_dia choose 1 or 2 by the matrix (FIIM_DIA_R=1 or 2 forces one).
 int dia_rows_per_lane(int vbytes);
-
-int build_dia_structure(DevCsr &M, cudaStream_t s, int vbytes, const std::vector<int> *segments = nullptr);
-int place_dia(DevCsr &M, const void *vals, cudaStream_t s);
-int dia_fits(DevCsr &M, cudaStream_t s, bool *fits);
-int build_dia(DevCsr &M, cudaStream_t s);
+int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std::vector<int> *segments = nullptr);
 int refresh_dia(DevCsr &M, cudaStream_t s);
+int refresh_dia_async(DevCsr &M, cudaStream_t copy_s, cudaStream_t aux, cudaEvent_t done, int *h_bad);
 void release_dia(DevCsr &M);
 void expand_sym_upper(int n, const int *rp, const int *ci, const double *v, HostCsr &out);
 void transpose_upper(int n, const int *rp, const int *ci, const double *v, HostCsr &out);
@@ -217,6 +215,12 @@ template <typename K>
 int grid_for(K kernel, long units_per_block, long units) {
     const long need = std::max<long>(1, (units + units_per_block - 1) / units_per_block);
     return (int)std::min<long>(need, (long)occupancy(kernel) * num_sms());
+}
+
+// CTAs of k_spmv_dia with one row a lane (four per SM, at most one 32-row slice a warp when the
+// matrix is small): the grid whose summation tree the sliced forms share.
+inline int dia_grid(long n) {
+    return (int)std::min<long>((n + 32 * 8 - 1) / (32 * 8), 4L * num_sms());
 }
 
 

@@ -36,6 +36,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "fiim_internal.h"
+
 namespace fiim {
 
 constexpr int kThreads = 256;
@@ -122,6 +124,39 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 // ---------------------------------------------------------------- reduction tail
+// The last CTA: the sums of `count` partials, then op.finish. sm holds at least kWarps rows.
+template <int NR, class Op>
+__device__ __forceinline__ void reduce_partials(int count, const double *__restrict__ partials, double (*sm)[NR],
+                                                DState *st, const Op &op) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    __threadfence();
+    double acc[NR];
+#pragma unroll
+    for (int j = 0; j < NR; ++j) acc[j] = 0.0;
+    for (int k = threadIdx.x; k < count; k += kThreads)
+#pragma unroll
+        for (int j = 0; j < NR; ++j) acc[j] += __ldcg(partials + (size_t)k * NR + j);
+#pragma unroll
+    for (int j = 0; j < NR; ++j) acc[j] = warp_sum(acc[j]);
+    __syncthreads();
+    if (lane == 0)
+#pragma unroll
+        for (int j = 0; j < NR; ++j) sm[w][j] = acc[j];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double tot[NR];
+#pragma unroll
+        for (int j = 0; j < NR; ++j) {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < kWarps; ++k) s += sm[k][j];
+            tot[j] = s;
+        }
+        st->ticket = 0u;
+        op.finish(st, tot);
+    }
+}
+
 // Reduce NR per-thread values over the grid. Every block must call it (uniformly).
 // The last block calls op.finish(st, totals) from thread 0.
 template <int NR, class Op>
@@ -150,32 +185,47 @@ __device__ __forceinline__ void grid_reduce(double (&v)[NR], double *__restrict_
     }
     __syncthreads();
     if (!last) return;
-    __threadfence();
-    double acc[NR];
+    reduce_partials<NR>((int)gridDim.x, partials, sm, st, op);
+}
+
+// grid_reduce for a grid whose warps each stand for two warps of a virtual grid of vgrid CTAs
+// (warp g for the virtual warps 2 g and 2 g + 1, whose lanes' sums are v[0] and v[1]): the same
+// tree as grid_reduce over the virtual grid. CTA b writes the partials of virtual CTAs 2 b, 2 b + 1.
+template <int NR, class Op>
+__device__ __forceinline__ void grid_reduce_pairs(double (&v)[2][NR], int vgrid, double *__restrict__ partials,
+                                                  DState *st, const Op &op) {
+    __shared__ double sm[2 * kWarps][NR];
+    __shared__ int last;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
-    for (int j = 0; j < NR; ++j) acc[j] = 0.0;
-    for (int k = threadIdx.x; k < (int)gridDim.x; k += kThreads)
-#pragma unroll
-        for (int j = 0; j < NR; ++j) acc[j] += __ldcg(partials + (size_t)k * NR + j);
-#pragma unroll
-    for (int j = 0; j < NR; ++j) acc[j] = warp_sum(acc[j]);
-    __syncthreads();
-    if (lane == 0)
-#pragma unroll
-        for (int j = 0; j < NR; ++j) sm[w][j] = acc[j];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double tot[NR];
+    for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int j = 0; j < NR; ++j) {
-            double s = 0.0;
-#pragma unroll
-            for (int k = 0; k < kWarps; ++k) s += sm[k][j];
-            tot[j] = s;
+            v[h][j] = warp_sum(v[h][j]);
+            if (lane == 0) sm[2 * w + h][j] = v[h][j];
         }
-        st->ticket = 0u;
-        op.finish(st, tot);
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        const int vb = 2 * (int)blockIdx.x + (int)threadIdx.x;
+        if (vb < vgrid)
+#pragma unroll
+            for (int j = 0; j < NR; ++j) {
+                double s = 0.0;
+#pragma unroll
+                for (int k = 0; k < kWarps; ++k) s += sm[kWarps * threadIdx.x + k][j];
+                partials[(size_t)vb * NR + j] = s;
+            }
+        __threadfence();
     }
+    __syncwarp();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned t = atomicAdd(&st->ticket, 1u);
+        last = (t == gridDim.x - 1);
+    }
+    __syncthreads();
+    if (!last) return;
+    reduce_partials<NR>(vgrid, partials, sm, st, op);
 }
 
 // ---------------------------------------------------------------- scalar steps
@@ -201,6 +251,14 @@ struct FinInit {   // ro = ||r0||, m1 = ro^2, rc = ro (AFIIM/src/bicgstab.cpp:16
     static constexpr int NR = nr;                 \
     static constexpr bool REDUCES = reduces;      \
     static constexpr bool GATED = gated
+
+// An epilogue whose sums steer the iteration (r0, alpha, omega) declares STEERS: their summation
+// tree is the same in the sliced forms with and without shared blocks (k_spmv_cls), so a solve's
+// iterates do not depend on which of them serves A.
+template <typename E, typename = void>
+struct Steers : std::false_type {};
+template <typename E>
+struct Steers<E, std::void_t<typename E::STEERS>> : std::true_type {};
 
 template <typename E, typename = void>
 struct HasPre : std::false_type {};
@@ -234,6 +292,7 @@ struct EpiNorm {                   // y = M x, ||y||^2 -> st->pc2 (stagnation te
 };
 struct EpiAlpha {                  // v = A pc, alpha = m1 / (r0 . v)
     FIIM_EPI(1, true, true);
+    using STEERS = void;
     double *y;
     const double *__restrict__ r0;
     __device__ const double *pre_ptr() const { return r0; }
@@ -256,6 +315,7 @@ struct EpiAlpha {                  // v = A pc, alpha = m1 / (r0 . v)
 };
 struct EpiOmega {                  // t = A sc, omega = (t . s) / (t . t)
     FIIM_EPI(2, true, true);
+    using STEERS = void;
     double *y;
     const double *__restrict__ sv;
     __device__ const double *pre_ptr() const { return sv; }
@@ -276,6 +336,7 @@ struct EpiOmega {                  // t = A sc, omega = (t . s) / (t . t)
 // p = b + (-1) s; r0 = p; r = p; sum r0^2 -> ro, m1 = ro^2, rc = ro.
 struct EpiInit {
     FIIM_EPI(1, true, true);
+    using STEERS = void;
     const double *__restrict__ b;
     double *p, *r0, *r;
     __device__ void emit(long i, double s, double (&red)[NR]) const {
@@ -631,45 +692,61 @@ k_narrow_cols(const int *__restrict__ ci, const int *__restrict__ eb, int nblk, 
 // few diagonals (R rows a lane: 1 or 2 for FP64 values, 2 for FP32, 4 for BF16, so that a
 // lane's values of one diagonal are one load). Slices never straddle a segment boundary (the
 // systems of a batch; one segment for a single system), so a segment's last slice may hold
-// fewer rows. Slice s holds its rows' diagonals d = col - row, ascending; each diagonal stores
-// one value per row slot of the slice (v[32 R k + row - first row], k counted over all
-// slices). A row's own entries keep their storage order (rows are sorted by column), and a
-// slot the row has no entry in holds the padding pattern (kDiaPad, kDiaPad32, kDiaPad16: NaN
-// bit patterns no entry of the matrix holds, checked when the values are placed). Each slice
-// has a record of rs ints (16 or 32): its first diagonal k0, its count m (with kDiaClamp when
-// a slot's column falls outside the matrix), its m offsets, and in its last two ints its first
-// row and its row count; a warp reads it in one coalesced load. Bytes per entry: the value's
-// width and the padding, plus 2 or 4 per R rows for the records, against the width plus 2 or
-// 4 per entry and 4 per row for the CSR streams.
+// fewer rows. A slice holds its rows' diagonals d = col - row, ascending; each diagonal stores
+// one value per row slot of the slice, lane l's R values at v[32 R k + R l + j], k counted over
+// all blocks. Lane l owns the rows first + R l + j or, with shared blocks, first + l + 32 j.
+// A row's own entries keep their storage order (rows are sorted by column), and a slot the row
+// has no entry in holds the padding pattern (kDiaPad, kDiaPad32, kDiaPad16: NaN bit patterns no
+// entry of the matrix holds, checked when the values are placed). A slice's record has rs ints
+// (16 or 32): its block's first diagonal k0, its count m (with kDiaClamp when a slot's column
+// falls outside the matrix) and its m offsets; a warp reads it in one coalesced load. Slices
+// that agree in all of this share one record and block (SHARED: cls names a slice's record).
+// Bytes per entry: the value's width and the padding, plus 2 or 4 per R rows for the records,
+// against the width plus 2 or 4 per entry and 4 per row for the CSR streams; shared, 4 per
+// slice, and the blocks stay in L1.
 constexpr unsigned long long kDiaPad = 0xFFF7D1A6B00C5A1DULL;   // FP64 padding; FP32 and BF16 below
 constexpr unsigned kDiaPad32 = 0xFFD1A6B5u;
 constexpr unsigned short kDiaPad16 = 0xFFD1u;
-constexpr int kDiaRecHead = 2;     // record: k0, count | flags, offsets ..., first row, rows
-constexpr int kDiaMaxDiags = 32 - kDiaRecHead - 2;   // diagonals of one slice at most
+constexpr int kDiaRecHead = 4;     // record: k0, count | flags, quads, 0, offsets
+constexpr int kDiaMaxDiags = 32 - kDiaRecHead;   // diagonals of one slice at most
+constexpr int kDiaQuad = 4;        // shared blocks hold whole quads of diagonals
 constexpr int kDiaCountMask = 0xffff, kDiaClamp = 1 << 30;   // record[1]: count | clamp flag
 
 template <typename V = double>
 struct DiaView {
-    const int *__restrict__ rec;      // nsl records of rs ints: k0, m, first row, rows, offsets
+    const int *__restrict__ rec;      // records of rs ints: k0, m, offsets
     const V *__restrict__ v;          // 32 R values per diagonal
+    const int *__restrict__ cls;      // record of each slice (null: its own)
+    const int2 *__restrict__ pos;     // first row and rows of each slice (several segments only)
     int n, nsl, rs;
 };
 
-// A lane's R values of one diagonal (one load of R values, streamed) and the padding test;
-// BF16 is widened by a shift or a mask, so the padding keeps its pattern in the upper half.
-// R is 1 or 2 for FP64, 2 for FP32, 4 for BF16.
+template <typename V, class M>
+DiaView<V> dia_view(const M &m) {   // M: DevCsr
+    return DiaView<V>{m.drec, static_cast<const V *>(m.dvals), m.dcls, m.dpos, (int)m.n, m.nsl, m.drs};
+}
+
+// A lane's R values of one diagonal (one load of R values: streamed, or KEEP: cached, for shared
+// blocks) and the padding test; BF16 is widened by a shift or a mask, so the padding keeps its
+// pattern in the upper half. R is 1 or 2 for FP64, 2 for FP32, 4 for BF16.
+template <bool KEEP, typename P>
+__device__ __forceinline__ P ld_block(const P *p) {
+    if constexpr (KEEP) return __ldg(p);
+    else return __ldcs(p);
+}
 template <typename V, int R>
 struct DiaLoad;
 template <int R>
 struct DiaLoad<double, R> {   // the upper word decides: no entry of a served matrix shares it
     using E = double;
+    template <bool KEEP>
     static __device__ __forceinline__ void get(const double *p, double (&a)[R]) {
         if constexpr (R == 2) {
-            const double2 w = __ldcs(reinterpret_cast<const double2 *>(p));
+            const double2 w = ld_block<KEEP>(reinterpret_cast<const double2 *>(p));
             a[0] = w.x;
             a[1] = w.y;
         } else {
-            a[0] = ldm(p);
+            a[0] = ld_block<KEEP>(p);
         }
     }
     static __device__ __forceinline__ bool pad(double a) { return __double2hiint(a) == (int)(kDiaPad >> 32); }
@@ -677,8 +754,9 @@ struct DiaLoad<double, R> {   // the upper word decides: no entry of a served ma
 template <>
 struct DiaLoad<float, 2> {
     using E = float;
+    template <bool KEEP>
     static __device__ __forceinline__ void get(const float *p, float (&a)[2]) {
-        const float2 w = __ldcs(reinterpret_cast<const float2 *>(p));
+        const float2 w = ld_block<KEEP>(reinterpret_cast<const float2 *>(p));
         a[0] = w.x;
         a[1] = w.y;
     }
@@ -687,8 +765,9 @@ struct DiaLoad<float, 2> {
 template <>
 struct DiaLoad<__nv_bfloat16, 4> {
     using E = float;
+    template <bool KEEP>
     static __device__ __forceinline__ void get(const __nv_bfloat16 *p, float (&a)[4]) {
-        const uint2 w = __ldcs(reinterpret_cast<const uint2 *>(p));
+        const uint2 w = ld_block<KEEP>(reinterpret_cast<const uint2 *>(p));
         a[0] = __uint_as_float(w.x << 16);
         a[1] = __uint_as_float(w.x & 0xffff0000u);
         a[2] = __uint_as_float(w.y << 16);
@@ -743,13 +822,12 @@ __device__ __forceinline__ void dia_gather(const T *__restrict__ x, int row0, in
 // factors in the batched solve) at the product.
 template <typename V, typename T, int R, typename Epi, typename Emit>
 __device__ __forceinline__ void dia_slice(const DiaView<V> &M, const T *__restrict__ x, const Epi &epi, int rec,
-                                          int lane, Emit &&emit) {
+                                          int first, int rows, int lane, Emit &&emit) {
     using E = typename DiaLoad<V, R>::E;
     constexpr int SH = 32 * R;
     constexpr int C = 64 / (R * (int)sizeof(E));   // diagonals a chunk: 64 bytes of values a thread
     const unsigned full = 0xffffffffu;
     const int k0 = __shfl_sync(full, rec, 0), mf = __shfl_sync(full, rec, 1);
-    const int first = __shfl_sync(full, rec, M.rs - 2), rows = __shfl_sync(full, rec, M.rs - 1);
     const int m = mf & kDiaCountMask;
     const int row0 = first + R * lane;
     T opnd[R], s[R];
@@ -773,7 +851,7 @@ __device__ __forceinline__ void dia_slice(const DiaView<V> &M, const T *__restri
                     xv[u][j] = T(0);
                 }
                 if (k + u < m) {
-                    DiaLoad<V, R>::get(M.v + (long)(k0 + k + u) * SH + R * lane, a[u]);
+                    DiaLoad<V, R>::template get<false>(M.v + (long)(k0 + k + u) * SH + R * lane, a[u]);
                     dia_gather<CL, R>(x, row0, d, M.n, xv[u]);
                 }
             }
@@ -848,7 +926,7 @@ k_spmv_dia(DiaView<V> M, const T *__restrict__ x, Epi epi, DState *st, double *_
                         xv[u][j] = T(0);
                     }
                     if (k + u < m) {
-                        DiaLoad<V, R>::get(M.v + (long)(k0 + k + u) * SH + R * lane, a[u]);
+                        DiaLoad<V, R>::template get<false>(M.v + (long)(k0 + k + u) * SH + R * lane, a[u]);
                         dia_gather<CL, R>(x, row0, d, M.n, xv[u]);
                     }
                 }
@@ -872,6 +950,128 @@ k_spmv_dia(DiaView<V> M, const T *__restrict__ x, Epi epi, DState *st, double *_
     }
     pdl_release();
     if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red, partials, st, epi);
+}
+
+// One slice through a shared record (class c). Lane l owns the rows first + l + 32 j, so every
+// gather is one run of 32 consecutive x, whatever the diagonal's parity, and the R gathers of a
+// diagonal share one address. Every lane reads the record itself (one address a warp, from L1),
+// its diagonals four at a time; the block is padded to whole quads, so no chunk has a remainder.
+// Slices that need a test of the column or hold fewer than 32 R rows are flagged (kDiaClamp) and
+// take the general path, which reads x only for entries. Row sums as in dia_slice.
+template <typename V, typename T, int R, typename Epi, typename Emit>
+__device__ __forceinline__ void cls_slice(const DiaView<V> &M, const T *__restrict__ x, const Epi &epi, int c,
+                                          int first, int rows, int lane, Emit &&emit) {
+    using E = typename DiaLoad<V, R>::E;
+    constexpr int SH = 32 * R;
+    const int4 *rec = reinterpret_cast<const int4 *>(M.rec) + c * (M.rs >> 2);
+    const int4 h = __ldg(rec);
+    const int row0 = first + lane;
+    const V *vp = M.v + h.x * SH + R * lane;
+    const T *xp = x + row0;
+    T opnd[R], s[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) s[j] = opnd[j] = T(0);
+    if (!(h.y & kDiaClamp)) {
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            if constexpr (HasPre<Epi>::value) opnd[j] = epi.pre(row0 + 32 * j);
+        for (int q = h.z; q > 0; --q, vp += kDiaQuad * SH) {
+            const int4 d4 = __ldg(++rec);
+            const int d[kDiaQuad] = {d4.x, d4.y, d4.z, d4.w};
+            E a[kDiaQuad][R];
+            T xv[kDiaQuad][R];
+#pragma unroll
+            for (int u = 0; u < kDiaQuad; ++u) {
+                DiaLoad<V, R>::template get<true>(vp + u * SH, a[u]);
+#pragma unroll
+                for (int j = 0; j < R; ++j) xv[u][j] = ldx(xp + d[u] + 32 * j);
+            }
+#pragma unroll
+            for (int u = 0; u < kDiaQuad; ++u)
+#pragma unroll
+                for (int j = 0; j < R; ++j)
+                    if (!DiaLoad<V, R>::pad(a[u][j])) s[j] = dia_fma(s[j], T(a[u][j]), xv[u][j]);
+        }
+#pragma unroll
+        for (int j = 0; j < R; ++j) emit(j, row0 + 32 * j, s[j], opnd[j]);
+    } else {
+        const int *d = reinterpret_cast<const int *>(rec + 1);
+        for (int k = 0; k < (h.y & kDiaCountMask); ++k, vp += SH) {
+            const int dk = __ldg(d + k);
+            E a[R];
+            DiaLoad<V, R>::template get<true>(vp, a);
+#pragma unroll
+            for (int j = 0; j < R; ++j)
+                if (!DiaLoad<V, R>::pad(a[j])) s[j] = dia_fma(s[j], T(a[j]), ldx(xp + dk + 32 * j));
+        }
+#pragma unroll
+        for (int j = 0; j < R; ++j)
+            if (lane + 32 * j < rows) {
+                if constexpr (HasPre<Epi>::value) opnd[j] = epi.pre(row0 + 32 * j);
+                emit(j, row0 + 32 * j, s[j], opnd[j]);
+            }
+    }
+}
+
+// One warp per slice of a single system whose slices share records and blocks, grid-stride; the
+// next slice's class is loaded while the current one is summed. Bound by the L1's data path and
+// instruction issue (every load but the vectors' hits it). Two rows a lane halve the address
+// arithmetic: G 17.1 / 14.0 against 21.7 / 17.9 us with one, A 20.3 / 18.1 against 24.5 / 22.4,
+// and every slice reading its own block 26.2 / 23.7 and 34.2 / 30.5 (H 21.3 against 39.0), all at
+// 128^3 in the body's order, constant coefficients.
+// An epilogue that steers the iteration sums as k_spmv_dia with one row a lane would: vgrid is
+// that kernel's grid, and warp g takes the slices of its warps 2 g (rows first + lane) and
+// 2 g + 1 (rows first + 32 + lane), each with its own running sums.
+template <typename Epi, int R>
+constexpr bool kClsPairs = Steers<Epi>::value && R == 2;
+template <typename V, typename T, int R, typename Epi>
+static __global__ void __launch_bounds__(kThreads, kClsPairs<Epi, R> ? 2 : 4)
+k_spmv_cls(DiaView<V> M, const T *__restrict__ x, Epi epi, DState *st, double *__restrict__ partials, int vgrid) {
+    static_assert(std::is_same_v<typename DiaLoad<V, R>::E, T>, "one system: values load as T");
+    constexpr bool PAIRS = kClsPairs<Epi, R>;
+    constexpr int SH = 32 * R;
+    const int lane = (int)threadIdx.x & 31;
+    const int nw = PAIRS ? vgrid * kWarps / 2 : (int)gridDim.x * kWarps;
+    int sl = (int)blockIdx.x * kWarps + ((int)threadIdx.x >> 5);
+    if (sl >= nw) sl = M.nsl;   // PAIRS: past the virtual grid
+    int c = sl < M.nsl ? __ldg(M.cls + sl) : 0;
+    pdl_enter();   // the classes are constant: their first load may precede the wait
+    if (Epi::GATED && st != nullptr && st->done) return;
+    double red[PAIRS ? 2 : 1][Epi::NR];
+#pragma unroll
+    for (int h = 0; h < (PAIRS ? 2 : 1); ++h)
+#pragma unroll
+        for (int j = 0; j < Epi::NR; ++j) red[h][j] = 0.0;
+    for (; sl < M.nsl; sl += nw) {
+        const int next = sl + nw < M.nsl ? __ldg(M.cls + sl + nw) : 0;
+        cls_slice<V, T, R>(M, x, epi, c, sl * SH, M.n - sl * SH, lane, [&](int j, int row, T s, T opnd) {
+            double(&rd)[Epi::NR] = red[PAIRS ? j : 0];
+            if constexpr (HasPre<Epi>::value) epi.emit_pre(row, s, opnd, rd);
+            else epi.emit(row, s, rd);
+        });
+        c = next;
+    }
+    pdl_release();
+    if constexpr (PAIRS) grid_reduce_pairs<Epi::NR>(red, vgrid, partials, st, epi);
+    else if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red[0], partials, st, epi);
+}
+
+// Launches k_spmv_cls over the shared blocks of M (a DevCsr).
+template <typename V, typename T, class M, typename Epi>
+cudaError_t spmv_cls(cudaStream_t s, const M &m, const DiaView<V> &view, const T *x, const Epi &epi, DState *st,
+                     double *partials) {
+    auto go = [&](auto kern, bool pairs) {
+        const int vgrid = dia_grid(m.n);
+        const int grid = pairs ? (vgrid + 1) / 2 : grid_for(kern, kWarps, m.nsl);
+        return launch_k(kern, grid, 0, s, view, x, epi, st, partials, vgrid);
+    };
+    if constexpr (sizeof(V) == 8) {
+        if (m.dsh == 64) return go(k_spmv_cls<V, T, 2, Epi>, kClsPairs<Epi, 2>);
+        return go(k_spmv_cls<V, T, 1, Epi>, false);
+    } else {
+        constexpr int R = sizeof(V) == 4 ? 2 : 4;
+        return go(k_spmv_cls<V, T, R, Epi>, kClsPairs<Epi, R>);
+    }
 }
 
 // ---------------------------------------------------------------- CSR-vector SpMV
@@ -1070,51 +1270,11 @@ static __global__ void k_count_outside(int n, const int *__restrict__ rp, const 
     if (c) atomicAdd(count, c);
 }
 
-// Sliced-diagonal values, moved as bit patterns B of the value's width (8, 4 or 2 bytes):
-// every slot padding, then each entry e to its slot map[e]; *bad is set when an entry holds
-// the padding's pattern.
+// The padding test on an entry's bits B (8, 4 or 2 bytes): the upper word decides for FP64.
 template <typename B>
-static __global__ void __launch_bounds__(kThreads)
-k_dia_fill(long slots, B *__restrict__ dv, B pad) {
-    FIIM_FOR_ROWS(i, slots) { dv[i] = pad; }
-}
-template <typename B>
-__device__ __forceinline__ bool dia_is_pad(B o, B pad) {   // the kernel's test (upper word of FP64)
+__device__ __forceinline__ bool dia_is_pad(B o, B pad) {
     if constexpr (sizeof(B) == 8) return (o >> 32) == (pad >> 32);
     else return o == pad;
-}
-template <typename B>
-static __global__ void __launch_bounds__(kThreads)
-k_dia_scatter(long nnz, const B *__restrict__ v, const int *__restrict__ map, B *__restrict__ dv, B pad, int *bad) {
-    FIIM_FOR_ROWS(e, nnz) {
-        const B o = v[e];
-        if (dia_is_pad(o, pad)) atomicExch(bad, 1);
-        dv[map[e]] = o;
-    }
-}
-
-// Whether new column indices (with unchanged row offsets) still fit the slices' diagonals:
-// entry e of row i of a slice must sit in slot map[e] = sh k + i - first of a diagonal k of
-// the slice (k0 <= k < k0 + m) whose offset is ci[e] - i; sh = 32 R row slots a slice. *bad
-// is set otherwise. One warp per slice, its lanes over the slice's rows.
-static __global__ void __launch_bounds__(kThreads)
-k_dia_check(int nsl, const int *__restrict__ rp, const int *__restrict__ ci, const int *__restrict__ map,
-            const int *__restrict__ rec, int rs, int sh, int *bad) {
-    const int lane = (int)threadIdx.x & 31;
-    for (int sl = (int)blockIdx.x * kWarps + ((int)threadIdx.x >> 5); sl < nsl; sl += (int)gridDim.x * kWarps) {
-        const int *r = rec + (long)sl * rs;
-        const int k0 = r[0], m = r[1] & kDiaCountMask, first = r[rs - 2], rows = r[rs - 1];
-        for (int t = lane; t < rows; t += 32) {
-            const int i = first + t;
-            for (int e = rp[i]; e < rp[i + 1]; ++e) {
-                const int slot = map[e], k = slot / sh - k0;
-                if (slot % sh != t || k < 0 || k >= m || r[kDiaRecHead + k] != ci[e] - i) {
-                    atomicExch(bad, 1);
-                    break;
-                }
-            }
-        }
-    }
 }
 
 // Order-sensitive hash of a column stream: the wrapping sum over entries of the splitmix64

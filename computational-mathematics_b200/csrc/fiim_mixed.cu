@@ -62,9 +62,11 @@ cudaError_t spmv_f(const DevCsr &M, const V *vals, cudaStream_t s, const float *
                    DState *st, double *partials) {
     if (M.dia && M.dvbytes == (int)sizeof(V)) {   // the sliced-diagonal copy of these values
         if (M.dseg) return cudaErrorInvalidValue;     // k_spmv_dia takes slices of one segment
-        const DiaView<V> view{M.drec, static_cast<const V *>(M.dvals), (int)M.n, M.nsl, M.drs};
-        auto kern = k_spmv_dia<V, float, sizeof(V) == 4 ? 2 : 4, Epi>;   // the rows a lane it was built for
-        return launch_k(kern, grid_for(kern, kWarps, M.nsl), 0, s, view, x, epi, st, partials);
+        constexpr int R = sizeof(V) == 4 ? 2 : 4;     // the rows a lane it was built for
+        const DiaView<V> view = dia_view<V>(M);
+        auto go = [&](auto kern) { return launch_k(kern, grid_for(kern, kWarps, M.nsl), 0, s, view, x, epi, st, partials); };
+        if (M.dcls) return spmv_cls<V, float>(s, M, view, x, epi, st, partials);
+        return go(k_spmv_dia<V, float, R, Epi>);
     }
     switch (M.tile) {
         case 1024: return rows_f<1024>(s, M, vals, x, epi, st, partials);
@@ -371,12 +373,9 @@ struct MixedSolver : SolverBase {
         // Sliced-diagonal copies of the inner products' values where the matrices allow them
         // (A's FP64 residual product keeps the CSR streams).
         const int vb = bf16 ? 2 : 4;
-        FIIM_TRY(build_dia_structure(A, stream, 4));
-        FIIM_TRY(place_dia(A, A32, stream));
-        FIIM_TRY(build_dia_structure(G, stream, vb));
-        FIIM_TRY(place_dia(G, bf16 ? (const void *)G16 : (const void *)G32, stream));
-        FIIM_TRY(build_dia_structure(H, stream, vb));
-        FIIM_TRY(place_dia(H, bf16 ? (const void *)H16 : (const void *)H32, stream));
+        FIIM_TRY(build_dia(A, stream, 4, A32));
+        FIIM_TRY(build_dia(G, stream, vb, bf16 ? (const void *)G16 : (const void *)G32));
+        FIIM_TRY(build_dia(H, stream, vb, bf16 ? (const void *)H16 : (const void *)H32));
         return build_graph();
     }
 

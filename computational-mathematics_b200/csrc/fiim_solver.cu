@@ -200,13 +200,10 @@ template <typename Epi>
 static cudaError_t spmv_dia(cudaStream_t s, const DevCsr &M, const double *x, const Epi &epi, DState *st,
                             double *partials) {
     if (M.dseg) return cudaErrorInvalidValue;   // k_spmv_dia takes slices of one segment
-    const DiaView<double> view{M.drec, static_cast<const double *>(M.dvals), (int)M.n, M.nsl, M.drs};
-    if (M.dsh == 64) {
-        auto kern = k_spmv_dia<double, double, 2, Epi>;
-        return launch_k(kern, grid_for(kern, kWarps, M.nsl), 0, s, view, x, epi, st, partials);
-    }
-    auto kern = k_spmv_dia<double, double, 1, Epi>;
-    return launch_k(kern, grid_for(kern, kWarps, M.nsl), 0, s, view, x, epi, st, partials);
+    const DiaView<double> view = dia_view<double>(M);
+    auto go = [&](auto kern) { return launch_k(kern, grid_for(kern, kWarps, M.nsl), 0, s, view, x, epi, st, partials); };
+    if (M.dcls) return spmv_cls<double, double>(s, M, view, x, epi, st, partials);
+    return M.dsh == 64 ? go(k_spmv_dia<double, double, 2, Epi>) : go(k_spmv_dia<double, double, 1, Epi>);
 }
 
 // Solver SpMV: the sliced-diagonal copy where the matrix has one, else CSR-stream over the
@@ -273,273 +270,6 @@ int build_narrow(DevCsr &M, cudaStream_t s) {
         FIIM_CUDA(cudaStreamSynchronize(s));
         M.narrow = wide ? 0 : 1;
     }
-    return FIIM_OK;
-}
-
-void release_dia(DevCsr &M) {
-    if (M.dia_mem) cudaFree(M.dia_mem);
-    M.dia_mem = nullptr;
-    M.dia_bytes = 0;
-    M.drec = M.dmap = M.dbad = nullptr;
-    M.dvals = nullptr;
-    M.dvbytes = 0;
-    M.dsh = 0;
-    M.dseg = false;
-    M.dia = 0;
-    M.nsl = 0;
-    M.drs = 0;
-    M.ndiag = 0;
-}
-
-bool dia_wanted() {
-    // FIIM_SPMV=rows / staged / warp keep a CSR-stream form; FIIM_DIA=0 never builds the copy.
-    const char *force = std::getenv("FIIM_SPMV"), *off_env = std::getenv("FIIM_DIA");
-    return !((force && std::strcmp(force, "dia") != 0) || (off_env && std::strcmp(off_env, "0") == 0));
-}
-
-template <typename B>
-static int place_bits(DevCsr &M, const void *vals, B pad, cudaStream_t s) {
-    const long slots = (long)M.dsh * M.ndiag;
-    B *dv = static_cast<B *>(M.dvals);
-    k_dia_fill<B><<<stream_grid(k_dia_fill<B>, slots), kThreads, 0, s>>>(slots, dv, pad);
-    FIIM_CUDA(cudaGetLastError());
-    k_dia_scatter<B><<<stream_grid(k_dia_scatter<B>, M.nnz), kThreads, 0, s>>>(M.nnz, static_cast<const B *>(vals),
-                                                                               M.dmap, dv, pad, M.dbad);
-    FIIM_CUDA(cudaGetLastError());
-    return FIIM_OK;
-}
-
-int place_dia(DevCsr &M, const void *vals, cudaStream_t s) {
-    if (!M.dia_mem) return FIIM_OK;
-    FIIM_CUDA(cudaMemsetAsync(M.dbad, 0, sizeof(int), s));
-    if (M.dvbytes == 8) FIIM_TRY(place_bits<unsigned long long>(M, vals, kDiaPad, s));
-    else if (M.dvbytes == 4) FIIM_TRY(place_bits<unsigned>(M, vals, kDiaPad32, s));
-    else FIIM_TRY(place_bits<unsigned short>(M, vals, kDiaPad16, s));
-    int bad = 0;
-    FIIM_CUDA(cudaMemcpyAsync(&bad, M.dbad, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FIIM_CUDA(cudaStreamSynchronize(s));
-    if (bad) release_dia(M);   // an entry holds the padding pattern: the CSR streams serve
-    else M.dia = 1;
-    return FIIM_OK;
-}
-
-static int col_hash(DevCsr &M, cudaStream_t s, unsigned long long *h) {
-    *h = 0;
-    if (M.nnz <= 0 || !M.dhash) return FIIM_OK;
-    FIIM_CUDA(cudaMemsetAsync(M.dhash, 0, sizeof(unsigned long long), s));
-    k_col_hash<<<stream_grid(k_col_hash, M.nnz), kThreads, 0, s>>>(M.nnz, M.ci, M.dhash);
-    FIIM_CUDA(cudaGetLastError());
-    FIIM_CUDA(cudaMemcpyAsync(h, M.dhash, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    FIIM_CUDA(cudaStreamSynchronize(s));
-    return FIIM_OK;
-}
-
-int dia_rows_per_lane(int vbytes) {
-    if (vbytes == 8) {
-        const char *e = std::getenv("FIIM_DIA_R");
-        return (e && (e[0] == '1' || e[0] == '2') && e[1] == 0) ? e[0] - '0' : 0;   // 0: by the matrix
-    }
-    return vbytes == 4 ? 2 : 4;
-}
-
-int build_dia_structure(DevCsr &M, cudaStream_t s, int vbytes, const std::vector<int> *segments) {
-    release_dia(M);
-    M.dia_tried = false;
-    M.hseg_sl.clear();
-    if (!dia_wanted()) return FIIM_OK;
-    const int n = (int)M.n;
-    const long nnz = M.nnz;
-    if (n <= 0 || nnz <= 0 || (long)M.hrp.size() != (long)n + 1) return FIIM_OK;
-    const std::vector<int> whole = {0, n};
-    const std::vector<int> &seg = segments ? *segments : whole;
-    if (seg.size() < 2 || seg.front() != 0 || seg.back() != n) return set_error(FIIM_EARG, "segments must cover the rows");
-    FIIM_TRY(col_hash(M, s, &M.dia_cols));
-    M.dia_tried = true;
-    std::vector<int> ci(nnz);
-    FIIM_CUDA(cudaMemcpyAsync(ci.data(), M.ci, sizeof(int) * nnz, cudaMemcpyDeviceToHost, s));
-    FIIM_CUDA(cudaStreamSynchronize(s));
-    const int *rp = M.hrp.data();
-    // Slices of up to sh rows, never straddling a segment: first row, rows, and each segment's
-    // first slice.
-    int sh = 0, nsl = 0;
-    std::vector<int> first, rows, seg_sl;
-    auto slices = [&](int R) {
-        sh = 32 * R;
-        first.clear();
-        rows.clear();
-        seg_sl.assign(1, 0);
-        for (size_t q = 0; q + 1 < seg.size(); ++q) {
-            for (int r = seg[q]; r < seg[q + 1]; r += sh) {
-                first.push_back(r);
-                rows.push_back(std::min(sh, seg[q + 1] - r));
-            }
-            seg_sl.push_back((int)first.size());
-        }
-        nsl = (int)first.size();
-    };
-    // The diagonals of a slice: its entries' col - row, sorted and distinct.
-    auto diagonals = [&](int sl, std::vector<int> &d, int &unsorted) {
-        d.clear();
-        const int r0 = first[sl], r1 = r0 + rows[sl];
-        for (int i = r0; i < r1; ++i)
-            for (int e = rp[i]; e < rp[i + 1]; ++e) {
-                if (e > rp[i] && ci[e] <= ci[e - 1]) unsorted = 1;
-                d.push_back(ci[e] - i);
-            }
-        std::sort(d.begin(), d.end());
-        d.erase(std::unique(d.begin(), d.end()), d.end());
-    };
-    // Diagonals per slice for R rows a lane (sp[sl + 1]); false when a row is unsorted or a
-    // slice has more than kDiaMaxDiags.
-    std::vector<int> sp;
-    auto count = [&](int R) -> bool {
-        slices(R);
-        sp.assign(nsl + 1, 0);
-        std::atomic<int> fail{0};   // a failed slice ends the analysis (random matrices fail at once)
-#pragma omp parallel
-        {
-            std::vector<int> d;
-#pragma omp for schedule(dynamic, 256)
-            for (int sl = 0; sl < nsl; ++sl) {
-                if (fail.load(std::memory_order_relaxed)) continue;
-                int bad = 0;
-                diagonals(sl, d, bad);
-                sp[sl + 1] = (int)d.size();
-                if (bad || (int)d.size() > kDiaMaxDiags) fail.store(1, std::memory_order_relaxed);
-            }
-        }
-        return !fail.load();
-    };
-    // FP64 takes two rows a lane when its 32-row slices average more diagonals than one chunk
-    // of the kernel holds (H at 128^3: 11 diagonals, 32.9 against 41.6 us a product; A and G,
-    // 7 diagonals, were slower with two).
-    int R = dia_rows_per_lane(vbytes);
-    if (R == 0) {
-        if (!count(1)) return FIIM_OK;
-        long nd1 = 0;
-        for (int sl = 0; sl < nsl; ++sl) nd1 += sp[sl + 1];
-        R = 1;
-        if (nd1 > 8L * nsl) {
-            if (count(2)) R = 2;
-            else if (!count(1)) return FIIM_OK;
-        }
-    } else if (!count(R)) {
-        return FIIM_OK;
-    }
-    int most = 0;
-    for (int sl = 0; sl < nsl; ++sl) {
-        most = std::max(most, sp[sl + 1]);
-        sp[sl + 1] += sp[sl];
-    }
-    const long ndiag = sp[nsl];
-    const int rs = most <= 16 - kDiaRecHead - 2 ? 16 : 32;
-    // Kept only when it moves fewer bytes than the CSR streams it replaces.
-    const double dia_bytes = (double)vbytes * sh * ndiag + 4.0 * rs * nsl;
-    const double csr_bytes_now = (double)nnz * (vbytes + (M.narrow ? 2 : 4)) + 4.0 * (n + 1);
-    if (!(dia_bytes < csr_bytes_now) || (long)sh * ndiag >= (1L << 31)) return FIIM_OK;
-    std::vector<int> rec((size_t)nsl * rs, 0), map(nnz);
-#pragma omp parallel
-    {
-        std::vector<int> d;
-        int unused = 0;
-#pragma omp for schedule(dynamic, 256)
-        for (int sl = 0; sl < nsl; ++sl) {
-            diagonals(sl, d, unused);
-            int *r = rec.data() + (size_t)sl * rs;
-            const int r0 = first[sl], r1 = r0 + rows[sl];
-            // Every slot of the slice (rows r0 .. r0 + sh - 1, padding included) gathers a column
-            // r + d: the slice is flagged when one of them falls outside [0, n).
-            const bool outside = !d.empty() && ((long)r0 + d.front() < 0 || (long)r0 + sh - 1 + d.back() > n - 1);
-            r[0] = sp[sl];
-            r[1] = (int)d.size() | (outside ? kDiaClamp : 0);
-            r[rs - 2] = r0;
-            r[rs - 1] = rows[sl];
-            std::copy(d.begin(), d.end(), r + kDiaRecHead);
-            for (int i = r0; i < r1; ++i)
-                for (int e = rp[i]; e < rp[i + 1]; ++e) {
-                    const int k = (int)(std::lower_bound(d.begin(), d.end(), ci[e] - i) - d.begin());
-                    map[e] = sh * (sp[sl] + k) + (i - r0);
-                }
-        }
-    }
-    const size_t b_rec = Arena::need(sizeof(int) * rec.size()), b_map = Arena::need(sizeof(int) * nnz),
-                 b_bad = Arena::need(sizeof(int)), b_v = Arena::need((size_t)vbytes * sh * ndiag);
-    char *mem = nullptr;
-    if (cudaMalloc(&mem, b_rec + b_map + b_bad + b_v) != cudaSuccess) {
-        cudaGetLastError();
-        return FIIM_OK;   // no room for the copy: the CSR streams serve
-    }
-    M.dia_mem = mem;
-    M.dia_bytes = b_rec + b_map + b_bad + b_v;
-    M.drec = reinterpret_cast<int *>(mem);
-    M.dmap = reinterpret_cast<int *>(mem + b_rec);
-    M.dbad = reinterpret_cast<int *>(mem + b_rec + b_map);
-    M.dvals = mem + b_rec + b_map + b_bad;
-    M.dvbytes = vbytes;
-    M.dsh = sh;
-    M.nsl = nsl;
-    M.drs = rs;
-    M.ndiag = ndiag;
-    M.hseg_sl = seg_sl;
-    M.dseg = seg.size() > 2;
-    FIIM_CUDA(cudaMemcpyAsync(M.drec, rec.data(), sizeof(int) * rec.size(), cudaMemcpyHostToDevice, s));
-    FIIM_CUDA(cudaMemcpyAsync(M.dmap, map.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice, s));
-    FIIM_CUDA(cudaStreamSynchronize(s));   // before the host arrays go
-    return FIIM_OK;
-}
-
-int dia_fits(DevCsr &M, cudaStream_t s, bool *fits) {
-    *fits = false;
-    if (!M.dia_mem) return FIIM_OK;
-    FIIM_CUDA(cudaMemsetAsync(M.dbad, 0, sizeof(int), s));
-    const int g = (int)std::min<long>((M.nsl + kWarps - 1) / kWarps, 16L * num_sms());
-    k_dia_check<<<std::max(g, 1), kThreads, 0, s>>>(M.nsl, M.rp, M.ci, M.dmap, M.drec, M.drs, M.dsh, M.dbad);
-    FIIM_CUDA(cudaGetLastError());
-    int bad = 0;
-    FIIM_CUDA(cudaMemcpyAsync(&bad, M.dbad, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FIIM_CUDA(cudaStreamSynchronize(s));
-    *fits = !bad;
-    return FIIM_OK;
-}
-
-int build_dia(DevCsr &M, cudaStream_t s) {
-    FIIM_TRY(build_dia_structure(M, s, 8));
-    return place_dia(M, M.v, s);
-}
-
-int refresh_dia(DevCsr &M, cudaStream_t s) {
-    if (!dia_wanted()) return FIIM_OK;
-    if (!M.dia) {   // not built for the previous columns: decide again only if they changed
-        unsigned long long h = 0;
-        FIIM_TRY(col_hash(M, s, &h));
-        if (M.dia_tried && h == M.dia_cols) return FIIM_OK;
-        return build_dia(M, s);
-    }
-    bool fits = false;
-    FIIM_TRY(dia_fits(M, s, &fits));
-    if (!fits) return build_dia(M, s);
-    return place_dia(M, M.v, s);
-}
-
-// refresh_dia for a copy whose row offsets did not change, enqueued on `aux` once the copies
-// of M's columns and values (issued on `copy_s` before this call) are done, so it runs while
-// later copies do. The columns fit only when they equal those the copy was built for (the
-// check holds each entry to its slot), so the padding slots stay as they were and need no
-// fill; the check and the value scatter share M.dbad, which lands in *h_bad (pinned). 0 there
-// after `aux` synchronizes: the copy holds the new values. Otherwise the values in the copy
-// are not to be used, and refresh_dia decides again.
-static int refresh_dia_async(DevCsr &M, cudaStream_t copy_s, cudaStream_t aux, cudaEvent_t done, int *h_bad) {
-    FIIM_CUDA(cudaEventRecord(done, copy_s));
-    FIIM_CUDA(cudaStreamWaitEvent(aux, done, 0));
-    FIIM_CUDA(cudaMemsetAsync(M.dbad, 0, sizeof(int), aux));
-    const int g = (int)std::min<long>((M.nsl + kWarps - 1) / kWarps, 16L * num_sms());
-    k_dia_check<<<std::max(g, 1), kThreads, 0, aux>>>(M.nsl, M.rp, M.ci, M.dmap, M.drec, M.drs, M.dsh, M.dbad);
-    FIIM_CUDA(cudaGetLastError());
-    using B = unsigned long long;
-    k_dia_scatter<B><<<stream_grid(k_dia_scatter<B>, M.nnz), kThreads, 0, aux>>>(
-        M.nnz, reinterpret_cast<const B *>(M.v), M.dmap, static_cast<B *>(M.dvals), kDiaPad, M.dbad);
-    FIIM_CUDA(cudaGetLastError());
-    FIIM_CUDA(cudaMemcpyAsync(h_bad, M.dbad, sizeof(int), cudaMemcpyDeviceToHost, aux));
     return FIIM_OK;
 }
 
@@ -1161,7 +891,7 @@ int Solver::create(int n_, const int *Ai, const int *Aj, const double *Av, const
                 FIIM_TRY(set_tile(M, default_tile(M), stream));
             }
         }
-        FIIM_TRY(build_dia(M, stream));   // serves the products where the matrix allows it
+        FIIM_TRY(build_dia(M, stream, 8, M.v));   // serves the products where the matrix allows it
     }
     {
         // FIIM_PERSIST=1: systems of at most kPersistMaxN rows solve as one cooperative launch.
@@ -1262,7 +992,7 @@ int Solver::reload(const int *Ai, const int *Aj, const double *Av, const int *Gi
         // Everything of the sliced-diagonal copy that a captured launch holds: a rebuilt copy
         // may reuse the freed allocation's address with another layout inside it.
         auto dia_args = [](const DevCsr &D) {
-            return std::make_tuple(D.dia, D.drec, D.dvals, D.nsl, D.drs, D.dsh);
+            return std::make_tuple(D.dia, D.drec, D.dvals, D.dcls, D.nsl, D.drs, D.dsh);
         };
         const auto was_dia = dia_args(M);
         if (M.rows_same && M.nblk > 0) {
@@ -1273,7 +1003,7 @@ int Solver::reload(const int *Ai, const int *Aj, const double *Av, const int *Gi
             }
         } else {
             FIIM_TRY(set_tile(M, M.tile, stream));
-            FIIM_TRY(build_dia(M, stream));
+            FIIM_TRY(build_dia(M, stream, 8, M.v));
         }
         regraph |= (M.nblk != old) || (M.narrow != was_narrow) || (dia_args(M) != was_dia);
     }

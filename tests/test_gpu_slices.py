@@ -1,0 +1,99 @@
+"""The sliced forms of the solver's matrices: every way a matrix can be laid out gives the
+CSR streams' products bit for bit (rows are summed in storage order in all of them), at sizes
+around the slices' edges, with shared and with own blocks, and for vectors with infinities
+and NaN, which must reach only the rows that have an entry there."""
+import numpy as np
+import pytest
+
+import fiim_b200 as FB
+import pyoracle as O
+from test_gpu_solve import identity_factors
+
+pytestmark = pytest.mark.gpu
+
+
+def banded(n, offsets, value, drop=0.0, seed=0):
+    """CSR with the diagonals `offsets`, entry value(row, offset), a share `drop` of the off-diagonal
+    entries left out at random."""
+    rng = np.random.default_rng(seed)
+    rows = np.repeat(np.arange(n), len(offsets))
+    d = np.tile(np.asarray(sorted(offsets)), n)
+    keep = (rows + d >= 0) & (rows + d < n) & ((d == 0) | (rng.random(len(d)) >= drop))
+    rows, d = rows[keep], d[keep]
+    rp = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=n))])
+    return rp.astype(np.int32), (rows + d).astype(np.int32), value(rows, d)
+
+
+def product(A, u, monkeypatch, **env):
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    n = len(A[0]) - 1
+    with FB.Solver(A, identity_factors(n)) as S:
+        y = S.apply(u, np.zeros(n), op="A")
+        form = S.spmv_shape(0)[1]
+    for k in env:
+        monkeypatch.delenv(k)
+    return y, form
+
+
+def same(a, b):
+    return np.array_equal(a, b, equal_nan=True)
+
+
+KINDS = {
+    # the same values in every row: all inner slices are one class
+    "constant": lambda i, d: np.where(d == 0, 7.5, -1.0 - 0.25 * (d > 0)),
+    # every slice differs
+    "varying": lambda i, d: np.where(d == 0, 7.5, -1.0) + 1e-3 * np.sin(i * 1.7 + d),
+    # two materials: a few hundred rows each
+    "layers": lambda i, d: np.where(d == 0, 7.5, -1.0) * (1.0 + (i // 300) % 2),
+}
+
+
+@pytest.mark.parametrize("kind", sorted(KINDS))
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 63, 64, 65, 127, 129, 1000, 4097])
+def test_banded_products(monkeypatch, kind, n):
+    offsets = [o for o in (-100, -33, -8, -1, 0, 1, 8, 32, 101) if abs(o) < n]
+    A = banded(n, offsets, KINDS[kind])
+    u = np.random.default_rng(n).standard_normal(n)
+    ref = O.csr_mv(*A, u)
+    for env in ({}, {"FIIM_DIA_SHARE": "0"}, {"FIIM_DIA_R": "1"}, {"FIIM_DIA_R": "2"}, {"FIIM_DIA": "0"}):
+        y, form = product(A, u, monkeypatch, **env)
+        assert same(y, ref), (env, form)
+
+
+@pytest.mark.parametrize("kind", sorted(KINDS))
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_nonfinite_vector_entries(monkeypatch, kind, bad):
+    """An infinity or NaN in the vector reaches exactly the rows with an entry in its column,
+    whatever the padding of the slices around it."""
+    n = 2000
+    A = banded(n, (-45, -1, 0, 1, 44), KINDS[kind], drop=0.1, seed=3)
+    u = np.random.default_rng(1).standard_normal(n)
+    u[[0, 31, 32, 700, n - 1]] = bad
+    ref = O.csr_mv(*A, u)
+    assert np.isfinite(ref).sum() > n - 40
+    for env in ({}, {"FIIM_DIA_SHARE": "0"}, {"FIIM_DIA": "0"}):
+        y, form = product(A, u, monkeypatch, **env)
+        assert same(y, ref), (env, form)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "bf16"])
+def test_batch_with_and_without_shared_blocks(monkeypatch, precision):
+    """A batch's solves with shared blocks and with every slice's own: the products are the same
+    bits and the per-slice partial sums are grouped alike or by rows of the same slice, so the
+    runs agree system by system to rounding, as do their iteration counts."""
+    systems, bs = [], []
+    for k, side in enumerate((9, 16, 33, 40)):
+        A = FB.gen_convdiff2d(side, 1.0 + k, 0.3 * k, 0.5)
+        systems.append((A, FB.pdfiim_build(A, 0.05, 2, 2, 1)))
+        bs.append(FB.rand_normal(side * side, 40 + k))
+    b, out = np.concatenate(bs), {}
+    for share in ("1", "0"):
+        monkeypatch.setenv("FIIM_DIA_SHARE", share)
+        with FB.BatchSolver(systems, variant="pdfiim", precision=precision) as S:
+            x = np.zeros(len(b))
+            out[share] = (S.solve(b, x, tol=1e-10, nmax=500), x)
+    assert np.array_equal(out["1"][0]["info"], out["0"][0]["info"]) and not out["1"][0]["info"].any()
+    assert np.all(np.abs(out["1"][0]["iter"] - out["0"][0]["iter"]) <= 2)
+    assert np.linalg.norm(out["1"][1] - out["0"][1]) <= 1e-7 * np.linalg.norm(out["0"][1])
