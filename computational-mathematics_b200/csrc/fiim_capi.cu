@@ -282,7 +282,7 @@ int fiim_solver_spmv_shape(fiim_solver_t h, int which, int *tile, int *form) {
     const fiim::DevCsr *m[] = {&s->A, &s->G, &s->H, &s->L, &s->U};
     if (which < 0 || which > 4) return fiim::set_error(FIIM_EARG, "which in 0..4 (A, G, H, L, U)");
     *tile = m[which]->tile;
-    *form = m[which]->dia ? fiim::kFormDia : m[which]->form;
+    *form = m[which]->dia ? fiim::kFormDia : m[which]->pack ? fiim::kFormPack : m[which]->form;
     return FIIM_OK;
 }
 
@@ -336,6 +336,7 @@ double fiim_solver_matrix_bytes(fiim_solver_t h, int which) {
     const fiim::DevCsr *m[] = {&s->A, &s->G, &s->H, &s->L, &s->U};
     const fiim::DevCsr &M = *m[which];
     if (M.dia) return (double)M.dsh * M.dvbytes * (double)M.ndiag + 4.0 * M.drs * M.dncls + (M.dcls ? 4.0 * M.nsl : 0.0);
+    if (M.pack) return 8.0 * (double)M.nnz + 8.0 * (double)M.ndiag + 16.0 * M.nsl;
     return (double)M.nnz * (8 + (M.narrow ? 2 : 4)) + 4.0 * (M.n + 1) + (M.narrow ? 4.0 * M.nblk : 0.0) +
            8.0 * (M.nblk + 1);
 }

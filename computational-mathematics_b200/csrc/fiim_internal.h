@@ -50,8 +50,8 @@ struct Arena {
 // Forms of the solver's SpMV. All give the same bits. The CSR-stream forms differ in how a
 // row block's streams reach shared memory: through registers, pipelined by one block
 // (kFormRows, fiim_kernels.cuh), by bulk copies into two buffers (kFormBulk, fiim_pipe.cuh),
-// or per warp (kFormWarp); kFormDia reads the sliced-diagonal copy of the values instead.
-constexpr int kFormRows = 0, kFormBulk = 1, kFormWarp = 2, kFormDia = 3;
+// or per warp (kFormWarp); kFormDia and kFormPack read a sliced copy of the values instead.
+constexpr int kFormRows = 0, kFormBulk = 1, kFormWarp = 2, kFormDia = 3, kFormPack = 4;
 
 // A CSR matrix resident on the device. v holds FP64 values; v32 / v16 are optional
 // FP32 / BF16 copies for the mixed-precision inner solve.
@@ -86,6 +86,11 @@ struct DevCsr {
     int dvbytes = 0;
     void *dia_mem = nullptr;
     size_t dia_bytes = 0;        // size of that allocation
+    // Packed slices (kFormPack; fiim_kernels.cuh, k_spmv_pack), in the same allocation with dvals:
+    // nsl slices of 32 rows.
+    int pack = 0;                // 1: built and current (then dia is 0)
+    int4 *khdr = nullptr;        // per slice: first record, records, first value
+    int2 *krec = nullptr;        // offset and row mask of each slice's diagonals (ndiag of them)
     bool dia_tried = false;      // the copy was considered for the columns hashed in dia_cols
     unsigned long long dia_cols = 0;
     unsigned long long *dhash = nullptr;   // device scratch of the column hash (in the arena)

@@ -1074,6 +1074,128 @@ cudaError_t spmv_cls(cudaStream_t s, const M &m, const DiaView<V> &view, const T
     }
 }
 
+// ---------------------------------------------------------------- packed-slice SpMV
+// For sorted rows whose slices share diagonals too loosely for the sliced-diagonal copy (factors
+// filtered by size: at a random coefficient field, a 32-row slice of H has 19 diagonals for 10.5
+// entries a row, and padding them would read more than the CSR streams). A slice of 32 rows
+// keeps, per diagonal, its offset d and a 32-bit mask of the rows that have it, and its values
+// packed by diagonal, then row: no padding and no column stream. 8 bytes per entry, plus 8 per
+// diagonal and 16 per slice (5 per row at that H), against 10 or 12 per entry and 4 per row for
+// the CSR streams.
+struct PackView {
+    const int4 *__restrict__ hdr;     // per slice: first record, records, first value, 2 values + edge
+    const int2 *__restrict__ rec;     // d, mask
+    const double *__restrict__ v;
+    int n, nsl;
+};
+constexpr int kPackMax = 64;          // diagonals of one slice at most
+constexpr int kPackChunk = 4;         // diagonals whose loads are issued ahead of their sums
+
+// One warp per slice, grid-stride, lane l owning row l. While a slice is summed, the next one's
+// records are loaded and its values brought into L2, and the header after it is loaded. Lane k
+// works out where diagonal k's values start and leaves that with its record in shared memory; a
+// diagonal's value of a row is at that start plus the rows before it in the mask, so both its
+// loads are one run, and a chunk's loads are issued before its sums. A slice with a slot whose
+// gather would leave the matrix (edge) loads for its entries only. Rows are summed in storage
+// order, products and sums rounded apart, as in every other form.
+// Bound by the L1's data path (62 % busy) and the loads' latency at 32 warps an SM. At 1.9 M
+// rows with random coefficients, in the body's order: H 57.0 / 55.6 against 64.1 / 62.7 us with
+// the CSR streams, G 38.0 / 35.0 against 40.6 / 36.8; at 152,000 rows H 8.1 / 6.5 against 10.4 /
+// 7.8, G 7.0 / 4.6 against 7.8 / 5.7. Without the prefetch H took 64.7, with the records
+// broadcast by shuffles 66.0, six or eight diagonals a chunk ran H at 60 - 62.
+template <typename Epi>
+static __global__ void __launch_bounds__(kThreads, 4)
+k_spmv_pack(PackView M, const double *__restrict__ x, Epi epi, DState *st, double *__restrict__ partials) {
+    const unsigned full = 0xffffffffu;
+    const int lane = (int)threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u, mine = 1u << lane;
+    const int nw = (int)gridDim.x * kWarps;
+    // a warp's records of the current slice: offset, mask, where its values start and end; a chunk
+    // may read past the 32nd when it does not divide 32
+    __shared__ int4 meta_all[kWarps][32 + kPackChunk];
+    int4 *meta = meta_all[threadIdx.x >> 5];
+    if (lane < kPackChunk) meta[32 + lane] = make_int4(0, 0, 0, 0);
+    int sl = (int)blockIdx.x * kWarps + ((int)threadIdx.x >> 5);
+    const int4 none = make_int4(0, 0, 0, 0);
+    auto records = [&](const int4 &h, int k) { return k + lane < h.y ? __ldcs(M.rec + h.x + k + lane) : make_int2(0, 0); };
+    int4 h = sl < M.nsl ? __ldg(M.hdr + sl) : none, hn = sl + nw < M.nsl ? __ldg(M.hdr + sl + nw) : none;
+    int2 r = records(h, 0);
+    pdl_enter();   // the matrix is constant: its first records may precede the wait
+    if (Epi::GATED && st != nullptr && st->done) return;
+    double red[Epi::NR];
+#pragma unroll
+    for (int j = 0; j < Epi::NR; ++j) red[j] = 0.0;
+    for (; sl < M.nsl; sl += nw) {
+        const int2 rn = records(hn, 0);
+        for (int o = lane * 16; o < hn.w >> 1; o += 32 * 16)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(M.v + hn.z + o));
+        const int4 h2 = sl + 2 * nw < M.nsl ? __ldg(M.hdr + sl + 2 * nw) : none;
+        const int row = sl * 32 + lane;
+        double opnd = 0.0, s = 0.0;
+        if constexpr (HasPre<Epi>::value)
+            if (row < M.n) opnd = epi.pre(row);
+        const double *xp = x + row;
+        const double *vp = M.v + h.z;
+        for (int k0 = 0; k0 < h.y; k0 += 32) {
+            if (k0) r = records(h, k0);
+            const int count = __popc(r.y);
+            int at = count;   // then: values of the diagonals before this one
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int u = __shfl_up_sync(full, at, o);
+                if (lane >= o) at += u;
+            }
+            __syncwarp();   // the last chunk's records are read
+            meta[lane] = make_int4(r.x, r.y, at - count, at);
+            __syncwarp();
+            const int m = min(h.y - k0, 32);
+            if (!(h.w & 1)) {
+                // every gather of the slice stays inside the matrix: rows without an entry load
+                // a neighbour's value and their own x like the others, and do not use them
+                for (int k = 0; k < m; k += kPackChunk) {   // masks past the last record are empty
+                    double a[kPackChunk], xv[kPackChunk];
+                    unsigned mask[kPackChunk];
+#pragma unroll
+                    for (int u = 0; u < kPackChunk; ++u) {
+                        const int4 q = meta[k + u];
+                        mask[u] = (unsigned)q.y;
+                        a[u] = __ldcs(vp + (unsigned)(q.z + __popc(mask[u] & below)));
+                        xv[u] = ldx(xp + q.x);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kPackChunk; ++u)
+                        if (mask[u] & mine) s = dia_fma(s, a[u], xv[u]);
+                }
+            } else {
+                for (int k = 0; k < m; ++k) {
+                    const int4 q = meta[k];
+                    const unsigned mask = (unsigned)q.y;
+                    if (mask & mine)
+                        s = dia_fma(s, __ldcs(vp + (q.z + __popc(mask & below))), ldx(xp + q.x));
+                }
+            }
+            vp += meta[31].w;
+        }
+        if (row < M.n) {
+            if constexpr (HasPre<Epi>::value) epi.emit_pre(row, s, opnd, red);
+            else epi.emit(row, s, red);
+        }
+        h = hn;
+        hn = h2;
+        r = rn;
+    }
+    pdl_release();
+    if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red, partials, st, epi);
+}
+
+// Launches k_spmv_pack over the packed slices of M (a DevCsr).
+template <class M, typename Epi>
+cudaError_t spmv_pack(cudaStream_t s, const M &m, const double *x, const Epi &epi, DState *st, double *partials) {
+    auto kern = k_spmv_pack<Epi>;
+    const PackView view{m.khdr, m.krec, static_cast<const double *>(m.dvals), (int)m.n, m.nsl};
+    return launch_k(kern, grid_for(kern, kWarps, m.nsl), 0, s, view, x, epi, st, partials);
+}
+
 // ---------------------------------------------------------------- CSR-vector SpMV
 // For callers without set-up (the kernel-level C-ABI): VEC lanes per row, 32/VEC rows
 // per warp, grid-stride over row groups. Each lane rounds its product; the group then

@@ -55,6 +55,9 @@ void release_dia(DevCsr &M) {
     M.nsl = M.dncls = 0;
     M.drs = 0;
     M.ndiag = 0;
+    M.pack = 0;
+    M.khdr = nullptr;
+    M.krec = nullptr;
 }
 
 static int col_hash(DevCsr &M, cudaStream_t s, unsigned long long *h) {
@@ -124,6 +127,56 @@ static sl::Args copy_args(const DevCsr &M, const void *vals) {
     return a;
 }
 
+static cudaError_t pack(bool place, const sl::Args &a, int4 *hdr, int2 *rec, cudaStream_t s) {
+    auto go = [&](auto kern) {
+        kern<<<grid_for(kern, kWarps, a.nsl), kThreads, 0, s>>>(a, hdr, rec);
+        return cudaGetLastError();
+    };
+    return place ? go(sl::k_pack<true>) : go(sl::k_pack<false>);
+}
+
+// The packed slices of M, where they are worth it: fewer bytes than the CSR streams, and at least
+// one slot in kPackFill of the slices' diagonals holds an entry (a product takes as many
+// instructions for an empty slot as for an entry).
+static int build_pack(DevCsr &M, cudaStream_t s, const void *vals, int nsl, const sl::Stats &st, int *m, int *id,
+                      int *k0) {
+    constexpr double kPackFill = 3.0;
+    const double bytes = (double)M.nnz * 8 + 8.0 * (double)st.ndiag + 16.0 * nsl;
+    const double csr = (double)M.nnz * (8 + (M.narrow ? 2 : 4)) + 4.0 * (M.n + 1);
+    if (st.refused || !(bytes < csr) || 32.0 * (double)st.ndiag > kPackFill * (double)M.nnz) return FIIM_OK;
+    const size_t b_hdr = Arena::need(sizeof(int4) * nsl), b_rec = Arena::need(sizeof(int2) * st.ndiag),
+                 b_st = Arena::need(sizeof(sl::Stats)),
+                 b_v = Arena::need(8UL * (M.nnz + 32));   // a lane past the last value reads one further
+    char *mem = nullptr;
+    if (cudaMalloc(&mem, b_hdr + b_rec + b_st + b_v) != cudaSuccess) {
+        cudaGetLastError();
+        return FIIM_OK;   // no room for the copy: the CSR streams serve
+    }
+    M.dia_mem = mem;
+    M.dia_bytes = b_hdr + b_rec + b_st + b_v;
+    M.khdr = reinterpret_cast<int4 *>(mem);
+    M.krec = reinterpret_cast<int2 *>(mem + b_hdr);
+    M.dstat = mem + b_hdr + b_rec;
+    M.dvals = mem + b_hdr + b_rec + b_st;
+    M.dvbytes = 8;
+    M.dsh = 32;
+    M.nsl = nsl;
+    M.ndiag = (long)st.ndiag;
+    FIIM_CUDA(cudaMemsetAsync(M.dstat, 0, sizeof(sl::Stats), s));
+    sl::k_offsets<<<1, 1024, 0, s>>>(nsl, m, nullptr, id, k0);
+    FIIM_CUDA(cudaGetLastError());
+    sl::Args a = copy_args(M, vals);
+    a.m = m;
+    a.k0 = k0;
+    FIIM_CUDA(pack(false, a, M.khdr, M.krec, s));
+    int bad = 0;
+    FIIM_CUDA(cudaMemcpyAsync(&bad, &a.stats->bad, sizeof(int), cudaMemcpyDeviceToHost, s));
+    FIIM_CUDA(cudaStreamSynchronize(s));   // before the scratch goes
+    if (bad) release_dia(M);
+    else M.pack = 1;
+    return FIIM_OK;
+}
+
 int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std::vector<int> *segments) {
     release_dia(M);
     M.dia_tried = false;
@@ -171,7 +224,7 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
     int *firsts = tmp.take<int>(table);   // 12 bytes a table entry with its key
     const bool share_on = share_wanted();
     // Diagonals, hashes and classes of the slices for R rows a lane; one read-back.
-    auto scan = [&](int R, int nsl) -> int {
+    auto scan = [&](int R, int nsl, int limit = kDiaMaxDiags) -> int {
         if (segmented) FIIM_CUDA(cudaMemcpyAsync(d_pos, pos.data(), sizeof(int2) * nsl, cudaMemcpyHostToDevice, s));
         FIIM_CUDA(cudaMemsetAsync(d_st, 0, sizeof(sl::Stats), s));
         FIIM_CUDA(cudaMemsetAsync(keys, 0, 8UL * table, s));
@@ -179,6 +232,7 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
         sl::Args a{};
         a.n = n;
         a.nsl = nsl;
+        a.most = limit;
         a.rp = M.rp;
         a.ci = M.ci;
         a.vals = vals;
@@ -204,7 +258,7 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
     auto smaller = [&](int R, int nsl) {
         const double dia = (double)vbytes * 32 * R * (double)st.ndiag + 4.0 * record_ints() * nsl;
         const double csr = (double)nnz * (vbytes + (M.narrow ? 2 : 4)) + 4.0 * (n + 1);
-        return !st.refused && !st.pad && dia < csr && 32.0 * R * (double)st.ndiag < 2147483648.0;
+        return !st.refused && !st.pad && st.max_m <= kDiaMaxDiags && dia < csr && 32.0 * R * (double)st.ndiag < 2147483648.0;
     };
     // Shared when at most half of the slices differ; otherwise the class numbers cost a load in
     // front of every block and most blocks are read once.
@@ -213,10 +267,12 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
     // 32-row slices average more diagonals than one chunk of the kernel holds (H at 128^3: 11
     // diagonals, 32.9 against 41.6 us a product; A and G, 7 diagonals, were slower with two).
     int R = dia_rows_per_lane(vbytes), nsl = 0;
+    const int asked = R;
+    bool dia = true;
     if (R) {
         nsl = slices(R);
         FIIM_TRY(scan(R, nsl));
-        if (!smaller(R, nsl)) return FIIM_OK;
+        dia = smaller(R, nsl);
     } else {
         R = 2;
         nsl = slices(R);
@@ -225,14 +281,26 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
         if (!two || !sharing(nsl)) {
             R = 1;
             nsl = slices(R);
-            FIIM_TRY(scan(R, nsl));
-            if (!smaller(R, nsl)) return FIIM_OK;
-            if (two && !sharing(nsl) && (long)st.ndiag > 8L * nsl) {
+            FIIM_TRY(scan(R, nsl, kPackMax));
+            dia = smaller(R, nsl);
+            if (dia && two && !sharing(nsl) && (long)st.ndiag > 8L * nsl) {
                 R = 2;
                 nsl = slices(R);
                 FIIM_TRY(scan(R, nsl));
             }
         }
+    }
+    if (!dia) {
+        const char *pe = std::getenv("FIIM_PACK");   // 0: the CSR streams instead of packed slices
+        if (pe && pe[0] == '0' && pe[1] == 0) return FIIM_OK;
+        // FP64 single systems only: with FP32 factors the CSR streams read 6 bytes an entry and the
+        // packed product's instructions weigh more (mixed solve 12.4 against 11.8 ms at 880,000 rows).
+        if (segmented || vbytes != 8) return FIIM_OK;
+        if (R != 1 || asked == 1) {   // scanned for the copy's limit of diagonals
+            nsl = slices(1);
+            FIIM_TRY(scan(1, nsl, kPackMax));
+        }
+        return build_pack(M, s, vals, nsl, st, m, id, k0);
     }
     const int sh = 32 * R, rs = record_ints();
     for (bool share = sharing(nsl);; share = false) {
@@ -293,14 +361,15 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
 static int enqueue_refresh(DevCsr &M, const void *vals, cudaStream_t s) {
     const sl::Args a = copy_args(M, vals);
     FIIM_CUDA(cudaMemsetAsync(M.dstat, 0, sizeof(sl::Stats), s));
-    if (M.dcls) FIIM_CUDA((walk<sl::kVerify, true>(M.dsh / 32, M.dvbytes, a, s)));
+    if (M.pack) FIIM_CUDA(pack(true, a, M.khdr, M.krec, s));
+    else if (M.dcls) FIIM_CUDA((walk<sl::kVerify, true>(M.dsh / 32, M.dvbytes, a, s)));
     else FIIM_CUDA((walk<sl::kPlace, false>(M.dsh / 32, M.dvbytes, a, s)));
     return FIIM_OK;
 }
 
 int refresh_dia(DevCsr &M, cudaStream_t s) {
     if (!dia_wanted()) return FIIM_OK;
-    if (!M.dia) {   // not built for the previous columns: decide again only if they changed
+    if (!M.dia && !M.pack) {   // not built for the previous columns: decide again only if they changed
         unsigned long long h = 0;
         FIIM_TRY(col_hash(M, s, &h));
         if (M.dia_tried && h == M.dia_cols) return FIIM_OK;

@@ -20,16 +20,15 @@ struct Stats {
     unsigned long long ndiag;        // diagonals over all slices
     unsigned long long uniq_ndiag;   // ... over the slices that are the first of their kind
     int max_m;                       // most diagonals of a slice
-    int refused;                     // a row not sorted by column, or a slice past kWalkMax
+    int refused;                     // a row not sorted by column, or a slice past `most`
     int pad;                         // an entry holds the padding pattern
     int uniq;                        // different slices
     int bad;                         // verify / place: the copy does not hold these values
 };
 
-constexpr int kWalkMax = kDiaMaxDiags;   // diagonals of one slice at most
-
 struct Args {
     int n, nsl;
+    int most;                        // scan: diagonals of one slice at most
     const int *__restrict__ rp;
     const int *__restrict__ ci;
     const void *vals;                // nnz values of B's width
@@ -104,7 +103,7 @@ static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
             for (int j = 1; j < R; ++j) d = min(d, cur[j]);
             d = __reduce_min_sync(full, d);
             if (d == INT_MAX) break;
-            if (k == (MODE == kScan ? kWalkMax : a.rs - kDiaRecHead) || (MODE >= kVerify && k == m_have)) {
+            if (k == (MODE == kScan ? a.most : a.rs - kDiaRecHead) || (MODE >= kVerify && k == m_have)) {
                 if (MODE == kScan) refused = true;
                 else bad = true;
                 break;
@@ -169,6 +168,63 @@ static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
     if (MODE == kScan && lane == 0 && max_m) {
         atomicAdd(&a.stats->ndiag, sum_m);
         atomicMax(&a.stats->max_m, max_m);
+    }
+}
+
+// The packed slices (one row a lane; fiim_kernels.cuh, k_spmv_pack): first, the records from the
+// scan's counts at the offsets k0, then the values. PLACE writes the values of a matrix whose
+// records are there already, and sets *bad when its columns are not those the records describe.
+template <bool PLACE>
+static __global__ void __launch_bounds__(kThreads)
+k_pack(Args a, int4 *hdr, int2 *rec) {
+    const unsigned full = 0xffffffffu;
+    const int lane = (int)threadIdx.x & 31;
+    const double *vals = static_cast<const double *>(a.vals);
+    double *dv = static_cast<double *>(a.dv);
+    for (int s = (int)blockIdx.x * kWarps + ((int)threadIdx.x >> 5); s < a.nsl; s += (int)gridDim.x * kWarps) {
+        const int row = s * 32 + lane;
+        const int k0 = PLACE ? hdr[s].x : a.k0[s], m = PLACE ? hdr[s].y : a.m[s];
+        const int v0 = __ldg(a.rp + s * 32);
+        int e = 0, end = 0;
+        if (row < a.n) {
+            e = __ldg(a.rp + row);
+            end = __ldg(a.rp + row + 1);
+        }
+        int cur = e < end ? __ldg(a.ci + e) - row : INT_MAX, at = v0;
+        bool bad = PLACE && hdr[s].z != v0;
+        int dlo = 0, dhi = 0;
+        for (int k = 0;; ++k) {
+            const int d = __reduce_min_sync(full, cur);
+            if (d == INT_MAX) {
+                if (k != m) bad = true;
+                break;
+            }
+            if (k == m) {
+                bad = true;
+                break;
+            }
+            if (k == 0) dlo = d;
+            dhi = d;
+            const unsigned mask = __ballot_sync(full, cur == d);
+            if (!PLACE && lane == 0) rec[k0 + k] = make_int2(d, (int)mask);
+            if (PLACE) {
+                const int2 q = rec[k0 + k];
+                if (q.x != d || q.y != (int)mask) {   // uniform in the warp
+                    bad = true;
+                    break;
+                }
+            }
+            if (cur == d) {
+                dv[at + __popc(mask & ((1u << lane) - 1u))] = vals[e];
+                cur = ++e < end ? __ldg(a.ci + e) - row : INT_MAX;
+                if (cur <= d) bad = true;   // not sorted: the next minimum would go back
+            }
+            at += __popc(mask);
+        }
+        // a chunk past the last record gathers at d = 0, so the slice's own rows count too
+        const bool edge = s * 32 + min(dlo, 0) < 0 || s * 32 + 31 + max(dhi, 0) > a.n - 1;
+        if (!PLACE && lane == 0) hdr[s] = make_int4(k0, m, v0, (at - v0) << 1 | (int)edge);
+        if (__any_sync(full, bad) && lane == 0) atomicExch(&a.stats->bad, 1);
     }
 }
 

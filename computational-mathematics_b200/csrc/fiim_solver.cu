@@ -213,6 +213,7 @@ template <typename Epi>
 cudaError_t launch_spmv(const DevCsr &M, cudaStream_t s, const double *x, const Epi &epi, DState *st,
                         double *partials, int *fault = nullptr) {
     if (M.dia) return spmv_dia(s, M, x, epi, st, partials);
+    if (M.pack) return spmv_pack(s, M, x, epi, st, partials);
     if (M.form == kFormWarp) return spmv_warp(s, M, x, epi, st, partials);
     if (M.form == kFormBulk && fault) {
         if (M.tile == 1024) return spmv_pipe<1024>(s, M, x, epi, st, partials, fault);
@@ -971,7 +972,7 @@ int Solver::reload(const int *Ai, const int *Aj, const double *Av, const int *Gi
         const bool dev[] = {dev_src, dev_src, dev_src, dev_src, dev_src};
         auto issued = [&](int k) -> int {
             DevCsr &M = *mats[k];
-            if (!aux || !M.rows_same || M.nblk <= 0 || !M.dia || M.dvbytes != 8) return FIIM_OK;
+            if (!aux || !M.rows_same || M.nblk <= 0 || !(M.dia || M.pack) || M.dvbytes != 8) return FIIM_OK;
             early[k] = true;
             h_spec[k] = 1;
             return refresh_dia_async(M, stream, aux, aux_ev[k], h_spec + k);
@@ -992,7 +993,7 @@ int Solver::reload(const int *Ai, const int *Aj, const double *Av, const int *Gi
         // Everything of the sliced-diagonal copy that a captured launch holds: a rebuilt copy
         // may reuse the freed allocation's address with another layout inside it.
         auto dia_args = [](const DevCsr &D) {
-            return std::make_tuple(D.dia, D.drec, D.dvals, D.dcls, D.nsl, D.drs, D.dsh);
+            return std::make_tuple(D.dia, D.pack, D.drec, D.khdr, D.dvals, D.dcls, D.nsl, D.drs, D.dsh);
         };
         const auto was_dia = dia_args(M);
         if (M.rows_same && M.nblk > 0) {

@@ -239,7 +239,8 @@ class Solver(_Handle):
 
     def spmv_shape(self, which: int):
         """(row-block size, form) of matrix `which` (0 A, 1 G, 2 H): form 0 CSR streams through
-        registers, 1 by bulk copies, 2 one warp per row block, 3 the sliced-diagonal copy."""
+        registers, 1 by bulk copies, 2 one warp per row block, 3 the sliced-diagonal copy,
+        4 packed slices."""
         t, f = C.c_int(0), C.c_int(0)
         _check(lib().fiim_solver_spmv_shape(self._h, C.c_int(which), C.byref(t), C.byref(f)))
         return t.value, f.value

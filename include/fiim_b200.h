@@ -157,9 +157,11 @@ int64_t fiim_solver_device_bytes(fiim_solver_t s);
 /* Row-block size (entries) and form of the SpMV for matrix `which` (0 A, 1 G, 2 H, 3 L,
    4 U). Forms: 0 CSR streams through registers, pipelined by one block; 1 bulk copies into
    two shared-memory buffers; 2 one warp per row block; 3 the sliced-diagonal copy (rows in
-   slices of 32 that share at most 28 diagonals; built when the rows are sorted by column and
-   it moves fewer bytes; FIIM_DIA=0 or FIIM_SPMV=rows/staged/warp keep the CSR streams). Every
-   form gives the same bits. */
+   slices of 32 or 64 that share at most 28 diagonals; built when the rows are sorted by column
+   and it moves fewer bytes; equal slices share one block); 4 packed slices (32 sorted rows that
+   share at most 64 diagonals more loosely: a row mask per diagonal, no padding). FIIM_DIA=0 or
+   FIIM_SPMV=rows/staged/warp keep the CSR streams, FIIM_PACK=0 keeps them in place of form 4,
+   FIIM_DIA_SHARE=0 gives every slice of form 3 its own block. Every form gives the same bits. */
 int fiim_solver_spmv_shape(fiim_solver_t s, int which, int *tile, int *form);
 
 /* y = A x (op 0) or y = M x, the preconditioner application (op 1), with the solver's
@@ -205,8 +207,9 @@ int fiim_solver_test_stall(fiim_solver_t s);
 double fiim_solver_iteration_bytes(fiim_solver_t s);
 
 /* Bytes that one product with matrix `which` (0 A, 1 G, 2 H, 3 L, 4 U) reads from the
- * matrix in the form it is served in (fiim_solver_spmv_shape): 256 per diagonal of a slice
- * plus the slice records for the sliced-diagonal copy; the values, the column stream (2 or 4
+ * matrix in the form it is served in (fiim_solver_spmv_shape): the blocks and records held and
+ * 4 per slice that shares one for the sliced-diagonal copy; the values and 8 per diagonal and 16
+ * per slice for packed slices; the values, the column stream (2 or 4
  * bytes an entry), the row offsets and the row-block bounds for the CSR streams. -1 for a bad
  * handle or index. */
 double fiim_solver_matrix_bytes(fiim_solver_t s, int which);

@@ -78,6 +78,68 @@ def test_nonfinite_vector_entries(monkeypatch, kind, bad):
         assert same(y, ref), (env, form)
 
 
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 1000, 4099])
+@pytest.mark.parametrize("width,drop", [(9, 0.5), (33, 0.6), (64, 0.62), (65, 0.6)])
+def test_packed_products(monkeypatch, n, width, drop):
+    """Rows that hold a random part of 9 to 65 diagonals (a slice's records in one or two loads;
+    65 in a full slice are one too many): packed slices where they serve, the same bits anyway,
+    also with infinities in the vector."""
+    rng = np.random.default_rng(width)
+    offsets = [0] + [int(o) for o in rng.permutation(np.r_[-40:0, 1:41])[:width - 1]]
+    A = banded(n, offsets, KINDS["varying"], drop=drop, seed=n)
+    u = np.random.default_rng(n).standard_normal(n)
+    u[n // 2] = np.inf
+    ref = O.csr_mv(*A, u)
+    forms = set()
+    for env in ({}, {"FIIM_PACK": "0"}, {"FIIM_DIA": "0"}):
+        y, form = product(A, u, monkeypatch, **env)
+        forms.add(form)
+        assert same(y, ref), (env, form)
+    if n >= 1000 and width <= 64:
+        assert 4 in forms
+    if n >= 1000 and width == 65:
+        assert 4 not in forms
+
+
+def uneven_system(c=40):
+    """3D convection-diffusion with a random coefficient field: the factors' slices do not share their
+    diagonals closely (packed slices)."""
+    A = FB.gen_convdiff3d(c, 0.5)
+    n = c ** 3
+    d = np.exp(0.5 * np.random.default_rng(2).standard_normal(n))
+    A = (A[0], A[1], A[2] * d[A[1]] / d[np.repeat(np.arange(n), np.diff(A[0]))])
+    return A, FB.pdfiim_build(A, 0.05, 2, 2, 1)
+
+
+def test_packed_reload():
+    """Drop-in calls over a system whose factors are served by packed slices: new values in the same
+    structure, then other columns with the same row offsets; each equals a fresh solver's result
+    bit for bit."""
+    A, F = uneven_system()
+    n = len(A[0]) - 1
+    H = (F["Hi"], F["Hj"], F["Hv"])
+    b = FB.rand_normal(n, 3)
+    # other columns, the same row lengths: each row's second entry moves one column on where that is free
+    moved = H[1].copy()
+    first = H[0][:-1][np.diff(H[0]) > 2] + 1
+    free = moved[first] + 1 < moved[first + 1]
+    moved[first[free]] += 1
+    assert free.sum() > 100
+    prev = FB.dropin_cache(False)
+    try:
+        for Hj, Hv in ((H[1], H[2]), (H[1], H[2] * 1.25), (moved, H[2]), (H[1], H[2])):
+            FF = dict(F, Hj=Hj, Hv=Hv)
+            with FB.Solver(A, FF, variant="pdfiim") as S:
+                y = np.zeros(n)
+                r1 = S.solve(b, y, tol=1e-10, nmax=60)
+                assert S.spmv_shape(2)[1] == 4
+            x = np.zeros(n)
+            r = FB.EPBiCGSTAB_pdfiim(A, b, 1e-10, 60, (F["Gi"], F["Gj"], F["Gv"]), F["IDv"], (H[0], Hj, Hv), x)
+            assert np.array_equal(x, y, equal_nan=True) and r[1] == r1["iter"]
+    finally:
+        FB.dropin_cache(prev)
+
+
 @pytest.mark.parametrize("precision", ["fp64", "fp32", "bf16"])
 def test_batch_with_and_without_shared_blocks(monkeypatch, precision):
     """A batch's solves with shared blocks and with every slice's own: the products are the same
