@@ -61,7 +61,6 @@ struct DevCsr {
     double *v = nullptr;
     float *v32 = nullptr;
     __nv_bfloat16 *v16 = nullptr;
-    int vec = 8;                 // lanes per row of the set-up-free SpMV
     int tile = 2048;             // entries per row block of the CSR-stream SpMV
     int form = 0;                // CSR-stream SpMV form, one of the kForm* constants
     int *rb = nullptr;           // row-block first rows (device), nblk + 1 entries
@@ -111,8 +110,6 @@ struct HostCsr {
     std::vector<int> rp, ci;
     std::vector<double> v;
 };
-
-int heuristic_vec(long n, long nnz);
 
 // Set-up helpers shared by the FP64 and mixed-precision solvers (fiim_solver.cu).
 void signature(DevCsr &M, const int *host_rp);

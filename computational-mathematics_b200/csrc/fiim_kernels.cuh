@@ -1200,9 +1200,8 @@ cudaError_t spmv_pack(cudaStream_t s, const M &m, const double *x, const Epi &ep
 // For callers without set-up (the kernel-level C-ABI): VEC lanes per row, 32/VEC rows
 // per warp, grid-stride over row groups. Each lane rounds its product; the group then
 // adds the products in storage order by broadcasting them lane by lane, so the sum is
-// the same as the left-to-right CSR loop for every VEC. FILL 0 uses every entry; 1
-// keeps col >= row and 2 keeps col <= row (MKL's TRIANGULAR descriptors).
-template <int VEC, typename Epi, int FILL = 0>
+// the same as the left-to-right CSR loop for every VEC. Serves the callers who name VEC.
+template <int VEC, typename Epi>
 static __global__ void __launch_bounds__(kThreads)
 k_spmv_vec(CsrView<double> M, const double *__restrict__ x, Epi epi, DState *st,
            double *__restrict__ partials) {
@@ -1227,22 +1226,129 @@ k_spmv_vec(CsrView<double> M, const double *__restrict__ x, Epi epi, DState *st,
         for (int t = 0; t < trips; ++t) {
             const int k = t * VEC + lir;
             double p = 0.0;
-            int keep = 0;
-            if (k < len) {
-                const int c = ldi(M.ci + beg + k);
-                keep = !((FILL == 1 && c < row) || (FILL == 2 && c > row));
-                if (keep) p = __dmul_rn(ldm(M.v + beg + k), ldx(x + c));
-            }
+            if (k < len) p = __dmul_rn(ldm(M.v + beg + k), ldx(x + ldi(M.ci + beg + k)));
 #pragma unroll
             for (int j = 0; j < VEC; ++j) {
                 const double pj = __shfl_sync(0xffffffffu, p, gbase + j);
-                const int kj = __shfl_sync(0xffffffffu, keep, gbase + j);
-                if (kj) s = __dadd_rn(s, pj);
+                if (t * VEC + j < len) s = __dadd_rn(s, pj);
             }
         }
         if (row < M.n && lir == 0) epi.emit(row, s, red);
     }
     if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red, partials, st, epi);
+}
+
+// ---------------------------------------------------------------- set-up-free CSR-stream SpMV
+// The kernel-level calls' product where the caller names no lane count: nothing about the matrix
+// is known on the host, so no copy of its entry count and no wait stand in front of the launch. A
+// warp takes `rpw` consecutive rows, whose entries are one run: it loads them coalesced, kStream
+// entries at a time, leaves the rounded products in its part of shared memory, and lane l adds row
+// l's products left to right, from tile to tile, so every sum is the reference's bit for bit.
+// FILL 0 uses every entry; 1 keeps col >= row and 2 keeps col <= row (MKL's TRIANGULAR
+// descriptors), told apart by the columns kept beside the products. rpw comes from the entry count read on the device: 32 rows while they hold about
+// two tiles, fewer for longer rows, and (while they hold more than 64) fewer while some warps of
+// the grid would have no rows.
+// The next rows' offsets are loaded while these are summed.
+constexpr int kStream = 256;
+template <typename Epi, int FILL>
+static __global__ void __launch_bounds__(kThreads, 4)
+k_spmv_stream(CsrView<double> M, const double *__restrict__ x, Epi epi) {
+    constexpr int PER = kStream / 32;
+    constexpr int AHEAD = 4;
+    constexpr int PAD = kStream + kStream / 16;   // one slot more every 16: rows of 4 or 8 entries spread over the banks
+    __shared__ double prod_all[kWarps][PAD];
+    __shared__ int col_all[FILL ? kWarps : 1][FILL ? kStream : 1];
+    const unsigned full = 0xffffffffu;
+    const int lane = (int)threadIdx.x & 31, w = (int)threadIdx.x >> 5;
+    double *prod = prod_all[w];
+    int *col = col_all[FILL ? w : 0];
+    const long nw = (long)gridDim.x * kWarps;
+    const long nnz = __ldg(M.rp + M.n);
+    int rpw = 32;
+    while (rpw > 1 && (rpw * nnz > 2L * kStream * M.n || (M.n < nw * rpw && rpw * nnz > 64L * M.n))) rpw >>= 1;
+    if (rpw == 1) {   // long rows: a warp each, its products passed to the sum lane by lane
+        pdl_enter();
+        for (long row = (long)blockIdx.x * kWarps + w; row < M.n; row += nw) {
+            const int e1 = __ldg(M.rp + row + 1);
+            double s = 0.0;
+            for (int t0 = __ldg(M.rp + row); t0 < e1; t0 += 32) {
+                const int e = t0 + lane, c = e < e1 ? ldi(M.ci + e) : 0;
+                // what is not added is a zero: a sum that starts at +0 is never -0, so +0 leaves it as it is
+                const bool keep = e < e1 && (FILL == 0 || (FILL == 1 ? c >= row : c <= row));
+                const double p = keep ? __dmul_rn(ldm(M.v + e), ldx(x + c)) : 0.0;
+#pragma unroll
+                for (int j = 0; j < 32; ++j) s = __dadd_rn(s, __shfl_sync(full, p, j));
+            }
+            if (lane == 0) {
+                double red[Epi::NR];
+                epi.emit(row, s, red);
+            }
+        }
+        pdl_release();
+        return;
+    }
+    auto at = [](int e) { return e + (e >> 4); };
+    long row = ((long)blockIdx.x * kWarps + w) * rpw + lane;
+    int beg = 0, end = 0;
+    auto offsets = [&](long r) {   // lanes past the group's rows repeat its end
+        const long last = min(r - lane + rpw, (long)M.n);
+        beg = __ldg(M.rp + min(r, last));
+        end = __ldg(M.rp + min(r + 1, last));
+    };
+    if (row - lane < M.n) offsets(row);
+    pdl_enter();   // the vector may still be written by the launch before this one; the matrix may not
+    for (; row - lane < M.n; row += nw * rpw) {
+        const int e0 = __shfl_sync(full, beg, 0), e1 = __shfl_sync(full, end, 31), rb = beg, re = end;
+        const bool live = lane < rpw && row < M.n;
+        if (row - lane + nw * rpw < M.n) offsets(row + nw * rpw);
+        double s = 0.0;
+        for (int t0 = e0; t0 < e1; t0 += kStream) {
+            int c[PER];
+            double v[PER];
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                const int e = t0 + u * 32 + lane;
+                c[u] = e < e1 ? ldi(M.ci + e) : 0;
+                v[u] = e < e1 ? ldm(M.v + e) : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                const int p = u * 32 + lane;
+                if (t0 + p < e1) {
+                    prod[at(p)] = __dmul_rn(v[u], ldx(x + c[u]));
+                    if (FILL) col[p] = c[u];
+                }
+            }
+            __syncwarp();
+            if (live) {
+                const int b = max(rb, t0) - t0, e = min(re, t0 + kStream) - t0;
+                auto keep = [&](int k) {
+                    return FILL == 0 || (FILL == 1 ? col[FILL ? k : 0] >= row : col[FILL ? k : 0] <= row);
+                };
+                int k = b;
+                for (; k + AHEAD <= e; k += AHEAD) {   // the products are read ahead of the chain of sums
+                    double p[AHEAD];
+                    bool in[AHEAD];
+#pragma unroll
+                    for (int u = 0; u < AHEAD; ++u) {
+                        p[u] = prod[at(k + u)];
+                        in[u] = keep(k + u);
+                    }
+#pragma unroll
+                    for (int u = 0; u < AHEAD; ++u)
+                        if (in[u]) s = __dadd_rn(s, p[u]);
+                }
+                for (; k < e; ++k)
+                    if (keep(k)) s = __dadd_rn(s, prod[at(k)]);
+            }
+            __syncwarp();
+        }
+        if (live) {
+            double red[Epi::NR];
+            epi.emit(row, s, red);
+        }
+    }
+    pdl_release();
 }
 
 // ---------------------------------------------------------------- streaming kernels

@@ -16,12 +16,11 @@
 
 #include <cuda_runtime.h>
 
-#include <algorithm>
 #include <mutex>
 
 #include "fiim_b200.h"
 #include "fiim_internal.h"
-#include "fiim_kernels.cuh"
+#include "fiim_solver.h"
 
 namespace {
 
@@ -56,17 +55,6 @@ int noalloc_scratch(double **out) {
     return FIIM_OK;
 }
 
-int grid_rows(long n, int rows_per_block) {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
-        cudaGetLastError();
-        sms = 148;
-    }
-    const long need = (n + rows_per_block - 1) / rows_per_block;
-    return (int)std::max<long>(1, std::min<long>(need, 8L * sms));
-}
-
 }  // namespace
 
 extern "C" int fiim_prec_apply_noalloc(int n, const int *Gi, const int *Gj, const double *Gv,
@@ -82,14 +70,5 @@ extern "C" int fiim_prec_apply_noalloc(int n, const int *Gi, const int *Gj, cons
     double *tm = nullptr;
     FIIM_TRY(noalloc_scratch(&tm));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // Eight lanes per row; every lane count gives the same sums (storage order).
-    constexpr int kVec = 8;
-    const int g = grid_rows(n, (32 / kVec) * fiim::kWarps);
-    fiim::k_spmv_vec<kVec, fiim::EpiScale, 2><<<g, fiim::kThreads, 0, s>>>(
-        fiim::CsrView<double>{Hi, Hj, Hv, n}, r, fiim::EpiScale{tm, IDv}, nullptr, nullptr);
-    FIIM_CUDA(cudaGetLastError());
-    fiim::k_spmv_vec<kVec, fiim::EpiStore, 1><<<g, fiim::kThreads, 0, s>>>(
-        fiim::CsrView<double>{Gi, Gj, Gv, n}, tm, fiim::EpiStore{z}, nullptr, nullptr);
-    FIIM_CUDA(cudaGetLastError());
-    return FIIM_OK;
+    return fiim::prec_launch(n, Gi, Gj, Gv, IDv, Hi, Hj, Hv, r, z, tm, s);
 }

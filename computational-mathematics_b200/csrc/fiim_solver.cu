@@ -55,7 +55,13 @@ int set_error(int code, const char *fmt, ...) {
 const char *last_error() { return g_err.c_str(); }
 
 int check_device(int *dev_out) {
+    static std::atomic<bool> known[64];   // a device found to be served stays so
     int dev = 0, count = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 && known[dev].load(std::memory_order_relaxed)) {
+        if (dev_out) *dev_out = dev;
+        return FIIM_OK;
+    }
+    cudaGetLastError();
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) {
         cudaGetLastError();
         return set_error(FIIM_ENODEV, "no CUDA device visible");
@@ -66,6 +72,7 @@ int check_device(int *dev_out) {
     if (major != 10)
         return set_error(FIIM_ENODEV, "device %d has compute capability %d.x; this library is built for sm_100a",
                          dev, major);
+    if (dev >= 0 && dev < 64) known[dev].store(true, std::memory_order_relaxed);
     if (dev_out) *dev_out = dev;
     return FIIM_OK;
 }
@@ -109,25 +116,25 @@ void Arena::release() {
 size_t Arena::need(size_t bytes) { return (bytes + 255) & ~size_t(255); }
 
 // ------------------------------------------------------------------ launch shapes
-template <int VEC, int FILL, typename Epi>
+template <int VEC, typename Epi>
 static cudaError_t spmv_vec(cudaStream_t s, const CsrView<double> &M, const double *x, const Epi &epi,
                             DState *st, double *partials) {
-    auto kern = k_spmv_vec<VEC, Epi, FILL>;
+    auto kern = k_spmv_vec<VEC, Epi>;
     const int g = grid_for(kern, (32 / VEC) * kWarps, M.n);
     kern<<<g, kThreads, 0, s>>>(M, x, epi, st, partials);
     return cudaGetLastError();
 }
 
 // Set-up-free SpMV (kernel-level C-ABI): VEC lanes per row, exact row order.
-template <int FILL = 0, typename Epi>
+template <typename Epi>
 cudaError_t launch_spmv_vec(int vec, cudaStream_t s, const CsrView<double> &M, const double *x,
                             const Epi &epi, DState *st, double *partials) {
     switch (vec) {
-        case 2: return spmv_vec<2, FILL>(s, M, x, epi, st, partials);
-        case 4: return spmv_vec<4, FILL>(s, M, x, epi, st, partials);
-        case 8: return spmv_vec<8, FILL>(s, M, x, epi, st, partials);
-        case 16: return spmv_vec<16, FILL>(s, M, x, epi, st, partials);
-        default: return spmv_vec<32, FILL>(s, M, x, epi, st, partials);
+        case 2: return spmv_vec<2>(s, M, x, epi, st, partials);
+        case 4: return spmv_vec<4>(s, M, x, epi, st, partials);
+        case 8: return spmv_vec<8>(s, M, x, epi, st, partials);
+        case 16: return spmv_vec<16>(s, M, x, epi, st, partials);
+        default: return spmv_vec<32>(s, M, x, epi, st, partials);
     }
 }
 
@@ -229,13 +236,6 @@ cudaError_t launch_spmv(const DevCsr &M, cudaStream_t s, const double *x, const 
 
 template <typename K>
 static int stream_grid(K kernel, long n) { return grid_for(kernel, kThreads, n); }
-
-int heuristic_vec(long n, long nnz) {
-    const double mean = n > 0 ? (double)nnz / (double)n : 1.0;
-    int v = 2;
-    while (v < 32 && v < mean) v <<= 1;
-    return v;
-}
 
 void build_row_blocks(const std::vector<int> &rp, int tile, int max_rows, std::vector<int> &rb) {
     const int n = (int)rp.size() - 1;
@@ -1328,17 +1328,33 @@ double Solver::iteration_bytes() const {
 }
 
 // ------------------------------------------------------------------ kernel-level API
+// One set-up-free product on s (k_spmv_stream). after_ours: the launch before it on s is ours and waited for all before itself, so this one may
+// read its matrix while that one finishes (programmatic dependent launch); otherwise the launch
+// before it may be the caller's, still writing the matrix.
+template <int FILL, typename Epi>
+static cudaError_t launch_stream(cudaStream_t s, const CsrView<double> &M, const double *x, const Epi &epi, bool after_ours) {
+    auto kern = k_spmv_stream<Epi, FILL>;
+    const int g = grid_for(kern, kWarps, M.n);   // enough for a warp a row
+    if (after_ours) return launch_k(kern, g, 0, s, M, x, epi);
+    kern<<<g, kThreads, 0, s>>>(M, x, epi);
+    return cudaGetLastError();
+}
+
 int spmv_api(int n, const int *Ai, const int *Aj, const double *Av, const double *x, double *y,
              int vec, cudaStream_t s) {
     if (n <= 0 || !Ai || !Aj || !Av || !x || !y) return set_error(FIIM_EARG, "null array or n <= 0");
     FIIM_TRY(check_device(nullptr));
-    if (vec != 2 && vec != 4 && vec != 8 && vec != 16 && vec != 32) {
-        int z = 0;
-        FIIM_CUDA(cudaMemcpyAsync(&z, Ai + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-        FIIM_CUDA(cudaStreamSynchronize(s));
-        vec = heuristic_vec(n, z);
-    }
-    FIIM_CUDA(launch_spmv_vec(vec, s, CsrView<double>{Ai, Aj, Av, n}, x, EpiStore{y}, nullptr, nullptr));
+    const CsrView<double> A{Ai, Aj, Av, n};
+    if (vec == 2 || vec == 4 || vec == 8 || vec == 16 || vec == 32)
+        FIIM_CUDA(launch_spmv_vec(vec, s, A, x, EpiStore{y}, nullptr, nullptr));
+    else FIIM_CUDA(launch_stream<0>(s, A, x, EpiStore{y}, false));
+    return FIIM_OK;
+}
+
+int prec_launch(int n, const int *Gi, const int *Gj, const double *Gv, const double *IDv_, const int *Hi, const int *Hj,
+                const double *Hv, const double *rr, double *z, double *tmv, cudaStream_t s) {
+    FIIM_CUDA(launch_stream<2>(s, CsrView<double>{Hi, Hj, Hv, n}, rr, EpiScale{tmv, IDv_}, false));
+    FIIM_CUDA(launch_stream<1>(s, CsrView<double>{Gi, Gj, Gv, n}, tmv, EpiStore{z}, true));
     return FIIM_OK;
 }
 
@@ -1347,15 +1363,7 @@ int prec_api(int n, const int *Gi, const int *Gj, const double *Gv, const double
     if (n <= 0 || !Gi || !Gj || !Gv || !IDv_ || !Hi || !Hj || !Hv || !rr || !z || !tmv)
         return set_error(FIIM_EARG, "null array or n <= 0");
     FIIM_TRY(check_device(nullptr));
-    int zz[2] = {0, 0};
-    FIIM_CUDA(cudaMemcpyAsync(&zz[0], Gi + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FIIM_CUDA(cudaMemcpyAsync(&zz[1], Hi + n, sizeof(int), cudaMemcpyDeviceToHost, s));
-    FIIM_CUDA(cudaStreamSynchronize(s));
-    FIIM_CUDA(launch_spmv_vec<2>(heuristic_vec(n, zz[1]), s, CsrView<double>{Hi, Hj, Hv, n}, rr,
-                             EpiScale{tmv, IDv_}, nullptr, nullptr));
-    FIIM_CUDA(launch_spmv_vec<1>(heuristic_vec(n, zz[0]), s, CsrView<double>{Gi, Gj, Gv, n}, tmv,
-                             EpiStore{z}, nullptr, nullptr));
-    return FIIM_OK;
+    return prec_launch(n, Gi, Gj, Gv, IDv_, Hi, Hj, Hv, rr, z, tmv, s);
 }
 
 }  // namespace fiim

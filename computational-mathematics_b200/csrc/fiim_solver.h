@@ -107,6 +107,9 @@ namespace fiim {
 
 int spmv_api(int n, const int *Ai, const int *Aj, const double *Av, const double *x, double *y,
              int vec, cudaStream_t s);
+// The two launches of z = G (IDv o (H r)), arguments checked by the caller.
+int prec_launch(int n, const int *Gi, const int *Gj, const double *Gv, const double *IDv, const int *Hi, const int *Hj,
+                const double *Hv, const double *r, double *z, double *tm, cudaStream_t s);
 int prec_api(int n, const int *Gi, const int *Gj, const double *Gv, const double *IDv,
              const int *Hi, const int *Hj, const double *Hv, const double *r, double *z,
              double *tm, cudaStream_t s);

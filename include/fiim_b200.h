@@ -286,7 +286,8 @@ int fiim_block_destroy(fiim_block_t s);
  * Kernel-level entry points (device arrays, caller's stream; asynchronous).
  * ======================================================================== */
 
-/* y = A x, FP64 CSR. vec = lanes per row (2,4,8,16,32) or 0 to choose from nnz/n.
+/* y = A x, FP64 CSR. vec = lanes per row (2,4,8,16,32), or 0 for a kernel that
+ * streams each run of rows and reads what it needs to know of the matrix on the device.
  * Replaces mkl_sparse_d_mv(NON_TRANSPOSE, 1.0, A, GENERAL, x, 0.0, y)
  * (AFIIM/src/bicgstab.cpp:151,178,195). */
 int fiim_spmv(int n, const int *Ai, const int *Aj, const double *Av, const double *x, double *y,
