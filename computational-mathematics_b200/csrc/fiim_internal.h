@@ -115,23 +115,30 @@ struct HostCsr {
 void signature(DevCsr &M, const int *host_rp);
 size_t csr_bytes(long n, long nnz);
 int carve_csr(Arena &ar, DevCsr &M, long n, long nnz);
-// Host-to-device copies from pageable memory through a ring of pinned buffers: a chunk is
-// copied into a pinned buffer by all host threads while the previous chunks' DMA runs, which
-// moves pageable data several times faster than a copy from pageable memory (staged by the
-// driver one page run at a time). Pinned sources and small copies go straight to
-// cudaMemcpyAsync. As with that call, the source is read completely before copy() returns;
-// the DMA from the pinned buffers may still be in flight.
+// Copies between pageable memory and the device through a ring of pinned buffers: all host
+// threads copy one chunk to or from a pinned buffer while the other chunks' DMA runs, which moves
+// pageable data several times faster than a copy from pageable memory (staged by the driver one
+// page run at a time). Pinned memory and small copies go straight to cudaMemcpyAsync. copy: the
+// source is read completely before it returns, the DMA may still be in flight on s; copy_out
+// returns with the destination written, and waits for nothing but its own stream.
+// One ring per thread and device (thread_stager), kept while the thread lives: pinning the
+// buffers costs more than most copies. 32 MB each, given back when the thread ends.
 struct Stager {
     static constexpr int kBufs = 4;
-    static constexpr size_t kChunk = size_t(16) << 20;
+    static constexpr size_t kChunk = size_t(8) << 20;
     static constexpr size_t kMinStaged = size_t(4) << 20;
     void *buf[kBufs] = {};
     cudaEvent_t ev[kBufs] = {};
     bool pending[kBufs] = {};
     int next = 0;
+    cudaStream_t out = nullptr;
     int copy(void *dst, const void *src, size_t bytes, cudaStream_t s);
+    int copy_out(void *dst, const void *src, size_t bytes);
+    bool ready();                // the pinned buffers (false: no pinned memory)
     void release();
+    ~Stager() { release(); }
 };
+Stager &thread_stager(int device);
 
 int upload_csr_async(DevCsr &M, long nnz_cap, int n, const int *rp, const int *ci, const double *v, bool device_src,
                      cudaStream_t s, Stager *stager = nullptr);

@@ -8,12 +8,12 @@
 //   * the dense LU with partial pivoting of the pattern's B (Golub & Van Loan Alg. 3.4.1,
 //     first largest pivot) eliminates one row per lane; every product and difference is
 //     rounded separately, as the host code compiled without contraction;
-//   * the assembly of the right-hand sides, the triangular solves, the filter norms and the
-//     D^{-1} sums keep the host's sequential order (lane 0);
+//   * the triangular solves, the filter norms and the D^{-1} sums add in the host's sequential
+//     order; products and independent sums are spread over the lanes;
 //   * kept entries are sorted by index through their ranks.
-// Two passes over the rows: the first counts the kept entries of every row, the host turns
-// the counts into offsets, the second writes the entries and D^{-1}. A row whose pattern
-// outgrows the warp's shared memory (CAP members in a solve, 4 CAP in the set; 2048 at the
+// One pass over the rows leaves every row's entries and D^{-1} in the next free places; running
+// totals of the counts and a transpose, all on the device, put them in order, and the second call
+// copies them from there into the caller's arrays. A row whose pattern outgrows the warp's shared memory (CAP members in a solve, 4 CAP in the set; 2048 at the
 // largest CAP) is listed and built again with a larger CAP; past the largest CAP the call
 // returns FIIM_EARG and the host construction serves.
 
@@ -45,9 +45,11 @@ struct Params {
 struct Out {
     int *gcnt, *hcnt;           // kept entries + unit diagonal, per row
     double *D;
-    const long *goff, *hoff;    // write pass: entry offsets of each row
-    int *gj, *hj;
-    double *gv, *hv;
+    long *at;                   // a row's first entry in ej / ev: g's, then h's
+    int *ej;
+    double *ev;
+    unsigned long long *used;   // entries asked for so far
+    unsigned long long room;    // entries ej and ev hold
     int *overflow, *noverflow;  // rows left for a larger CAP
 };
 
@@ -114,6 +116,20 @@ struct RowBuilder {
         return -1;
     }
 
+    // x at the pattern's members from -(row i of M), columns below i; a column stored twice
+    // counts as its last entry does.
+    __device__ void assemble(const CsrD &M, double *x, int len) {
+        const int beg = M.rp[i], end = M.rp[i + 1];
+        for (int base = beg; base < end; base += 32) {
+            const int k = base + lane;
+            const int c = k < end ? M.ci[k] : INT_MAX;
+            const int q = c < i ? pos_of(c, len) : -1;
+            const unsigned same = __match_any_sync(0xffffffffu, q);
+            if (q >= 0 && (same >> lane) == 1u) x[q] = -M.v[k];
+            __syncwarp();
+        }
+    }
+
     // LU with partial pivoting of B (len x len, row-major), then B g = g, B^T h = h.
     __device__ void factor_solve(int len) {
         double *B = s.B;
@@ -152,49 +168,87 @@ struct RowBuilder {
             for (int r = k + 1 + lane; r < len; r += 32) {
                 const double l = B[r * len + k] / d;
                 B[r * len + k] = l;
-                for (int c = k + 1; c < len; ++c)
-                    B[r * len + c] = __dsub_rn(B[r * len + c], __dmul_rn(l, B[k * len + c]));
+                // four entries of the row in flight: the compiler cannot tell the rows apart
+                double *Br = B + r * len;
+                const double *Bk = B + k * len;
+                int c = k + 1;
+                for (; c + 4 <= len; c += 4) {
+                    double q[4], p[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        q[u] = Br[c + u];
+                        p[u] = Bk[c + u];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) Br[c + u] = __dsub_rn(q[u], __dmul_rn(l, p[u]));
+                }
+                for (; c < len; ++c) Br[c] = __dsub_rn(Br[c], __dmul_rn(l, Bk[c]));
             }
             __syncwarp();
         }
-        if (lane == 0) {
-            double *g = s.g, *h = s.h;
-            const int *piv = s.piv;
-            // B g = g: row swaps, forward, backward (lu_solve)
+        solve_pair(len);
+    }
+
+    // B g = g and B^T h = h with the factors of factor_solve, both at once. Each unknown's sum is
+    // subtracted in ascending order of the other unknown's index, as a sequential solve does. The
+    // forward solves go column by column over the lanes, which is that order. A backward solve
+    // needs its row's products lowest index first, so the lanes form them and one lane
+    // subtracts them: lane 0 for g, lane 1 for h, whose chains are as long. (Lane 0 doing all four
+    // solves alone was three quarters of the kernel.) The products lie in the set's list, which is
+    // written again after the solve.
+    __device__ void solve_pair(int len) {
+        static_assert(WarpSmem<CAP>::SET * sizeof(int) >= 2 * CAP * sizeof(double), "two rows of products");
+        const double *B = s.B;
+        double *g = s.g, *h = s.h, *pg = reinterpret_cast<double *>(s.list), *ph = pg + CAP;
+        const int *piv = s.piv;
+        if (lane == 0)
             for (int k = 0; k < len; ++k)
                 if (piv[k] != k) {
                     const double t = g[k];
                     g[k] = g[piv[k]];
                     g[piv[k]] = t;
                 }
-            for (int r = 0; r < len; ++r) {
-                double acc = g[r];
-                for (int c = 0; c < r; ++c) acc = __dsub_rn(acc, __dmul_rn(B[r * len + c], g[c]));
-                g[r] = acc;
+        __syncwarp();
+        for (int c = 0; c < len; ++c) {
+            const double gc = g[c], hc = h[c] / B[c * len + c];
+            __syncwarp();
+            if (lane == 0) h[c] = hc;
+            for (int r = c + 1 + lane; r < len; r += 32) {
+                g[r] = __dsub_rn(g[r], __dmul_rn(B[r * len + c], gc));
+                h[r] = __dsub_rn(h[r], __dmul_rn(B[c * len + r], hc));
             }
-            for (int r = len - 1; r >= 0; --r) {
-                double acc = g[r];
-                for (int c = r + 1; c < len; ++c) acc = __dsub_rn(acc, __dmul_rn(B[r * len + c], g[c]));
-                g[r] = acc / B[r * len + r];
+            __syncwarp();
+        }
+        for (int r = len - 1; r >= 0; --r) {
+            for (int c = r + 1 + lane; c < len; c += 32) {
+                pg[c] = __dmul_rn(B[r * len + c], g[c]);
+                ph[c] = __dmul_rn(B[c * len + r], h[c]);
             }
-            // B^T h = h (lu_solve_t)
-            for (int r = 0; r < len; ++r) {
-                double acc = h[r];
-                for (int c = 0; c < r; ++c) acc = __dsub_rn(acc, __dmul_rn(B[c * len + r], h[c]));
-                h[r] = acc / B[r * len + r];
+            __syncwarp();
+            if (lane < 2) {
+                const double *p = lane ? ph : pg;
+                double acc = lane ? h[r] : g[r];
+                int c = r + 1;
+                for (; c + 4 <= len; c += 4) {
+                    double q[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) q[u] = p[c + u];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) acc = __dsub_rn(acc, q[u]);
+                }
+                for (; c < len; ++c) acc = __dsub_rn(acc, p[c]);
+                if (lane) h[r] = acc;
+                else g[r] = acc / B[r * len + r];
             }
-            for (int r = len - 1; r >= 0; --r) {
-                double acc = h[r];
-                for (int c = r + 1; c < len; ++c) acc = __dsub_rn(acc, __dmul_rn(B[c * len + r], h[c]));
-                h[r] = acc;
-            }
+            __syncwarp();
+        }
+        if (lane == 0)
             for (int k = len - 1; k >= 0; --k)
                 if (piv[k] != k) {
                     const double t = h[k];
                     h[k] = h[piv[k]];
                     h[piv[k]] = t;
                 }
-        }
         __syncwarp();
     }
 };
@@ -214,7 +268,7 @@ __device__ double filter_norm(char filttype, const double *x, int len) {
 }
 
 // Rows rows[0..nrows) (or 1..n-1 when rows == NULL), one warp each.
-template <int CAP, bool WRITE>
+template <int CAP>
 static __global__ void __launch_bounds__(256)
 k_pdfiim_rows(int n, const int *__restrict__ rows, int nrows, CsrD A, CsrD At, Params P, Out o) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -273,22 +327,13 @@ k_pdfiim_rows(int n, const int *__restrict__ rows, int nrows, CsrD A, CsrD At, P
                 if (s.B[j * len + j] == 0.0) s.B[j * len + j] = floor_diag;
             }
             __syncwarp();
-            if (lane == 0) {   // g from A^T row i, h from A row i, in storage order
-                for (int kk = At.rp[i]; kk < At.rp[i + 1]; ++kk)
-                    if (At.ci[kk] < i) {
-                        const int q = rb.pos_of(At.ci[kk], len);
-                        if (q >= 0) s.g[q] = -At.v[kk];
-                    }
-                for (int kk = A.rp[i]; kk < A.rp[i + 1]; ++kk)
-                    if (A.ci[kk] < i) {
-                        const int q = rb.pos_of(A.ci[kk], len);
-                        if (q >= 0) s.h[q] = -A.v[kk];
-                    }
-            }
+            rb.assemble(At, s.g, len);   // g from A^T row i, h from A row i
+            rb.assemble(A, s.h, len);
             __syncwarp();
             rb.factor_solve(len);
-            ng = __shfl_sync(0xffffffffu, lane == 0 ? filter_norm(P.filttype, s.g, len) : 0.0, 0);
-            nh = __shfl_sync(0xffffffffu, lane == 0 ? filter_norm(P.filttype, s.h, len) : 0.0, 0);
+            const double norm = lane < 2 ? filter_norm(P.filttype, lane ? s.h : s.g, len) : 0.0;
+            ng = __shfl_sync(0xffffffffu, norm, 0);
+            nh = __shfl_sync(0xffffffffu, norm, 1);
             // New set: kept g entries in order, then kept h entries not yet in it.
             rb.size = 0;
             int c = 0, c2 = 0;
@@ -332,7 +377,7 @@ k_pdfiim_rows(int n, const int *__restrict__ rows, int nrows, CsrD A, CsrD At, P
             if (rb.size == kept) break;
         }
         if (rb.over) {
-            if (!WRITE && lane == 0) o.overflow[atomicAdd(o.noverflow, 1)] = i;
+            if (lane == 0) o.overflow[atomicAdd(o.noverflow, 1)] = i;
             __syncwarp();
             continue;
         }
@@ -357,61 +402,247 @@ k_pdfiim_rows(int n, const int *__restrict__ rows, int nrows, CsrD A, CsrD At, P
             }
             cnt[which] = kc;
             __syncwarp();
-            if (WRITE) {
-                const long off = which == 0 ? o.goff[i] : o.hoff[i];
-                int *oj = which == 0 ? o.gj : o.hj;
-                double *ov = which == 0 ? o.gv : o.hv;
-                for (int j = lane; j < tlen; j += 32)
-                    if (s.rank[j] >= 0) {
-                        oj[off + s.rank[j]] = s.inds[j];
-                        ov[off + s.rank[j]] = x[j];
+            if (which == 0)   // the ranks are used below: g's aside, in the list
+                for (int j = lane; j < tlen; j += 32) s.list[j] = s.rank[j];
+            __syncwarp();
+        }
+        // Entries to the next free places: g's and h's kept ones, each with its unit diagonal.
+        const int gn = cnt[0] + 1, hn = cnt[1] + 1;
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(o.used, (unsigned long long)(gn + hn));
+        at = __shfl_sync(0xffffffffu, at, 0);
+        if (lane == 0) {
+            o.gcnt[i] = gn;
+            o.hcnt[i] = hn;
+            o.at[i] = (long)at;
+        }
+        if (at + gn + hn > o.room) {   // counted; the host makes room and runs the rows again
+            __syncwarp();
+            continue;
+        }
+        for (int which = 0; which < 2; ++which) {
+            const double *x = which == 0 ? s.g : s.h;
+            const int *rank = which == 0 ? s.list : s.rank;
+            const long off = (long)at + (which == 0 ? 0 : gn);
+            for (int j = lane; j < tlen; j += 32)
+                if (rank[j] >= 0) {
+                    o.ej[off + rank[j]] = s.inds[j];
+                    o.ev[off + rank[j]] = x[j];
+                }
+            if (lane == 0) {
+                o.ej[off + cnt[which]] = i;
+                o.ev[off + cnt[which]] = 1.0;
+            }
+        }
+        __syncwarp();
+        // D^{-1}_i = 1 / sum_j h_j (A g)_j over the kept patterns (parPrec.cpp:502-532): each lane
+        // takes entries of h, walks the row of A beside g's sorted entries and leaves its products
+        // where the sequential sum takes them; one lane adds them.
+        const int *gj = o.ej + at, *hj = gj + gn;
+        const double *gv = o.ev + at, *hv = gv + gn;
+        auto walk = [&](int j, auto hit) {
+            const int hr = hj[j], end = A.rp[hr + 1];
+            int kk = A.rp[hr], cc = 0;
+            while (kk < end && cc < gn) {
+                const int c = A.ci[kk], gc = gj[cc];
+                if (c == gc) hit(kk, cc);
+                if (c <= gc) ++kk;
+                if (c >= gc) ++cc;
+            }
+        };
+        double sum = 0.0;
+        for (int base = 0; base < hn; base += 32) {
+            const int j = base + lane;
+            int hits = 0;
+            if (j < hn) walk(j, [&](int, int) { ++hits; });
+            int before = hits;
+            for (int q = 1; q < 32; q <<= 1) {
+                const int u = __shfl_up_sync(0xffffffffu, before, q);
+                if (lane >= q) before += u;
+            }
+            const int all = __shfl_sync(0xffffffffu, before, 31);
+            before -= hits;
+            const bool fits = all <= CAP * CAP;   // B is free by now
+            if (fits && j < hn) {
+                const double hvj = hv[j];
+                int put = before;
+                walk(j, [&](int kk, int cc) { s.B[put++] = __dmul_rn(__dmul_rn(hvj, A.v[kk]), gv[cc]); });
+            }
+            __syncwarp();
+            if (lane == 0) {
+                if (fits) {
+                    for (int q = 0; q < all; ++q) sum = __dadd_rn(sum, s.B[q]);
+                } else {
+                    for (int jj = base; jj < min(base + 32, hn); ++jj) {
+                        const double hvj = hv[jj];
+                        walk(jj, [&](int kk, int cc) {
+                            sum = __dadd_rn(sum, __dmul_rn(__dmul_rn(hvj, A.v[kk]), gv[cc]));
+                        });
                     }
-                if (lane == 0) {
-                    oj[off + kc] = i;
-                    ov[off + kc] = 1.0;
                 }
             }
             __syncwarp();
         }
-        if (!WRITE) {
-            if (lane == 0) {
-                o.gcnt[i] = cnt[0] + 1;
-                o.hcnt[i] = cnt[1] + 1;
-            }
-        } else if (lane == 0) {
-            // D^{-1}_i = 1 / sum_j h_j (A g)_j over the kept patterns (parPrec.cpp:502-532).
-            const long go = o.goff[i], ho = o.hoff[i];
-            const int gn = cnt[0] + 1, hn = cnt[1] + 1;
-            double sum = 0.0;
-            for (int j = 0; j < hn; ++j) {
-                const int hr = o.hj[ho + j];
-                const double hvj = o.hv[ho + j];
-                int kk = A.rp[hr], cc = 0;
-                while (kk < A.rp[hr + 1] && cc < gn) {
-                    const int gc = o.gj[go + cc];
-                    if (A.ci[kk] == gc) {
-                        sum = __dadd_rn(sum, __dmul_rn(__dmul_rn(hvj, A.v[kk]), o.gv[go + cc]));
-                        ++kk;
-                        ++cc;
-                    } else if (A.ci[kk] < gc) {
-                        ++kk;
-                    } else {
-                        ++cc;
-                    }
-                }
-            }
-            o.D[i] = 1.0 / sum;
-        }
+        if (lane == 0) o.D[i] = 1.0 / sum;
         __syncwarp();
     }
 }
 
-template <int CAP, bool WRITE>
+// ---------------------------------------------------------------- transposes and offsets
+// Counts, then their running totals over chunks of kScan (chunk sums, the sums' totals in one
+// CTA, the chunks again), then entries to their rows in whatever order the threads arrive, then
+// each row's entries to their ranks: the order a sequential counting sort gives.
+constexpr int kScan = 4 * 1024;
+
+static __global__ void __launch_bounds__(kThreads) k_count(long nnz, const int *__restrict__ c, int *cnt) {
+    FIIM_FOR_ROWS(k, nnz) { atomicAdd(cnt + c[k], 1); }
+}
+
+__device__ __forceinline__ long block_scan(long v, long *all) {   // exclusive over 1,024 threads
+    __shared__ long sm[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    long x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+        const long u = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += u;
+    }
+    if (lane == 31) sm[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        long t = sm[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const long u = __shfl_up_sync(0xffffffffu, t, o);
+            if (lane >= o) t += u;
+        }
+        sm[lane] = t;
+    }
+    __syncthreads();
+    const long out = x - v + (w ? sm[w - 1] : 0);
+    *all = sm[31];
+    __syncthreads();
+    return out;
+}
+
+// sums[b]: the counts of chunk b.
+static __global__ void __launch_bounds__(1024) k_scan_sums(int n, const int *__restrict__ cnt, long *sums) {
+    long v = 0, all;
+    for (int u = 0; u < 4; ++u) {
+        const long i = (long)blockIdx.x * kScan + threadIdx.x * 4 + u;
+        if (i < n) v += cnt[i];
+    }
+    block_scan(v, &all);
+    if (threadIdx.x == 0) sums[blockIdx.x] = all;
+}
+// sums[b]: the counts before chunk b; sums[nb]: all of them. One CTA.
+static __global__ void __launch_bounds__(1024) k_scan_top(int nb, long *sums) {
+    long base = 0;
+    for (int b0 = 0; b0 < nb; b0 += 1024) {
+        const int b = b0 + (int)threadIdx.x;
+        long all;
+        const long before = block_scan(b < nb ? sums[b] : 0, &all);
+        if (b < nb) sums[b] = base + before;
+        base += all;
+    }
+    if (threadIdx.x == 0) sums[nb] = base;
+}
+// ptr[i], i <= n: the counts before i; next[i] the same, for the scatter (may be null).
+static __global__ void __launch_bounds__(1024)
+k_scan_write(int n, const int *__restrict__ cnt, const long *__restrict__ sums, int *ptr, int *next) {
+    int c[4];
+    long v = 0, all;
+    for (int u = 0; u < 4; ++u) {
+        const long i = (long)blockIdx.x * kScan + threadIdx.x * 4 + u;
+        c[u] = i < n ? cnt[i] : 0;
+        v += c[u];
+    }
+    long at = sums[blockIdx.x] + block_scan(v, &all);
+    for (int u = 0; u < 4; ++u) {
+        const long i = (long)blockIdx.x * kScan + threadIdx.x * 4 + u;
+        if (i < n) {
+            ptr[i] = (int)at;
+            if (next) next[i] = (int)at;
+        }
+        at += c[u];
+        if (i == n - 1) ptr[n] = (int)at;
+    }
+}
+
+// Entries of a CSR matrix to their columns' lists: (position in the matrix, row).
+static __global__ void __launch_bounds__(kThreads)
+k_to_columns(int n, const int *__restrict__ rp, const int *__restrict__ ci, int *next, int *key, int *row) {
+    FIIM_FOR_ROWS(r, n) {
+        for (int k = rp[r]; k < rp[r + 1]; ++k) {
+            const int q = atomicAdd(next + ci[k], 1);
+            key[q] = k;
+            row[q] = (int)r;
+        }
+    }
+}
+// Task i's g entries (rows ej, column i) counted by row, and then to their rows' lists.
+static __global__ void __launch_bounds__(kThreads) k_count_g(int n, Out o, int *cnt) {
+    FIIM_FOR_ROWS(i, n) {
+        for (int q = 0; q < o.gcnt[i]; ++q) atomicAdd(cnt + o.ej[o.at[i] + q], 1);
+    }
+}
+static __global__ void __launch_bounds__(kThreads) k_g_to_rows(int n, Out o, int *next, int *key, double *val) {
+    FIIM_FOR_ROWS(i, n) {
+        for (int q = 0; q < o.gcnt[i]; ++q) {
+            const int at = atomicAdd(next + o.ej[o.at[i] + q], 1);
+            key[at] = (int)i;
+            val[at] = o.ev[o.at[i] + q];
+        }
+    }
+}
+// Task i's h entries are row i of H.
+static __global__ void __launch_bounds__(kThreads) k_h_rows(int n, Out o, const int *__restrict__ Hi, int *Hj, double *Hv) {
+    const int lane = (int)threadIdx.x & 31;
+    for (long i = ((long)blockIdx.x * kThreads + threadIdx.x) >> 5; i < n; i += ((long)gridDim.x * kThreads) >> 5)
+        for (int q = lane; q < o.hcnt[i]; q += 32) {
+            Hj[Hi[i] + q] = o.ej[o.at[i] + o.gcnt[i] + q];
+            Hv[Hi[i] + q] = o.ev[o.at[i] + o.gcnt[i] + q];
+        }
+}
+// The lists ptr[c] .. ptr[c + 1] to ascending keys (distinct within a list): entry q moves to the
+// place its key has among the list's. val null: the value is vals[key]. A warp per list; lists past
+// kLong are noted for k_rank_long, where every thread of the grid takes entries.
+constexpr int kLong = 1024;
+struct Lists {
+    const int *ptr, *key, *idx;      // idx: what goes to oj (may be key)
+    const double *val, *vals;
+    int *oj;
+    double *ov;
+};
+__device__ __forceinline__ void place(const Lists &l, int b, int e, int q) {
+    const int key = l.key[q];
+    int rank = 0;
+    for (int p = b; p < e; ++p) rank += l.key[p] < key;
+    l.oj[b + rank] = l.idx[q];
+    l.ov[b + rank] = l.val ? l.val[q] : l.vals[key];
+}
+static __global__ void __launch_bounds__(kThreads) k_rank(int n, Lists l, int *longs, int *nlongs) {
+    const int lane = (int)threadIdx.x & 31;
+    for (long c = ((long)blockIdx.x * kThreads + threadIdx.x) >> 5; c < n; c += ((long)gridDim.x * kThreads) >> 5) {
+        const int b = l.ptr[c], e = l.ptr[c + 1];
+        if (e - b > kLong) {
+            if (lane == 0) longs[atomicAdd(nlongs, 1)] = (int)c;
+            continue;
+        }
+        for (int q = b + lane; q < e; q += 32) place(l, b, e, q);
+    }
+}
+static __global__ void __launch_bounds__(kThreads) k_rank_long(Lists l, const int *__restrict__ longs, const int *nlongs) {
+    for (int k = 0; k < *nlongs; ++k) {
+        const int b = l.ptr[longs[k]], e = l.ptr[longs[k] + 1];
+        FIIM_FOR_ROWS(t, e - b) { place(l, b, e, b + (int)t); }
+    }
+}
+
+template <int CAP>
 int launch_rows(int n, const int *rows, int nrows, const CsrD &A, const CsrD &At, const Params &P, const Out &o,
                 cudaStream_t st) {
     constexpr int warps = CAP <= 32 ? 8 : (CAP <= 64 ? 4 : 1);
     constexpr size_t smem = sizeof(WarpSmem<CAP>) * warps;
-    auto kern = k_pdfiim_rows<CAP, WRITE>;
+    auto kern = k_pdfiim_rows<CAP>;
     FIIM_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     FIIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * warps, smem));
@@ -423,57 +654,85 @@ int launch_rows(int n, const int *rows, int nrows, const CsrD &A, const CsrD &At
     return FIIM_OK;
 }
 
-struct DevBuf {
-    std::vector<void *> ptrs;
-    template <typename T>
-    T *get(size_t count) {
-        void *p = nullptr;
-        if (cudaMalloc(&p, sizeof(T) * std::max<size_t>(count, 1)) != cudaSuccess) {
-            cudaGetLastError();
-            return nullptr;
-        }
-        ptrs.push_back(p);
-        return static_cast<T *>(p);
+// One device allocation carved into pieces.
+struct Slab {
+    char *p = nullptr;
+    size_t used = 0;
+    Slab() = default;
+    Slab(const Slab &) = delete;
+    Slab &operator=(const Slab &) = delete;
+    ~Slab() { release(); }
+    void release() {
+        if (p) cudaFree(p);
+        p = nullptr;
+        used = 0;
     }
-    ~DevBuf() {
-        for (void *p : ptrs) cudaFree(p);
+    int reserve(size_t bytes) {
+        release();
+        if (cudaMalloc(&p, bytes) == cudaSuccess) return FIIM_OK;
+        cudaGetLastError();
+        p = nullptr;
+        return set_error(FIIM_ENOMEM, "device allocation of %zu bytes for the factor construction failed", bytes);
+    }
+    template <typename T>
+    static size_t need(size_t count) {
+        return Arena::need(sizeof(T) * std::max<size_t>(count, 1));
+    }
+    template <typename T>
+    T *take(size_t count) {
+        char *at = p + used;
+        used += need<T>(count);
+        return reinterpret_cast<T *>(at);
     }
 };
 
+// Factors built by the thread's last first call, on the device until the second call copies them
+// out (or another first call replaces them).
 struct BuiltGpu {
-    int n = 0;
-    std::vector<int> Gi, Gj, Hi, Hj;
-    std::vector<double> Gv, Hv, D;
+    int n = 0, device = -1;
+    long nG = 0, nH = 0;
+    Slab mem;
+    int *Gi = nullptr, *Gj = nullptr, *Hi = nullptr, *Hj = nullptr;
+    double *Gv = nullptr, *Hv = nullptr, *D = nullptr;
+    void clear() {
+        mem.release();
+        n = 0;
+    }
 };
 thread_local BuiltGpu g_built_gpu;
 
 constexpr int kCaps[3] = {32, 64, 128};
 
-template <bool WRITE>
 int run_cap(int cap, int n, const int *rows, int nrows, const CsrD &A, const CsrD &At, const Params &P, const Out &o,
             cudaStream_t st) {
-    if (cap == 32) return launch_rows<32, WRITE>(n, rows, nrows, A, At, P, o, st);
-    if (cap == 64) return launch_rows<64, WRITE>(n, rows, nrows, A, At, P, o, st);
-    return launch_rows<128, WRITE>(n, rows, nrows, A, At, P, o, st);
+    if (cap == 32) return launch_rows<32>(n, rows, nrows, A, At, P, o, st);
+    if (cap == 64) return launch_rows<64>(n, rows, nrows, A, At, P, o, st);
+    return launch_rows<128>(n, rows, nrows, A, At, P, o, st);
+}
+
+// ptr[0..n] (and next, if not null) from cnt[0..n) on st; sums: n / kScan + 2 longs of scratch.
+int scan(int n, const int *cnt, long *sums, int *ptr, int *next, cudaStream_t st) {
+    const int nb = (n + kScan - 1) / kScan;
+    k_scan_sums<<<nb, 1024, 0, st>>>(n, cnt, sums);
+    k_scan_top<<<1, 1024, 0, st>>>(nb, sums);
+    k_scan_write<<<nb, 1024, 0, st>>>(n, cnt, sums, ptr, next);
+    FIIM_CUDA(cudaGetLastError());
+    return FIIM_OK;
+}
+
+int rank_lists(int n, const Lists &l, int *longs, int *nlongs, cudaStream_t st) {
+    FIIM_CUDA(cudaMemsetAsync(nlongs, 0, sizeof(int), st));
+    k_rank<<<grid_for(k_rank, kWarps, n), kThreads, 0, st>>>(n, l, longs, nlongs);
+    k_rank_long<<<num_sms(), kThreads, 0, st>>>(l, longs, nlongs);
+    FIIM_CUDA(cudaGetLastError());
+    return FIIM_OK;
 }
 
 int build_gpu(int n, const int *Ai, const int *Aj, const double *Av, const Params &P, BuiltGpu &out) {
-    FIIM_TRY(check_device(nullptr));
+    out.clear();
+    int dev = -1;
+    FIIM_TRY(check_device(&dev));
     const long nnz = Ai[n];
-    // A^T by counting sort (columns ascend within each row), as the host construction.
-    std::vector<int> tp(n + 1, 0), tc(std::max<long>(nnz, 1));
-    std::vector<double> tv(std::max<long>(nnz, 1));
-    for (long k = 0; k < nnz; ++k) tp[Aj[k] + 1]++;
-    for (int r = 0; r < n; ++r) tp[r + 1] += tp[r];
-    {
-        std::vector<int> pos(tp.begin(), tp.end() - 1);
-        for (int r = 0; r < n; ++r)
-            for (int k = Ai[r]; k < Ai[r + 1]; ++k) {
-                const int q = pos[Aj[k]]++;
-                tc[q] = r;
-                tv[q] = Av[k];
-            }
-    }
     cudaStream_t st = nullptr;
     FIIM_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     struct StreamGuard {
@@ -482,119 +741,137 @@ int build_gpu(int n, const int *Ai, const int *Aj, const double *Av, const Param
             cudaStreamSynchronize(s);
             cudaStreamDestroy(s);
         }
-    } guard{st};
-    DevBuf mem;
-    int *dAi = mem.get<int>(n + 1), *dAj = mem.get<int>(nnz), *dTi = mem.get<int>(n + 1), *dTj = mem.get<int>(nnz);
-    double *dAv = mem.get<double>(nnz), *dTv = mem.get<double>(nnz), *dD = mem.get<double>(n);
-    int *gcnt = mem.get<int>(n), *hcnt = mem.get<int>(n), *ovf = mem.get<int>(n), *novf = mem.get<int>(1);
-    long *goff = mem.get<long>(n), *hoff = mem.get<long>(n);
-    int *rows2 = mem.get<int>(n);
-    if (!dAi || !dAj || !dTi || !dTj || !dAv || !dTv || !dD || !gcnt || !hcnt || !ovf || !novf || !goff || !hoff ||
-        !rows2)
-        return set_error(FIIM_ENOMEM, "device allocation for the factor construction failed");
-    FIIM_CUDA(cudaMemcpyAsync(dAi, Ai, sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st));
-    FIIM_CUDA(cudaMemcpyAsync(dAj, Aj, sizeof(int) * nnz, cudaMemcpyHostToDevice, st));
-    FIIM_CUDA(cudaMemcpyAsync(dAv, Av, sizeof(double) * nnz, cudaMemcpyHostToDevice, st));
-    FIIM_CUDA(cudaMemcpyAsync(dTi, tp.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, st));
-    FIIM_CUDA(cudaMemcpyAsync(dTj, tc.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice, st));
-    FIIM_CUDA(cudaMemcpyAsync(dTv, tv.data(), sizeof(double) * nnz, cudaMemcpyHostToDevice, st));
+    };
+    Slab mem, entries;
+    StreamGuard guard{st};   // after the slabs: synchronized before they go
+    const int nb = (n + kScan - 1) / kScan;
+    FIIM_TRY(mem.reserve(2 * Slab::need<int>(n + 1) + 4 * Slab::need<int>(nnz) + 2 * Slab::need<double>(nnz) +
+                         7 * Slab::need<int>(n) + Slab::need<double>(n) + Slab::need<long>(n) + Slab::need<long>(nb + 1) +
+                         3 * Slab::need<long>(1)));
+    int *dAi = mem.take<int>(n + 1), *dTi = mem.take<int>(n + 1), *dAj = mem.take<int>(nnz), *dTj = mem.take<int>(nnz),
+        *key = mem.take<int>(nnz), *row = mem.take<int>(nnz);
+    double *dAv = mem.take<double>(nnz), *dTv = mem.take<double>(nnz), *dD = mem.take<double>(n);
+    int *gcnt = mem.take<int>(n), *hcnt = mem.take<int>(n), *ovf = mem.take<int>(n), *rows2 = mem.take<int>(n),
+        *cnt = mem.take<int>(n), *next = mem.take<int>(n), *longs = mem.take<int>(n);
+    long *at = mem.take<long>(n), *sums = mem.take<long>(nb + 1);
+    unsigned long long *used = mem.take<unsigned long long>(1);
+    int *novf = mem.take<int>(1), *nlongs = mem.take<int>(1);
+    Stager &stager = thread_stager(dev);
+    FIIM_TRY(stager.copy(dAi, Ai, sizeof(int) * (n + 1), st));
+    if (nnz > 0) {
+        FIIM_TRY(stager.copy(dAj, Aj, sizeof(int) * nnz, st));
+        FIIM_TRY(stager.copy(dAv, Av, sizeof(double) * nnz, st));
+    }
+    // A^T: rows ascend within each column's list.
+    FIIM_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * n, st));
+    k_count<<<grid_for(k_count, kThreads, nnz), kThreads, 0, st>>>(nnz, dAj, cnt);
+    FIIM_TRY(scan(n, cnt, sums, dTi, next, st));
+    k_to_columns<<<grid_for(k_to_columns, kThreads, n), kThreads, 0, st>>>(n, dAi, dAj, next, key, row);
+    FIIM_TRY(rank_lists(n, Lists{dTi, key, row, nullptr, dAv, dTj, dTv}, longs, nlongs, st));
     const CsrD A{dAi, dAj, dAv}, At{dTi, dTj, dTv};
-    Out o{gcnt, hcnt, dD, goff, hoff, nullptr, nullptr, nullptr, nullptr, ovf, novf};
-    // Pass 1: counts; rows that outgrow a CAP are run again at the next one.
-    std::vector<std::vector<int>> pending(3);   // rows each larger CAP serves
-    {
+    // Every row's entries and D^{-1}, in one pass: they go to the next free places, which are then
+    // put in order. Room for four entries per entry of A and row; a construction that keeps more is
+    // counted, given exactly what it needs, and run again.
+    Out o{gcnt, hcnt, dD, at, nullptr, nullptr, used, 0, ovf, novf};
+    unsigned long long room = 4ULL * (unsigned long long)(nnz + n), asked = 0;
+    for (;;) {
+        FIIM_TRY(entries.reserve(Slab::need<int>(room) + Slab::need<double>(room)));
+        o.ej = entries.take<int>(room);
+        o.ev = entries.take<double>(room);
+        o.room = room;
+        const unsigned long long two = 2;   // row 0: the unit entries of g and h
+        const int one = 1, zero[2] = {0, 0};
+        const double unit[2] = {1.0, 1.0}, d0 = 1.0 / Av[0];   // D = 1 / (first stored entry of row 0)
+        const long at0 = 0;
+        FIIM_CUDA(cudaMemcpyAsync(used, &two, sizeof two, cudaMemcpyHostToDevice, st));
+        FIIM_CUDA(cudaMemcpyAsync(gcnt, &one, sizeof one, cudaMemcpyHostToDevice, st));
+        FIIM_CUDA(cudaMemcpyAsync(hcnt, &one, sizeof one, cudaMemcpyHostToDevice, st));
+        FIIM_CUDA(cudaMemcpyAsync(at, &at0, sizeof at0, cudaMemcpyHostToDevice, st));
+        FIIM_CUDA(cudaMemcpyAsync(o.ej, zero, sizeof zero, cudaMemcpyHostToDevice, st));
+        FIIM_CUDA(cudaMemcpyAsync(o.ev, unit, sizeof unit, cudaMemcpyHostToDevice, st));
+        FIIM_CUDA(cudaMemcpyAsync(dD, &d0, sizeof d0, cudaMemcpyHostToDevice, st));
         const int *rows = nullptr;
         int nrows = n - 1;
-        std::vector<int> h_rows;
-        for (int c = 0; c < 3 && n > 1; ++c) {
+        for (int c = 0; c < 3 && n > 1; ++c) {   // rows that outgrow a CAP run again at the next one
             FIIM_CUDA(cudaMemsetAsync(novf, 0, sizeof(int), st));
-            FIIM_TRY(run_cap<false>(kCaps[c], n, rows, nrows, A, At, P, o, st));
+            FIIM_TRY(run_cap(kCaps[c], n, rows, nrows, A, At, P, o, st));
             int no = 0;
             FIIM_CUDA(cudaMemcpyAsync(&no, novf, sizeof(int), cudaMemcpyDeviceToHost, st));
             FIIM_CUDA(cudaStreamSynchronize(st));
-            if (c > 0) pending[c] = h_rows;
             if (no == 0) break;
-            h_rows.resize(no);
-            FIIM_CUDA(cudaMemcpy(h_rows.data(), ovf, sizeof(int) * no, cudaMemcpyDeviceToHost));
-            std::sort(h_rows.begin(), h_rows.end());
+            std::vector<int> left(no);
+            FIIM_CUDA(cudaMemcpy(left.data(), ovf, sizeof(int) * no, cudaMemcpyDeviceToHost));
+            std::sort(left.begin(), left.end());
             if (c == 2)
                 return set_error(FIIM_EARG, "row %d's pattern outgrows %d members; use the host construction "
-                                            "(fiim_pdfiim_build) or a warpsize cap", h_rows[0], kCaps[2]);
-            FIIM_CUDA(cudaMemcpy(rows2, h_rows.data(), sizeof(int) * no, cudaMemcpyHostToDevice));
+                                            "(fiim_pdfiim_build) or a warpsize cap", left[0], kCaps[2]);
+            FIIM_CUDA(cudaMemcpy(rows2, left.data(), sizeof(int) * no, cudaMemcpyHostToDevice));
             rows = rows2;
             nrows = no;
         }
+        FIIM_CUDA(cudaMemcpyAsync(&asked, used, sizeof asked, cudaMemcpyDeviceToHost, st));
+        FIIM_CUDA(cudaStreamSynchronize(st));
+        if (asked <= room) break;
+        room = asked;
     }
-    // Offsets on the host; row 0 is the unit row with D = 1 / (first stored entry of row 0).
-    std::vector<int> hg(n, 1), hh(n, 1);
-    if (n > 1) {
-        FIIM_CUDA(cudaMemcpy(hg.data() + 1, gcnt + 1, sizeof(int) * (n - 1), cudaMemcpyDeviceToHost));
-        FIIM_CUDA(cudaMemcpy(hh.data() + 1, hcnt + 1, sizeof(int) * (n - 1), cudaMemcpyDeviceToHost));
-    }
-    std::vector<long> go(n), ho(n);
-    long tg = 0, th = 0;
-    for (int i = 0; i < n; ++i) {
-        go[i] = tg;
-        ho[i] = th;
-        tg += hg[i];
-        th += hh[i];
-    }
-    if (tg > 0x7fffffffL || th > 0x7fffffffL) return set_error(FIIM_EARG, "factors too large for int32 CSR");
-    int *dgj = mem.get<int>(tg), *dhj = mem.get<int>(th);
-    double *dgv = mem.get<double>(tg), *dhv = mem.get<double>(th);
-    if (!dgj || !dhj || !dgv || !dhv) return set_error(FIIM_ENOMEM, "device allocation for the factors failed");
-    FIIM_CUDA(cudaMemcpyAsync(goff, go.data(), sizeof(long) * n, cudaMemcpyHostToDevice, st));
-    FIIM_CUDA(cudaMemcpyAsync(hoff, ho.data(), sizeof(long) * n, cudaMemcpyHostToDevice, st));
-    o.gj = dgj;
-    o.hj = dhj;
-    o.gv = dgv;
-    o.hv = dhv;
-    // Pass 2: write, every row at the CAP that served it (a row over a CAP skips there).
-    if (n > 1) {
-        FIIM_TRY(run_cap<true>(kCaps[0], n, nullptr, n - 1, A, At, P, o, st));
-        for (int c = 1; c < 3; ++c)
-            if (!pending[c].empty()) {
-                FIIM_CUDA(cudaMemcpyAsync(rows2, pending[c].data(), sizeof(int) * pending[c].size(),
-                                          cudaMemcpyHostToDevice, st));
-                FIIM_TRY(run_cap<true>(kCaps[c], n, rows2, (int)pending[c].size(), A, At, P, o, st));
-                FIIM_CUDA(cudaStreamSynchronize(st));
-            }
-    }
-    std::vector<int> gj(tg), hj(th);
-    std::vector<double> gv(tg), hv(th);
-    out.D.resize(n);
-    FIIM_CUDA(cudaMemcpyAsync(gj.data(), dgj, sizeof(int) * tg, cudaMemcpyDeviceToHost, st));
-    FIIM_CUDA(cudaMemcpyAsync(gv.data(), dgv, sizeof(double) * tg, cudaMemcpyDeviceToHost, st));
-    FIIM_CUDA(cudaMemcpyAsync(hj.data(), dhj, sizeof(int) * th, cudaMemcpyDeviceToHost, st));
-    FIIM_CUDA(cudaMemcpyAsync(hv.data(), dhv, sizeof(double) * th, cudaMemcpyDeviceToHost, st));
-    FIIM_CUDA(cudaMemcpyAsync(out.D.data(), dD, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
+    // H: the tasks' h lists one after another; G: the tasks' g lists, columns, turned into rows.
+    const size_t cap = (size_t)asked;   // entries of G and H together
+    if (cap > 2UL * 0x7fffffffUL) return set_error(FIIM_EARG, "factors too large for int32 CSR");
+    FIIM_TRY(out.mem.reserve(2 * Slab::need<int>(n + 1) + Slab::need<double>(n) + 2 * (Slab::need<int>(cap) + Slab::need<double>(cap))));
+    out.Gi = out.mem.take<int>(n + 1);
+    out.Hi = out.mem.take<int>(n + 1);
+    out.D = out.mem.take<double>(n);
+    long tot[2] = {0, 0};
+    FIIM_TRY(scan(n, hcnt, sums, out.Hi, nullptr, st));
+    FIIM_CUDA(cudaMemcpyAsync(&tot[1], sums + nb, sizeof(long), cudaMemcpyDeviceToHost, st));
     FIIM_CUDA(cudaStreamSynchronize(st));
-    gj[go[0]] = 0;
-    gv[go[0]] = 1.0;
-    hj[ho[0]] = 0;
-    hv[ho[0]] = 1.0;
-    out.D[0] = 1.0 / Av[0];
-    // G: column i holds rows gj of row task i; assemble row-wise CSR (ascending i per row).
-    out.n = n;
-    out.Gi.assign(n + 1, 0);
-    for (long q = 0; q < tg; ++q) out.Gi[gj[q] + 1]++;
-    for (int r = 0; r < n; ++r) out.Gi[r + 1] += out.Gi[r];
-    out.Gj.resize(tg);
-    out.Gv.resize(tg);
-    {
-        std::vector<int> pos(out.Gi.begin(), out.Gi.end() - 1);
-        for (int i = 0; i < n; ++i)
-            for (long q = go[i]; q < go[i] + hg[i]; ++q) {
-                const int at = pos[gj[q]]++;
-                out.Gj[at] = i;
-                out.Gv[at] = gv[q];
-            }
+    tot[0] = (long)asked - tot[1];
+    if (tot[0] > 0x7fffffffL || tot[1] > 0x7fffffffL) {
+        out.clear();
+        return set_error(FIIM_EARG, "factors too large for int32 CSR");
     }
-    out.Hi.assign(n + 1, 0);
-    for (int i = 0; i < n; ++i) out.Hi[i + 1] = out.Hi[i] + hh[i];
-    out.Hj.swap(hj);
-    out.Hv.swap(hv);
+    out.nG = tot[0];
+    out.nH = tot[1];
+    out.Gj = out.mem.take<int>(out.nG);
+    out.Gv = out.mem.take<double>(out.nG);
+    out.Hj = out.mem.take<int>(out.nH);
+    out.Hv = out.mem.take<double>(out.nH);
+    k_h_rows<<<grid_for(k_h_rows, kWarps, n), kThreads, 0, st>>>(n, o, out.Hi, out.Hj, out.Hv);
+    FIIM_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * n, st));
+    k_count_g<<<grid_for(k_count_g, kThreads, n), kThreads, 0, st>>>(n, o, cnt);
+    FIIM_TRY(scan(n, cnt, sums, out.Gi, next, st));
+    Slab lists;
+    FIIM_TRY(lists.reserve(Slab::need<int>(out.nG) + Slab::need<double>(out.nG)));
+    int *gkey = lists.take<int>(out.nG);
+    double *gval = lists.take<double>(out.nG);
+    k_g_to_rows<<<grid_for(k_g_to_rows, kThreads, n), kThreads, 0, st>>>(n, o, next, gkey, gval);
+    FIIM_TRY(rank_lists(n, Lists{out.Gi, gkey, gkey, gval, nullptr, out.Gj, out.Gv}, longs, nlongs, st));
+    FIIM_CUDA(cudaMemcpyAsync(out.D, dD, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
+    FIIM_CUDA(cudaStreamSynchronize(st));
+    out.n = n;
+    out.device = dev;
     return FIIM_OK;
+}
+
+// The second call: straight into the caller's arrays.
+int copy_out(const BuiltGpu &b, double *Gv, int *Gj, int *Gi, double *D, double *Hv, int *Hj, int *Hi) {
+    int was = -1;
+    FIIM_CUDA(cudaGetDevice(&was));
+    FIIM_CUDA(cudaSetDevice(b.device));
+    Stager &stager = thread_stager(b.device);
+    const size_t n = (size_t)b.n, g = (size_t)b.nG, h = (size_t)b.nH;
+    const struct {
+        void *to;
+        const void *from;
+        size_t bytes;
+    } parts[] = {{Gi, b.Gi, sizeof(int) * (n + 1)}, {Gj, b.Gj, sizeof(int) * g}, {Gv, b.Gv, sizeof(double) * g},
+                 {Hi, b.Hi, sizeof(int) * (n + 1)}, {Hj, b.Hj, sizeof(int) * h}, {Hv, b.Hv, sizeof(double) * h},
+                 {D, b.D, sizeof(double) * n}};
+    int rc = FIIM_OK;
+    for (const auto &p : parts)
+        if (rc == FIIM_OK) rc = stager.copy_out(p.to, p.from, p.bytes);
+    cudaSetDevice(was);
+    return rc;
 }
 
 }  // namespace pg
@@ -609,26 +886,19 @@ extern "C" int fiim_pdfiim_build_gpu(int n, const int *Ai, const int *Aj, const 
         if (n <= 0 || !Ai || !Aj || !Av || !nnzG || !nnzH) return fiim::set_error(FIIM_EARG, "null argument or n <= 0");
         if (patt != 'B') return fiim::set_error(FIIM_EARG, "only the two-sided pattern 'B' is served");
         if (warpsize == 0 || warpsize < -1) return fiim::set_error(FIIM_EARG, "warpsize is -1 or positive");
-        g_built_gpu = fiim::pg::BuiltGpu();
         const fiim::pg::Params P{prefill, lfill, postfill, warpsize, ftol, filttype};
         const int rc = fiim::pg::build_gpu(n, Ai, Aj, Av, P, g_built_gpu);
         if (rc != FIIM_OK) {
-            g_built_gpu = fiim::pg::BuiltGpu();
+            g_built_gpu.clear();
             return rc;
         }
-        *nnzG = g_built_gpu.Gi[n];
-        *nnzH = g_built_gpu.Hi[n];
+        *nnzG = (int)g_built_gpu.nG;
+        *nnzH = (int)g_built_gpu.nH;
         return FIIM_OK;
     }
-    if (g_built_gpu.n != n || !Gj || !Gi || !D || !Hv || !Hj || !Hi)
+    if (g_built_gpu.n <= 0 || g_built_gpu.n != n || !Gj || !Gi || !D || !Hv || !Hj || !Hi)
         return fiim::set_error(FIIM_EARG, "call first with Gv == NULL, then with every output");
-    std::memcpy(Gi, g_built_gpu.Gi.data(), sizeof(int) * (n + 1));
-    std::memcpy(Gj, g_built_gpu.Gj.data(), sizeof(int) * g_built_gpu.Gj.size());
-    std::memcpy(Gv, g_built_gpu.Gv.data(), sizeof(double) * g_built_gpu.Gv.size());
-    std::memcpy(Hi, g_built_gpu.Hi.data(), sizeof(int) * (n + 1));
-    std::memcpy(Hj, g_built_gpu.Hj.data(), sizeof(int) * g_built_gpu.Hj.size());
-    std::memcpy(Hv, g_built_gpu.Hv.data(), sizeof(double) * g_built_gpu.Hv.size());
-    std::memcpy(D, g_built_gpu.D.data(), sizeof(double) * n);
-    g_built_gpu = fiim::pg::BuiltGpu();
-    return FIIM_OK;
+    const int rc = fiim::pg::copy_out(g_built_gpu, Gv, Gj, Gi, D, Hv, Hj, Hi);
+    g_built_gpu.clear();
+    return rc;
 }

@@ -432,42 +432,81 @@ void signature(DevCsr &M, const int *host_rp) {
 // fill 1 keeps col >= row, fill 2 keeps col <= row (AFIIM/src/bicgstab.cpp:140-147). The check
 // runs on the device; the rare matrix with entries outside its triangle is compacted on the
 // host. A caller uploading several matrices issues every copy and check before one sync.
-int Stager::copy(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+bool Stager::ready() {
+    if (buf[0]) return true;
+    for (int k = 0; k < kBufs; ++k)
+        if (cudaHostAlloc(&buf[k], kChunk, cudaHostAllocPortable) != cudaSuccess ||
+            cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming) != cudaSuccess) {
+            cudaGetLastError();
+            release();
+            return false;
+        }
+    return true;
+}
+
+static bool pageable(const void *p) {
     cudaPointerAttributes attr{};
-    const bool pageable = cudaPointerGetAttributes(&attr, src) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
+    const bool yes = cudaPointerGetAttributes(&attr, p) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
-    if (!pageable || bytes < kMinStaged) {
+    return yes;
+}
+
+static void copy_parallel(void *to, const void *from, size_t len) {
+    const long parts = (long)((len + (size_t(1) << 19) - 1) >> 19);
+#pragma omp parallel for schedule(static)
+    for (long q = 0; q < parts; ++q) {
+        const size_t a = (size_t)q << 19, e = std::min(len, a + (size_t(1) << 19));
+        std::memcpy(static_cast<char *>(to) + a, static_cast<const char *>(from) + a, e - a);
+    }
+}
+
+int Stager::copy(void *dst, const void *src, size_t bytes, cudaStream_t s) {
+    if (bytes < kMinStaged || !pageable(src) || !ready()) {
         FIIM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));
         return FIIM_OK;
     }
-    if (!buf[0]) {
-        for (int k = 0; k < kBufs; ++k) {
-            if (cudaHostAlloc(&buf[k], kChunk, cudaHostAllocDefault) != cudaSuccess) {
-                cudaGetLastError();
-                release();
-                FIIM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s));   // no pinned memory
-                return FIIM_OK;
-            }
-            FIIM_CUDA(cudaEventCreateWithFlags(&ev[k], cudaEventDisableTiming));
-        }
-    }
     const char *in = static_cast<const char *>(src);
-    char *out = static_cast<char *>(dst);
+    char *to = static_cast<char *>(dst);
     for (size_t off = 0; off < bytes; off += kChunk) {
         const size_t len = std::min(kChunk, bytes - off);
         const int k = next;
         next = (next + 1) % kBufs;
         if (pending[k]) FIIM_CUDA(cudaEventSynchronize(ev[k]));   // the buffer's previous DMA
-        char *pb = static_cast<char *>(buf[k]);
-        const long parts = (long)((len + (size_t(1) << 20) - 1) >> 20);
-#pragma omp parallel for schedule(static)
-        for (long q = 0; q < parts; ++q) {
-            const size_t a = (size_t)q << 20, e = std::min(len, a + (size_t(1) << 20));
-            std::memcpy(pb + a, in + off + a, e - a);
-        }
-        FIIM_CUDA(cudaMemcpyAsync(out + off, pb, len, cudaMemcpyHostToDevice, s));
+        copy_parallel(buf[k], in + off, len);
+        FIIM_CUDA(cudaMemcpyAsync(to + off, buf[k], len, cudaMemcpyHostToDevice, s));
         FIIM_CUDA(cudaEventRecord(ev[k], s));
         pending[k] = true;
+    }
+    return FIIM_OK;
+}
+
+int Stager::copy_out(void *dst, const void *src, size_t bytes) {
+    if (!out) FIIM_CUDA(cudaStreamCreateWithFlags(&out, cudaStreamNonBlocking));
+    if (bytes < kMinStaged || !pageable(dst) || !ready()) {
+        FIIM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, out));
+        FIIM_CUDA(cudaStreamSynchronize(out));
+        return FIIM_OK;
+    }
+    const char *from = static_cast<const char *>(src);
+    char *to = static_cast<char *>(dst);
+    const size_t chunks = (bytes + kChunk - 1) / kChunk;
+    size_t issued = 0;
+    int slot[kBufs];
+    for (size_t done = 0; done < chunks; ++done) {
+        for (; issued < chunks && issued < done + kBufs; ++issued) {
+            const int k = slot[issued % kBufs] = next;
+            next = (next + 1) % kBufs;
+            if (pending[k]) FIIM_CUDA(cudaEventSynchronize(ev[k]));
+            const size_t off = issued * kChunk;
+            FIIM_CUDA(cudaMemcpyAsync(buf[k], from + off, std::min(kChunk, bytes - off), cudaMemcpyDeviceToHost, out));
+            FIIM_CUDA(cudaEventRecord(ev[k], out));
+            pending[k] = true;
+        }
+        const int k = slot[done % kBufs];
+        const size_t off = done * kChunk;
+        FIIM_CUDA(cudaEventSynchronize(ev[k]));
+        pending[k] = false;
+        copy_parallel(to + off, buf[k], std::min(kChunk, bytes - off));
     }
     return FIIM_OK;
 }
@@ -483,7 +522,14 @@ void Stager::release() {
         buf[k] = nullptr;
         pending[k] = false;
     }
+    if (out) cudaStreamDestroy(out);
+    out = nullptr;
     next = 0;
+}
+
+Stager &thread_stager(int device) {
+    thread_local std::map<int, Stager> rings;   // events belong to a device
+    return rings[device];
 }
 
 int upload_csr_async(DevCsr &M, long nnz_cap, int n, const int *rp, const int *ci, const double *v, bool device_src,
@@ -861,7 +907,7 @@ int Solver::create(int n_, const int *Ai, const int *Aj, const double *Av, const
     FIIM_CUDA(cudaMemsetAsync(fault, 0, sizeof(int), stream));
 
     if (dev_src) FIIM_CUDA(cudaMemcpyAsync(IDv, IDv_, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
-    else FIIM_TRY(stager.copy(IDv, IDv_, sizeof(double) * n, stream));
+    else FIIM_TRY(thread_stager(device).copy(IDv, IDv_, sizeof(double) * n, stream));
     {
         DevCsr *mats[] = {&A, &G, &H, &L, &U};
         const long caps[] = {capA, capG, capH, capL, capU};
@@ -870,7 +916,7 @@ int Solver::create(int n_, const int *Ai, const int *Aj, const double *Av, const
         const int fills[] = {0, 1, 2, 2, 1};
         const bool dev[] = {a_dev, dev_src, h_dev, dev_src, dev_src};
         FIIM_TRY(upload_all(mats, caps, rps, cis, vs, fills, dev, combined ? 5 : 3, n, stream, d_count, h_count,
-                             &stager));
+                             &thread_stager(device)));
     }
 
     DevCsr *mats[] = {&A, &G, &H, &L, &U};
@@ -956,7 +1002,7 @@ int Solver::reload(const int *Ai, const int *Aj, const double *Av, const int *Gi
     const bool combined = (opt.variant == FIIM_ACIFIM && opt.mode == 'C' && opt.nr > 1);
     if (opt.issym) return set_error(FIIM_EARG, "reload does not serve symmetric input");
     if (dev_src) FIIM_CUDA(cudaMemcpyAsync(IDv, IDv_, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
-    else FIIM_TRY(stager.copy(IDv, IDv_, sizeof(double) * n, stream));
+    else FIIM_TRY(thread_stager(device).copy(IDv, IDv_, sizeof(double) * n, stream));
     bool early[5] = {};   // refreshed on `aux` while the copies ran
     if (!aux && dia_wanted()) {
         FIIM_CUDA(cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking));
@@ -978,7 +1024,7 @@ int Solver::reload(const int *Ai, const int *Aj, const double *Av, const int *Gi
             return refresh_dia_async(M, stream, aux, aux_ev[k], h_spec + k);
         };
         const int rc = upload_all(mats, caps, rps, cis, vs, fills, dev, combined ? 5 : 3, n, stream, d_count,
-                                  h_count, &stager, issued);
+                                  h_count, &thread_stager(device), issued);
         if (aux) FIIM_CUDA(cudaStreamSynchronize(aux));
         if (rc != FIIM_OK) return rc;
     }
@@ -1028,8 +1074,8 @@ int Solver::solve_start(const double *b_in, const double *x_in, double tol, int 
         FIIM_CUDA(cudaMemcpyAsync(b, b_in, sizeof(double) * n, in_kind, stream));
         FIIM_CUDA(cudaMemcpyAsync(x, x_in, sizeof(double) * n, in_kind, stream));
     } else {
-        FIIM_TRY(stager.copy(b, b_in, sizeof(double) * n, stream));
-        FIIM_TRY(stager.copy(x, x_in, sizeof(double) * n, stream));
+        FIIM_TRY(thread_stager(device).copy(b, b_in, sizeof(double) * n, stream));
+        FIIM_TRY(thread_stager(device).copy(x, x_in, sizeof(double) * n, stream));
     }
 
     DState h = {};
@@ -1158,8 +1204,8 @@ int Solver::stage_inputs(const double *b_in, const double *x_in) {
         FIIM_CUDA(cudaMemcpyAsync(b, b_in, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
         FIIM_CUDA(cudaMemcpyAsync(x, x_in, sizeof(double) * n, cudaMemcpyDeviceToDevice, stream));
     } else {
-        FIIM_TRY(stager.copy(b, b_in, sizeof(double) * n, stream));
-        FIIM_TRY(stager.copy(x, x_in, sizeof(double) * n, stream));
+        FIIM_TRY(thread_stager(device).copy(b, b_in, sizeof(double) * n, stream));
+        FIIM_TRY(thread_stager(device).copy(x, x_in, sizeof(double) * n, stream));
     }
     inputs_staged = true;
     return FIIM_OK;
@@ -1208,7 +1254,6 @@ void Solver::destroy() {
     h_spec = nullptr;
     if (hst) cudaFreeHost(hst);
     hst = nullptr;
-    stager.release();
     for (DevCsr *M : {&A, &G, &H, &L, &U}) release_dia(*M);
     arena.release();
 }

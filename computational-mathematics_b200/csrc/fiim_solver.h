@@ -54,7 +54,6 @@ struct Solver : SolverBase {
     int solve_start(const double *b, const double *x, double tol, int nmax);
     int solve_finish(double *x_io, fiim_result *res);
     int pending_launches = 0, host_loops = 0;
-    Stager stager;               // host-to-device copies from pageable memory
     // The reference-facing call's reload: b and x0 are copied ahead of the matrices
     // (stage_inputs; the next solve_start then copies no inputs), and each sliced-diagonal
     // copy is refreshed on the second stream `aux` while the later matrices' copies run.
