@@ -136,21 +136,38 @@ struct RowBuilder {
         for (int k = 0; k < len; ++k) {
             // First row of largest |B(r, k)|, r >= k, as a sequential scan from r = k finds it
             // (a NaN at (k, k) keeps row k, a NaN below is never taken).
-            double best = -1.0;
             int p = len;
-            for (int r = k + lane; r < len; r += 32) {
-                const double v = fabs(B[r * len + k]);
-                if (v > best) {
-                    best = v;
-                    p = r;
+            if constexpr (CAP <= 32) {
+                // One row a lane: the largest upper word decides, and the lower words only where
+                // several lanes share it (upper words of non-negative doubles order as they do).
+                const double v = lane >= k && lane < len ? fabs(B[lane * len + k]) : nan("");
+                const bool in = !isnan(v);
+                const unsigned hi = in ? (unsigned)__double2hiint(v) : 0u;
+                const unsigned top = __reduce_max_sync(0xffffffffu, hi);   // every lane, before any test
+                unsigned at = __ballot_sync(0xffffffffu, in && hi == top);
+                if (at & (at - 1u)) {   // the same in every lane
+                    const bool tie = at >> lane & 1u;
+                    const unsigned lo = tie ? (unsigned)__double2loint(v) : 0u;
+                    const unsigned low = __reduce_max_sync(0xffffffffu, lo);
+                    at = __ballot_sync(0xffffffffu, tie && lo == low);
                 }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int op = __shfl_xor_sync(0xffffffffu, p, o);
-                if (ob > best || (ob == best && op < p)) {
-                    best = ob;
-                    p = op;
+                if (at) p = __ffs(at) - 1;
+            } else {
+                double best = -1.0;
+                for (int r = k + lane; r < len; r += 32) {
+                    const double v = fabs(B[r * len + k]);
+                    if (v > best) {
+                        best = v;
+                        p = r;
+                    }
+                }
+                for (int o = 16; o > 0; o >>= 1) {
+                    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+                    const int op = __shfl_xor_sync(0xffffffffu, p, o);
+                    if (ob > best || (ob == best && op < p)) {
+                        best = ob;
+                        p = op;
+                    }
                 }
             }
             if (isnan(B[k * len + k])) p = k;
