@@ -966,7 +966,10 @@ int Solver::create(int n_, const int *Ai, const int *Aj, const double *Av, const
             cluster_rows = (n + kClusterCtas - 1) / kClusterCtas;
             const int smem = (int)cluster_smem(cluster_rows);
             FIIM_CUDA(cudaFuncSetAttribute(k_solve_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            FIIM_CUDA(cudaFuncSetAttribute(k_solve_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            // The most any system asks for: the attribute is the process's, and another handle's
+            // smaller value would refuse this one's launches.
+            FIIM_CUDA(cudaFuncSetAttribute(k_solve_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)cluster_smem(kClusterMaxRows)));
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute attr[1];
             attr[0].id = cudaLaunchAttributeClusterDimension;
