@@ -60,19 +60,6 @@ uint64_t content_hash(const void *p, size_t bytes) {
     return acc + mix64(tail ^ 0xd1b54a32d192ed03ULL) + mix64((uint64_t)bytes);
 }
 
-Stamp stamp(const void *p, size_t bytes) { return Stamp{p, bytes, p ? content_hash(p, bytes) : 0}; }
-
-void stamp_csr(std::vector<Stamp> &out, int n, const int *rp, const int *ci, const double *v) {
-    if (!rp) {
-        out.push_back(Stamp{nullptr, 0, 0});
-        return;
-    }
-    const size_t nnz = (size_t)std::max(rp[n], 0);
-    out.push_back(stamp(rp, sizeof(int) * (n + 1)));
-    out.push_back(stamp(ci, sizeof(int) * nnz));
-    out.push_back(stamp(v, sizeof(double) * nnz));
-}
-
 thread_local int g_cache = [] {
     const char *e = std::getenv("FIIM_DROPIN_CACHE");
     return (e && e[0] == '0' && e[1] == 0) ? 0 : 1;
@@ -110,68 +97,83 @@ int oneshot(int variant, int issym, char mode, int nr, int n, const double *Av, 
     std::vector<long> key = {variant, issym, (long)mode, combined ? nr : 1, n, Ai[n], Gi[n],
                              (!issym && Hi) ? Hi[n] : -1, (combined && Li) ? Li[n] : -1,
                              (combined && Ui) ? Ui[n] : -1};
-    int rc = FIIM_OK;
-    std::vector<Stamp> st;
-    auto stamp_all = [&] {
-        stamp_csr(st, n, Ai, Aj, Av);
-        stamp_csr(st, n, Gi, Gj, Gv);
-        stamp_csr(st, n, Hi, Hj, Hv);
-        stamp_csr(st, n, combined ? Li : nullptr, Lj, Lv);
-        stamp_csr(st, n, combined ? Ui : nullptr, Uj, Uv);
-        st.push_back(stamp(IDv, sizeof(double) * n));
+    // The arrays of the call in stamping order: address and size, and the content hash when asked.
+    auto stamps = [&](bool content) {
+        std::vector<Stamp> st;
+        auto add = [&](const void *p, size_t bytes) { st.push_back(Stamp{p, bytes, p && content ? content_hash(p, bytes) : 0}); };
+        auto csr = [&](const int *rp, const int *ci, const double *v) {
+            const size_t nnz = rp ? (size_t)std::max(rp[n], 0) : 0;
+            add(rp, rp ? sizeof(int) * (n + 1) : 0);
+            add(rp ? ci : nullptr, sizeof(int) * nnz);
+            add(rp ? v : nullptr, sizeof(double) * nnz);
+        };
+        csr(Ai, Aj, Av);
+        csr(Gi, Gj, Gv);
+        csr(Hi, Hj, Hv);
+        csr(combined ? Li : nullptr, Lj, Lv);
+        csr(combined ? Ui : nullptr, Uj, Uv);
+        add(IDv, sizeof(double) * n);
+        return st;
     };
     auto report = [&](const fiim_result &r) {
         *resval = r.resval;
         *iter = r.iter;
         if (r.info >= 0) *info = r.info;   // NMAX < 0: the reference leaves info untouched
     };
-    if (g_cache && g_one.s && g_one.key == key && !g_one.stamps.empty()) {
-        // The same shape as the previous call, whose arrays are on the device: start the
-        // solve on those copies at once and stamp the arrays while it runs. x is copied back
+    auto same_arrays = [&] {   // the previous call's addresses and sizes
+        const std::vector<Stamp> now = stamps(false);
+        return std::equal(now.begin(), now.end(), g_one.stamps.begin(), g_one.stamps.end(),
+                          [](const Stamp &x, const Stamp &y) { return x.p == y.p && x.bytes == y.bytes; });
+    };
+    fiim_result r{};
+    if (g_cache && g_one.s && g_one.key == key && same_arrays()) {
+        // The previous call's arrays by address and size, whose contents are on the device: start
+        // the solve on those copies at once and hash the arrays while it runs. x is copied back
         // only if every stamp still matches; otherwise the result is discarded and the call
-        // uploads the arrays and solves again.
+        // uploads the arrays and solves again. (Arrays at other addresses are uploaded without
+        // trying: a solve on the previous system's copies would be thrown away.)
         g_one.s->opt.verbose = verbose;
         FIIM_TRY(g_one.s->solve_start(b, x, tol, NMAX));
-        stamp_all();
-        if (st == g_one.stamps) {
-            fiim_result r{};
+        if (stamps(true) == g_one.stamps) {
             FIIM_TRY(g_one.s->solve_finish(x, &r));
             report(r);
             return FIIM_OK;
         }
         FIIM_TRY(g_one.s->solve_finish(nullptr, nullptr));
-    } else if (g_cache) {
-        stamp_all();
     }
+    g_one.stamps.clear();
+    int rc = FIIM_OK, dev = -1;
     if (g_one.s && g_one.key == key && !issym) {
-        g_one.stamps.clear();
         g_one.s->opt.verbose = verbose;
         rc = g_one.s->stage_inputs(b, x);   // ahead of the matrix copies
         if (rc == FIIM_OK) rc = g_one.s->reload(Ai, Aj, Av, Gi, Gj, Gv, IDv, Hi, Hj, Hv, Li, Lj, Lv, Ui, Uj, Uv);
-        if (rc == FIIM_OK) g_one.stamps = st;
-        else g_one.s->inputs_staged = false;
+        if (rc != FIIM_OK) g_one.s->inputs_staged = false;
     } else {
-        g_one.stamps.clear();
-        if (g_one.s) {
+        // Another shape: set the thread's solver up again, in the memory, stream and events it has
+        // (on the device it was made on; a thread that moved gets a new one).
+        g_one.key.clear();
+        if (g_one.s && (cudaGetDevice(&dev) != cudaSuccess || dev != g_one.s->device)) {
             g_one.s->destroy();
             delete g_one.s;
             g_one.s = nullptr;
         }
-        auto *s = new fiim::Solver;
+        auto *s = g_one.s ? g_one.s : new fiim::Solver;
         rc = s->create(n, Ai, Aj, Av, Gi, Gj, Gv, IDv, Hi, Hj, Hv, Li, Lj, Lv, Ui, Uj, Uv, o);
         if (rc != FIIM_OK) {
             s->destroy();
             delete s;
+            g_one.s = nullptr;
             return rc;
         }
         g_one.s = s;
         g_one.key = key;
-        g_one.stamps = st;
     }
     if (rc != FIIM_OK) return rc;
-    fiim_result r{};
-    rc = g_one.s->solve(b, x, tol, NMAX, &r);
-    if (rc != FIIM_OK) return rc;
+    FIIM_TRY(g_one.s->solve_start(b, x, tol, NMAX));
+    std::vector<Stamp> now;
+    if (g_cache) now = stamps(true);   // while the solve runs
+    FIIM_TRY(g_one.s->solve_finish(x, &r));
+    g_one.stamps.swap(now);
     report(r);
     return FIIM_OK;
 }

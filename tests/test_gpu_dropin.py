@@ -1,0 +1,73 @@
+"""The reference-facing call over changing systems: one thread's solver is set up again in place for
+another shape and reused for the same one, and every call equals a fresh solver's result bit for
+bit, with the device-copy reuse on and off, from one thread and from several."""
+import threading
+
+import numpy as np
+import pytest
+
+import fiim_b200 as FB
+
+pytestmark = pytest.mark.gpu
+
+
+def system(kind):
+    """Shapes that grow, shrink and change their layout: cluster-sized, mid-sized, symmetric storage."""
+    side, seed = kind
+    A = FB.gen_convdiff3d(side, 0.3 + 0.05 * seed)
+    F = FB.pdfiim_build(A, 0.05, 2, 2, 1)
+    return A, F, FB.rand_normal(side ** 3, seed)
+
+
+KINDS = [(12, 1), (40, 2), (33, 3), (12, 4), (40, 5), (40, 2), (36, 6), (12, 1)]
+
+
+def check(systems):
+    for A, F, b in systems:
+        n = len(b)
+        with FB.Solver(A, F, variant="pdfiim") as S:
+            y = np.zeros(n)
+            r1 = S.solve(b, y, tol=1e-10, nmax=500)
+        x = np.zeros(n)
+        r = FB.EPBiCGSTAB_pdfiim(A, b, 1e-10, 500, (F["Gi"], F["Gj"], F["Gv"]), F["IDv"],
+                                 (F["Hi"], F["Hj"], F["Hv"]), x)
+        assert r[2] == r1["info"] == 0 and r[1] == r1["iter"] and np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("cache", [True, False])
+def test_changing_shapes(cache):
+    prev = FB.dropin_cache(cache)
+    try:
+        check([system(k) for k in KINDS])
+    finally:
+        FB.dropin_cache(prev)
+
+
+def test_same_arrays_other_addresses():
+    """The same system in other arrays, then the first arrays changed in place, then as they were."""
+    A, F, b = system((34, 7))
+    prev = FB.dropin_cache(True)
+    try:
+        copies = (tuple(a.copy() for a in A), {k: v.copy() for k, v in F.items()}, b)
+        check([(A, F, b), copies, (A, F, b)])
+        A[2][7] *= 1.5
+        check([(A, F, b), copies])
+    finally:
+        FB.dropin_cache(prev)
+
+
+def test_threads():
+    errors = []
+
+    def work(seed):
+        try:
+            check([system((20 + 8 * (seed % 3), seed)), system((34, seed)), system((16, seed))])
+        except BaseException as e:   # noqa: BLE001 - reported below
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
