@@ -51,6 +51,7 @@ struct DState {
     int iter, nmax, stag, msteps, maxmsteps, info, done, alpha_guard;
     unsigned int ticket;       // last-block counter, reset by the last block
     int loops;                 // iteration bodies run by the device loop (guard + accounting)
+    int npc;                   // partial sums of ||pc||^2 that EpiNormPart left
 };
 
 template <typename V>
@@ -228,6 +229,35 @@ __device__ __forceinline__ void grid_reduce_pairs(double (&v)[2][NR], int vgrid,
     reduce_partials<NR>(vgrid, partials, sm, st, op);
 }
 
+// An epilogue that declares DEFERS leaves its CTAs' partial sums where they are, for a later
+// launch's last CTA to add (reduce_with): no fence, no ticket and no last CTA at the end of a
+// product whose sum nothing needs yet.
+template <typename E, typename = void>
+struct Defers : std::false_type {};
+template <typename E>
+struct Defers<E, std::void_t<typename E::DEFERS>> : std::true_type {};
+
+// The end of a product's launch: the sums of its epilogue, if it has any.
+template <class Epi>
+__device__ __forceinline__ void end_sums(double (&v)[Epi::NR], double *__restrict__ partials, DState *st, const Epi &epi) {
+    if constexpr (Defers<Epi>::value) {
+        static_assert(Epi::NR == 1, "one deferred sum");
+        __shared__ double sm[kWarps];
+        const double s = warp_sum(v[0]);
+        if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double t = 0.0;
+#pragma unroll
+            for (int k = 0; k < kWarps; ++k) t += sm[k];
+            partials[blockIdx.x] = t;
+            if (blockIdx.x == 0) st->npc = (int)gridDim.x;
+        }
+    } else if constexpr (Epi::REDUCES) {
+        grid_reduce<Epi::NR>(v, partials, st, epi);
+    }
+}
+
 // ---------------------------------------------------------------- scalar steps
 struct FinInit {   // ro = ||r0||, m1 = ro^2, rc = ro (AFIIM/src/bicgstab.cpp:161-165)
     __device__ void finish(DState *st, const double *t) const {
@@ -290,6 +320,12 @@ struct EpiNorm {                   // y = M x, ||y||^2 -> st->pc2 (stagnation te
     __device__ void emit(long i, double s, double (&r)[NR]) const { y[i] = s; r[0] += s * s; }
     __device__ void finish(DState *st, const double *t) const { st->pc2 = t[0]; }
 };
+struct EpiNormPart {               // y = M x, ||y||^2 left as partial sums for FinControlN's launch
+    FIIM_EPI(1, true, true);
+    using DEFERS = void;
+    double *y;
+    __device__ void emit(long i, double s, double (&r)[NR]) const { y[i] = s; r[0] += s * s; }
+};
 struct EpiAlpha {                  // v = A pc, alpha = m1 / (r0 . v)
     FIIM_EPI(1, true, true);
     using STEERS = void;
@@ -348,6 +384,23 @@ struct EpiInit {
     }
     __device__ void finish(DState *st, const double *t) const { FinInit{}.finish(st, t); }
 };
+// The same start for the solver whose x / r update leaves the next iteration's norms
+// (FinControlN): also sum x^2, the first iteration's ||r||^2 and ||x||^2 (:201, :216).
+struct EpiStart : EpiInit {
+    FIIM_EPI(2, true, true);
+    const double *__restrict__ x;
+    __device__ void emit(long i, double s, double (&red)[NR]) const {
+        double r0[1] = {red[0]};
+        EpiInit::emit(i, s, r0);
+        red[0] = r0[0];
+        red[1] += x[i] * x[i];
+    }
+    __device__ void finish(DState *st, const double *t) const {
+        FinInit{}.finish(st, t);
+        st->r2 = t[0];
+        st->x2 = t[1];
+    }
+};
 // True residual r = b - A x in FP64, sum r^2 and sum b^2 -> st->ts, st->tt. Runs after
 // the solve has finished, so it is not gated.
 struct EpiResid {
@@ -390,15 +443,15 @@ struct EpiAccumScale {             // y = (M x) + y; z = y o d (last relaxation 
     }
     __device__ void finish(DState *, const double *) const {}
 };
-struct EpiAccumNorm {              // y = (M x) + y, ||y||^2 -> st->pc2
+struct EpiAccumNorm {              // y = (M x) + y, ||y||^2 left as partial sums (EpiNormPart)
     FIIM_EPI(1, true, true);
+    using DEFERS = void;
     double *y;
     __device__ void emit(long i, double s, double (&r)[NR]) const {
         const double t = __dadd_rn(s, y[i]);
         y[i] = t;
         r[0] += t * t;
     }
-    __device__ void finish(DState *st, const double *t) const { st->pc2 = t[0]; }
 };
 
 // ---------------------------------------------------------------- CSR-stream SpMV
@@ -544,7 +597,7 @@ k_spmv_rows(CsrView<double> M, const int *__restrict__ rb, const int *__restrict
         }
     }
     pdl_release();
-    if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red, partials, st, epi);
+    end_sums(red, partials, st, epi);
 }
 
 // Warp-block form of the CSR-stream SpMV: the same arithmetic as k_spmv_rows (rounded
@@ -643,7 +696,7 @@ k_spmv_warp(CsrView<double> M, const int *__restrict__ rb, const int *__restrict
         }
     }
     pdl_release();
-    if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red, partials, st, epi);
+    end_sums(red, partials, st, epi);
 }
 
 // Narrow column stream for k_spmv_rows: per row block, base = smallest column + 32768 and
@@ -949,7 +1002,7 @@ k_spmv_dia(DiaView<V> M, const T *__restrict__ x, Epi epi, DState *st, double *_
         rec = rec_next;
     }
     pdl_release();
-    if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red, partials, st, epi);
+    end_sums(red, partials, st, epi);
 }
 
 // One slice through a shared record (class c). Lane l owns the rows first + l + 32 j, so every
@@ -1053,7 +1106,7 @@ k_spmv_cls(DiaView<V> M, const T *__restrict__ x, Epi epi, DState *st, double *_
     }
     pdl_release();
     if constexpr (PAIRS) grid_reduce_pairs<Epi::NR>(red, vgrid, partials, st, epi);
-    else if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red[0], partials, st, epi);
+    else end_sums(red[0], partials, st, epi);
 }
 
 // Launches k_spmv_cls over the shared blocks of M (a DevCsr).
@@ -1185,7 +1238,7 @@ k_spmv_pack(PackView M, const double *__restrict__ x, Epi epi, DState *st, doubl
         r = rn;
     }
     pdl_release();
-    if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red, partials, st, epi);
+    end_sums(red, partials, st, epi);
 }
 
 // Launches k_spmv_pack over the packed slices of M (a DevCsr).
@@ -1235,7 +1288,7 @@ k_spmv_vec(CsrView<double> M, const double *__restrict__ x, Epi epi, DState *st,
         }
         if (row < M.n && lir == 0) epi.emit(row, s, red);
     }
-    if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red, partials, st, epi);
+    end_sums(red, partials, st, epi);
 }
 
 // ---------------------------------------------------------------- set-up-free CSR-stream SpMV
@@ -1458,6 +1511,61 @@ k_update_xr(long n, const double *__restrict__ pc, const double *__restrict__ sc
         });
     pdl_release();
     grid_reduce<1>(red, partials, st, fin);
+}
+
+// s = r + (-alpha) v alone, for the solver whose x / r update takes the norms: one read less (x)
+// and no reduction. 128^3 in the body's order: 14.9 us with the norms.
+static __global__ void __launch_bounds__(kThreads)
+k_form_s(long n, const double *__restrict__ r, const double *__restrict__ v, double *__restrict__ s, DState *st) {
+    pdl_enter();
+    if (st->done) return;
+    const double na = -st->alpha;
+    stream_rows<4>(
+        n, [&](long i) { return make_double2(r[i], v[i]); },
+        [&](long i, const double2 &q) { s[i] = __dadd_rn(q.x, __dmul_rn(na, q.y)); });
+    pdl_release();
+}
+
+// The tests with this iteration's norms (st->r2, st->x2 from the launch that wrote r and x,
+// st->pc2 from t[3]), then the next iteration's: t = r0 . r, ||r||^2, ||x||^2, ||pc||^2.
+struct FinControlN {
+    __device__ void finish(DState *st, const double *t) const {
+        st->pc2 = t[3];
+        FinControl{}.finish(st, t);
+        st->r2 = t[1];
+        st->x2 = t[2];
+    }
+};
+
+// k_update_xr that also takes the next iteration's norms, whose vectors it writes, and adds up
+// the partial sums of ||pc||^2 (pcs, st->npc of them). The grid is the caller's: the tree of
+// r0 . r, which steers the iteration, follows it.
+static __global__ void __launch_bounds__(kThreads, 5)
+k_update_xrn(long n, const double *__restrict__ pc, const double *__restrict__ sc, const double *__restrict__ s,
+             const double *__restrict__ t, const double *__restrict__ r0, double *__restrict__ x,
+             double *__restrict__ r, DState *st, double *__restrict__ partials, const double *__restrict__ pcs) {
+    pdl_enter();
+    if (st->done) return;
+    const double a = st->alpha, om = st->omega, nom = -st->omega;
+    const int npc = st->npc;
+    double red[4] = {0.0, 0.0, 0.0, 0.0};
+    stream_rows<4>(
+        n, [&](long i) { return Ld6{x[i], pc[i], sc[i], s[i], t[i], r0[i]}; },
+        [&](long i, const Ld6 &q) {
+            double xi = q.a;
+            xi = __dadd_rn(xi, __dmul_rn(a, q.b));
+            xi = __dadd_rn(xi, __dmul_rn(om, q.c));
+            x[i] = xi;
+            const double ri = __dadd_rn(q.d, __dmul_rn(nom, q.e));
+            r[i] = ri;
+            red[0] += q.f * ri;
+            red[1] += ri * ri;
+            red[2] += xi * xi;
+        });
+    // each CTA's share of the partial sums, in order
+    for (int k = (int)(blockIdx.x * kThreads + threadIdx.x); k < npc; k += (int)gridDim.x * kThreads) red[3] += pcs[k];
+    pdl_release();
+    grid_reduce<4>(red, partials, st, FinControlN{});
 }
 
 // p = (-beta omega) v + beta p; p = p + r (cblas_daxpby + cblas_daxpy,

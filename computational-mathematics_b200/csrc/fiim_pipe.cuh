@@ -168,7 +168,7 @@ k_spmv_pipe(CsrView<double> M, const int *__restrict__ rb, int nblk, const doubl
         }
     }
     pdl_release();
-    if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red, partials, st, epi);
+    end_sums(red, partials, st, epi);
 }
 
 }  // namespace fiim

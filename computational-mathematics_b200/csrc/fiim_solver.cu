@@ -678,14 +678,14 @@ size_t csr_bytes(long n, long nnz) {
 
 // ------------------------------------------------------------------ preconditioner
 // out = M in for the chosen preconditioner; the last product's epilogue stores the
-// result and, when `norm`, also accumulates ||out||^2 into st->pc2.
+// result and, when `norm`, also leaves partial sums of ||out||^2 (pc_partials).
 int Solver::enqueue_prec(const double *in, double *out, bool norm) {
     cudaStream_t s = stream;
     const bool combined = (opt.variant == FIIM_ACIFIM && opt.mode == 'C' && opt.nr > 1);
     if (!combined) {
         // tm = IDv o (H in); out = G tm   (AFIIM/src/bicgstab.cpp:172-175)
         FIIM_CUDA(launch_spmv(H, s, in, EpiScale{tm, IDv}, st, partials, fault));
-        if (norm) FIIM_CUDA(launch_spmv(G, s, tm, EpiNorm{out}, st, partials, fault));
+        if (norm) FIIM_CUDA(launch_spmv(G, s, tm, EpiNormPart{out}, st, pc_partials(), fault));
         else FIIM_CUDA(launch_spmv(G, s, tm, EpiStore{out}, st, partials, fault));
         return FIIM_OK;
     }
@@ -702,7 +702,7 @@ int Solver::enqueue_prec(const double *in, double *out, bool norm) {
     for (int it = 1; it < opt.nr; ++it) {
         FIIM_CUDA(launch_spmv(U, s, out, EpiSubFrom{t3, t2}, st, partials, fault));
         if (it == opt.nr - 1 && norm)
-            FIIM_CUDA(launch_spmv(G, s, t3, EpiAccumNorm{out}, st, partials, fault));
+            FIIM_CUDA(launch_spmv(G, s, t3, EpiAccumNorm{out}, st, pc_partials(), fault));
         else
             FIIM_CUDA(launch_spmv(G, s, t3, EpiAccum{out}, st, partials, fault));
     }
@@ -721,12 +721,11 @@ int Solver::enqueue_iteration(bool cond, cudaGraphConditionalHandle h) {
     const long nn = n;
     FIIM_TRY(enqueue_prec(p, pc, true));                                             // K1-K2
     FIIM_CUDA(launch_spmv(A, s, pc, EpiAlpha{v, r0}, st, partials, fault));     // K3
-    FIIM_CUDA(launch_k(k_update_s<FinS>, stream_grid(k_update_s<FinS>, nn), 0, s, nn, r, v, x, sv, st, partials,
-                       FinS{}));                                                        // K4
+    FIIM_CUDA(launch_k(k_form_s, stream_grid(k_form_s, nn), 0, s, nn, r, v, sv, st));   // K4
     FIIM_TRY(enqueue_prec(sv, sc, false));                                           // K5-K6
     FIIM_CUDA(launch_spmv(A, s, sc, EpiOmega{t, sv}, st, partials, fault));    // K7
-    FIIM_CUDA(launch_k(k_update_xr<FinControl>, stream_grid(k_update_xr<FinControl>, nn), 0, s, nn, pc, sc, sv,
-                       t, r0, x, r, st, partials, FinControl{}));                       // K8
+    FIIM_CUDA(launch_k(k_update_xrn, xr_grid(), 0, s, nn, pc, sc, sv, t, r0, x, r, st, partials,
+                       (const double *)pc_partials()));                                 // K8
     FIIM_CUDA(launch_k(k_update_p, stream_grid(k_update_p, nn), 0, s, nn, r, v, p, st, h, cond ? 1 : 0));  // K9
     return FIIM_OK;
 }
@@ -1106,7 +1105,7 @@ int Solver::solve_start(const double *b_in, const double *x_in, double tol, int 
         return launch_cluster();
     }
     // Start: r = b - A x, r0 = r, p = r, ro = ||r0|| (AFIIM/src/bicgstab.cpp:151-165).
-    FIIM_CUDA(launch_spmv(A, stream, x, EpiInit{b, p, r0, r}, st, partials, fault));
+    FIIM_CUDA(launch_spmv(A, stream, x, EpiStart{{b, p, r0, r}, x}, st, partials, fault));
     pending_launches = 1;
     if (use_cond) {
         FIIM_CUDA(cudaGraphLaunch(exec, stream));
@@ -1303,12 +1302,12 @@ int Solver::kernel_times(int reps, int max_k, double *ms, double *bytes, char *n
     const long nn = n;
     std::vector<Item> items = {
         {"H_spmv_scale", S(H) + 3 * nv, [&] { return launch_spmv(H, stream, p, EpiScale{tm, IDv}, st, partials, fault); }},
-        {"G_spmv_norm", S(G) + 2 * nv, [&] { return launch_spmv(G, stream, tm, EpiNorm{pc}, st, partials, fault); }},
+        {"G_spmv_norm", S(G) + 2 * nv, [&] { return launch_spmv(G, stream, tm, EpiNormPart{pc}, st, pc_partials(), fault); }},
         {"A_spmv_alpha", S(A) + 3 * nv, [&] { return launch_spmv(A, stream, pc, EpiAlpha{v, r0}, st, partials, fault); }},
-        {"update_s", 4 * nv, [&] { k_update_s<FinS><<<stream_grid(k_update_s<FinS>, nn), kThreads, 0, stream>>>(nn, r, v, x, sv, st, partials, FinS{}); return cudaGetLastError(); }},
+        {"update_s", 3 * nv, [&] { return launch_k(k_form_s, stream_grid(k_form_s, nn), 0, stream, nn, r, v, sv, st); }},
         {"G_spmv", S(G) + 2 * nv, [&] { return launch_spmv(G, stream, tm, EpiStore{sc}, st, partials, fault); }},
         {"A_spmv_omega", S(A) + 3 * nv, [&] { return launch_spmv(A, stream, sc, EpiOmega{t, sv}, st, partials, fault); }},
-        {"update_xr", 8 * nv, [&] { k_update_xr<FinControl><<<stream_grid(k_update_xr<FinControl>, nn), kThreads, 0, stream>>>(nn, pc, sc, sv, t, r0, x, r, st, partials, FinControl{}); return cudaGetLastError(); }},
+        {"update_xr", 8 * nv, [&] { return launch_k(k_update_xrn, xr_grid(), 0, stream, nn, pc, sc, sv, t, r0, x, r, st, partials, (const double *)pc_partials()); }},
         {"update_p", 4 * nv, [&] { k_update_p<<<stream_grid(k_update_p, nn), kThreads, 0, stream>>>(nn, r, v, p, st, cudaGraphConditionalHandle{}, 0); return cudaGetLastError(); }},
     };
     if (in_sequence)   // the body's second H product (K5), between the s update and G's product

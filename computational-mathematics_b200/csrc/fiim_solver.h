@@ -82,6 +82,11 @@ struct Solver : SolverBase {
     int enqueue_prec(const double *in, double *out, bool norm);
     int enqueue_iteration(bool cond, cudaGraphConditionalHandle h);
     int build_graph();
+    // Partial sums of ||pc||^2 (EpiNormPart), behind the ones a launch adds up itself (at most four
+    // per CTA of a full grid of eight CTAs per SM; the buffer holds 4 x 32 per SM).
+    double *pc_partials() const { return partials + (size_t)64 * num_sms(); }
+    // CTAs of the x / r update: five per SM, which its r0 . r is summed over.
+    int xr_grid() const { return (int)std::min<long>(((long)n + kThreads - 1) / kThreads, 5L * num_sms()); }
     int kernels_per_iteration() const;
     void print_status(int info, int iter, double rel) const;
     int apply(int op, const double *in, double *out);
