@@ -125,8 +125,18 @@ struct MixedSolver : SolverBase {
 
     template <typename Epi>
     cudaError_t spmv_gh(const DevCsr &M, bool is_g, const float *xx, const Epi &epi) {
-        if (bf16) return spmv_f(M, is_g ? G16 : H16, stream, xx, epi, st, partials);
-        return spmv_f(M, is_g ? G32 : H32, stream, xx, epi, st, partials);
+        double *sums = Defers<Epi>::value ? pc_partials() : partials;
+        if (bf16) return spmv_f(M, is_g ? G16 : H16, stream, xx, epi, st, sums);
+        return spmv_f(M, is_g ? G32 : H32, stream, xx, epi, st, sums);
+    }
+    // Partial sums of ||pc||^2, behind the ones a launch adds up itself (at most four per CTA of a
+    // full grid of eight CTAs per SM; the buffer holds 4 x 32 per SM).
+    double *pc_partials() const { return partials + (size_t)64 * num_sms(); }
+    template <int PER_SM, class Fin>
+    cudaError_t update_xr(const Fin &fin) {
+        const int g = (int)std::min<long>(((long)n + kThreads - 1) / kThreads, (long)PER_SM * num_sms());
+        return launch_k(mx::k_update_xr_f<Fin, PER_SM>, g, 0, stream, (long)n, pc, sc, s, t, r0, e, r, st, partials,
+                        (const double *)pc_partials(), fin);
     }
 
     // cond: bit 0 = set the WHILE node's condition (hw), bit 1 = set the IF node's (hif,
@@ -136,20 +146,17 @@ struct MixedSolver : SolverBase {
         FIIM_CUDA(spmv_gh(H, false, p, mx::EpiScaleF{tm, D32}));
         FIIM_CUDA(spmv_gh(G, true, tm, mx::EpiNormF{pc}));
         FIIM_CUDA(spmv_f(A, A32, stream, pc, mx::EpiAlphaF{v, r0}, st, partials));
-        FIIM_CUDA(launch_k(mx::k_update_s_f, sgrid(mx::k_update_s_f, nn), 0, stream, nn, r, v, e, s, st, partials));
+        FIIM_CUDA(launch_k(mx::k_update_s_f, sgrid(mx::k_update_s_f, nn), 0, stream, nn, r, v, s, st));
         FIIM_CUDA(spmv_gh(H, false, s, mx::EpiScaleF{tm, D32}));
         FIIM_CUDA(spmv_gh(G, true, tm, mx::EpiStoreF{sc}));
         FIIM_CUDA(spmv_f(A, A32, stream, sc, mx::EpiOmegaF{t, s}, st, partials));
         if (reliable) {
-            auto kxr = mx::k_update_xr_f<mx::FinControlR>;
-            FIIM_CUDA(launch_k(kxr, sgrid(kxr, nn), 0, stream, nn, pc, sc, s, t, r0, e, r, st, partials,
-                               mx::FinControlR{rs}));
+            FIIM_CUDA(update_xr<4>(mx::FinControlR{rs}));
             FIIM_CUDA(launch_k(mx::k_update_p_r, sgrid(mx::k_update_p_r, nn), 0, stream, nn, r, v, p, st,
                                (const mx::RState *)rs, hw, hif, cond));
             return FIIM_OK;
         }
-        auto kxr = mx::k_update_xr_f<FinControl>;
-        FIIM_CUDA(launch_k(kxr, sgrid(kxr, nn), 0, stream, nn, pc, sc, s, t, r0, e, r, st, partials, FinControl{}));
+        FIIM_CUDA(update_xr<5>(FinControl{}));
         FIIM_CUDA(launch_k(mx::k_update_p_f, sgrid(mx::k_update_p_f, nn), 0, stream, nn, r, v, p, st, hw,
                            (cond & 1) ? 1 : 0));
         return FIIM_OK;

@@ -36,14 +36,14 @@ struct EpiScaleF {                 // y = d o (M x)
     __device__ void emit(long i, float s, double (&r)[NR]) const { emit_pre(i, s, pre(i), r); }
     __device__ void finish(DState *, const double *) const {}
 };
-struct EpiNormF {                  // y = M x, ||y||^2 -> st->pc2
+struct EpiNormF {                  // y = M x, ||y||^2 left as partial sums for the x / r update
     FIIM_EPI(1, true, true);
+    using DEFERS = void;
     float *y;
     __device__ void emit(long i, float s, double (&r)[NR]) const {
         y[i] = s;
         r[0] += (double)s * (double)s;
     }
-    __device__ void finish(DState *st, const double *t) const { st->pc2 = t[0]; }
 };
 struct EpiAlphaF {                 // v = A pc, alpha = m1 / (r0 . v)
     FIIM_EPI(1, true, true);
@@ -168,7 +168,7 @@ k_spmv_rows_f(CsrView<V> M, const int *__restrict__ rb, const int *__restrict__ 
         }
     }
     pdl_release();
-    if constexpr (Epi::REDUCES) grid_reduce<Epi::NR>(red, partials, st, epi);
+    end_sums(red, partials, st, epi);
 }
 
 // ---------------------------------------------------------------- inner start / updates
@@ -186,7 +186,15 @@ __device__ __forceinline__ void rows4(long n, F4 f4, F1 f1) {
 }
 
 // Inner start from e = 0: r = r0 = p = r64 / ||r64|| in FP32 (||r64||^2 is sto->ts from
-// the residual kernel); ||r0||^2 accumulated in FP64 -> ro, m1, rc (FinInit).
+// the residual kernel); ||r0||^2 accumulated in FP64 -> ro, m1, rc (FinInit), and the first
+// iteration's norms ||r||^2 and ||e||^2 = 0.
+struct FinStart {
+    __device__ void finish(DState *st, const double *t) const {
+        FinInit{}.finish(st, t);
+        st->r2 = t[0];
+        st->x2 = 0.0;
+    }
+};
 static __global__ void __launch_bounds__(kThreads)
 k_inner_init(long n, const double *__restrict__ r64, const DState *sto, float *__restrict__ r,
              float *__restrict__ r0, float *__restrict__ p, float *__restrict__ e, DState *st,
@@ -203,50 +211,65 @@ k_inner_init(long n, const double *__restrict__ r64, const DState *sto, float *_
         red[0] += (double)ri * (double)ri;
     }
     pdl_release();
-    grid_reduce<1>(red, partials, st, FinInit{});
+    grid_reduce<1>(red, partials, st, FinStart{});
 }
 
+// s = r - alpha v.
 static __global__ void __launch_bounds__(kThreads)
-k_update_s_f(long n, const float *__restrict__ r, const float *__restrict__ v,
-             const float *__restrict__ e, float *__restrict__ s, DState *st,
-             double *__restrict__ partials) {
+k_update_s_f(long n, const float *__restrict__ r, const float *__restrict__ v, float *__restrict__ s, DState *st) {
     pdl_enter();
     if (st->done) return;
     const float na = (float)(-st->alpha);
-    double red[2] = {0.0, 0.0};
-    auto row = [&](float ri, float vi, float ei) {
-        red[0] += (double)ri * (double)ri;
-        red[1] += (double)ei * (double)ei;
-        return fmaf(na, vi, ri);
-    };
     rows4(
         n,
         [&](long q) {
-            const float4 r4 = ld4(r, q), v4 = ld4(v, q), e4 = ld4(e, q);
-            st4(s, q, make_float4(row(r4.x, v4.x, e4.x), row(r4.y, v4.y, e4.y), row(r4.z, v4.z, e4.z),
-                                  row(r4.w, v4.w, e4.w)));
+            const float4 r4 = ld4(r, q), v4 = ld4(v, q);
+            st4(s, q, make_float4(fmaf(na, v4.x, r4.x), fmaf(na, v4.y, r4.y), fmaf(na, v4.z, r4.z),
+                                  fmaf(na, v4.w, r4.w)));
         },
-        [&](long i) { s[i] = row(r[i], v[i], e[i]); });
+        [&](long i) { s[i] = fmaf(na, v[i], r[i]); });
     pdl_release();
-    grid_reduce<2>(red, partials, st, FinS{});
 }
 
-template <class Fin = FinControl>
-static __global__ void __launch_bounds__(kThreads)
+// Fin's tests with this iteration's norms (st->r2, st->x2 from the launch that wrote r and e,
+// st->pc2 from t[3]), then the next iteration's: t = r0 . r, ||r||^2, ||e||^2, ||pc||^2.
+template <class Fin>
+struct FinNorms {
+    Fin fin;
+    __device__ void finish(DState *st, const double *t) const {
+        st->pc2 = t[3];
+        fin.finish(st, t);
+        st->r2 = t[1];
+        st->x2 = t[2];
+    }
+};
+
+// e += alpha pc + omega sc; r = s - omega t; r0 . r, the next iteration's norms of the two vectors
+// it writes (the s update then reads neither e nor a sum), and the partial sums of ||pc||^2 (pcs,
+// st->npc of them) added up. PER_SM CTAs an SM, all resident: the tree of r0 . r, which steers
+// the iteration, follows the grid.
+template <class Fin, int PER_SM>
+static __global__ void __launch_bounds__(kThreads, PER_SM)
 k_update_xr_f(long n, const float *__restrict__ pc, const float *__restrict__ sc,
               const float *__restrict__ s, const float *__restrict__ t,
               const float *__restrict__ r0, float *__restrict__ e, float *__restrict__ r,
-              DState *st, double *__restrict__ partials, Fin fin = Fin{}) {
+              DState *st, double *__restrict__ partials, const double *__restrict__ pcs, Fin fin) {
     pdl_enter();
     if (st->done) return;
     const float a = (float)st->alpha, om = (float)st->omega;
-    double red[1] = {0.0};
+    const int npc = st->npc;
+    double red[4] = {0.0, 0.0, 0.0, 0.0};
     auto res = [&](float si, float ti, float r0i) {   // r = s - omega t; r0 . r
         const float ri = fmaf(-om, ti, si);
         red[0] += (double)r0i * (double)ri;
+        red[1] += (double)ri * (double)ri;
         return ri;
     };
-    auto cor = [&](float ei, float pci, float sci) { return fmaf(om, sci, fmaf(a, pci, ei)); };   // e update
+    auto cor = [&](float ei, float pci, float sci) {   // e update
+        const float en = fmaf(om, sci, fmaf(a, pci, ei));
+        red[2] += (double)en * (double)en;
+        return en;
+    };
     rows4(
         n,
         [&](long q) {
@@ -261,8 +284,9 @@ k_update_xr_f(long n, const float *__restrict__ pc, const float *__restrict__ sc
             e[i] = cor(e[i], pc[i], sc[i]);
             r[i] = res(s[i], t[i], r0[i]);
         });
+    for (int k = (int)(blockIdx.x * kThreads + threadIdx.x); k < npc; k += (int)gridDim.x * kThreads) red[3] += pcs[k];
     pdl_release();
-    grid_reduce<1>(red, partials, st, fin);
+    grid_reduce<4>(red, partials, st, FinNorms<Fin>{fin});
 }
 
 static __global__ void __launch_bounds__(kThreads)
@@ -391,10 +415,11 @@ k_replace_x(long n, float *__restrict__ e, double *__restrict__ x, const RState 
 
 // Replacement, second half: the epilogue of the FP64 product A x. Per row, the true
 // residual b - A x (FP64), the new scaled FP32 residual, p moved by the change in r; sums
-// ||b - A x||^2 and r0 . r_new. The finish sets m1, restarts the running maximum, and at a
+// ||b - A x||^2, r0 . r_new and ||r_new||^2. The finish sets m1 and the next iteration's norms (e
+// is zero again), restarts the running maximum, and at a
 // verification ends the solve when the FP64 target is met (or after max_verify attempts).
 struct EpiReplace {
-    FIIM_EPI(2, true, false);
+    FIIM_EPI(3, true, false);
     const double *__restrict__ b;
     float *r;
     float *p;
@@ -407,10 +432,13 @@ struct EpiReplace {
         r[i] = rn;
         red[0] += rt * rt;
         red[1] += (double)r0[i] * (double)rn;
+        red[2] += (double)rn * (double)rn;
     }
     __device__ void finish(DState *st, const double *t) const {
         rs->true_r = sqrt(t[0]);
         st->m1 = t[1];
+        st->r2 = t[2];
+        st->x2 = 0.0;
         rs->rmax = rs->true_r * rs->inv_sigma;
         rs->update = 0;
         rs->replacements++;
