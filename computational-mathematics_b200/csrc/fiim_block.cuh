@@ -98,7 +98,8 @@ __device__ __forceinline__ void rhs_reduce(double (&v)[VW][NR], int k, double *_
 }
 
 // ---------------------------------------------------------------- epilogues
-// emit(at, s, red) finishes entry `at` of the n x k output block from its row sum s;
+// emit_pre(at, s, q, red) finishes entry `at` of the n x k output block from its row sum s and
+// its operand q = pre(at, row), which can be loaded before the sum is ready;
 // emit2(at, s0, s1, red0, red1) finishes the two consecutive entries at, at + 1 (at even)
 // with the same arithmetic per entry, reading and writing both as one 16-byte pair (the
 // sparse products with two or four right-hand sides per lane).
@@ -110,14 +111,11 @@ __device__ __forceinline__ void rhs_reduce(double (&v)[VW][NR], int k, double *_
 __device__ __forceinline__ void st2(double *p, double a, double b) { *reinterpret_cast<double2 *>(p) = make_double2(a, b); }
 __device__ __forceinline__ double2 ld2(const double *__restrict__ p) { return __ldg(reinterpret_cast<const double2 *>(p)); }
 
-// pre(at) is the operand that emit_pre(at, s, operand, red) finishes entry `at` with, for a kernel
-// that loads it before the sum is ready; emit is the two together.
 struct KEpiStore {
     FIIM_BEPI(1, false, true);
     double *y;
-    __device__ double pre(size_t) const { return 0.0; }
+    __device__ double pre(size_t, long) const { return 0.0; }
     __device__ void emit_pre(size_t at, double s, double, double (&)[NR]) const { y[at] = s; }
-    __device__ void emit(size_t at, double s, double (&)[NR]) const { y[at] = s; }
     __device__ void emit2(size_t at, double s0, double s1, double (&)[NR], double (&)[NR]) const { st2(y + at, s0, s1); }
     __device__ void finish(BState &, int, const double *) const {}
 };
@@ -126,9 +124,8 @@ struct KEpiScale {                 // y = d o (M x), d per row
     double *y;
     const double *__restrict__ d;
     int k;
-    __device__ double pre(size_t at) const { return __ldg(d + at / k); }
+    __device__ double pre(size_t, long row) const { return __ldg(d + row); }
     __device__ void emit_pre(size_t at, double s, double di, double (&)[NR]) const { y[at] = __dmul_rn(di, s); }
-    __device__ void emit(size_t at, double s, double (&r)[NR]) const { emit_pre(at, s, pre(at), r); }
     __device__ void emit2(size_t at, double s0, double s1, double (&)[NR], double (&)[NR]) const {
         const double di = __ldg(d + at / k);
         st2(y + at, __dmul_rn(di, s0), __dmul_rn(di, s1));
@@ -138,9 +135,8 @@ struct KEpiScale {                 // y = d o (M x), d per row
 struct KEpiNorm {
     FIIM_BEPI(1, true, true);
     double *y;
-    __device__ double pre(size_t) const { return 0.0; }
-    __device__ void emit_pre(size_t at, double s, double, double (&r)[NR]) const { emit(at, s, r); }
-    __device__ void emit(size_t at, double s, double (&r)[NR]) const { y[at] = s; r[0] += s * s; }
+    __device__ double pre(size_t, long) const { return 0.0; }
+    __device__ void emit_pre(size_t at, double s, double, double (&r)[NR]) const { y[at] = s; r[0] += s * s; }
     __device__ void emit2(size_t at, double s0, double s1, double (&ra)[NR], double (&rb)[NR]) const {
         st2(y + at, s0, s1);
         ra[0] += s0 * s0;
@@ -152,12 +148,11 @@ struct KEpiAlpha {
     FIIM_BEPI(1, true, true);
     double *y;
     const double *__restrict__ r0;
-    __device__ double pre(size_t at) const { return __ldg(r0 + at); }
+    __device__ double pre(size_t at, long) const { return __ldg(r0 + at); }
     __device__ void emit_pre(size_t at, double s, double q, double (&r)[NR]) const {
         y[at] = s;
         r[0] += q * s;
     }
-    __device__ void emit(size_t at, double s, double (&r)[NR]) const { emit_pre(at, s, pre(at), r); }
     __device__ void emit2(size_t at, double s0, double s1, double (&ra)[NR], double (&rb)[NR]) const {
         st2(y + at, s0, s1);
         const double2 q = ld2(r0 + at);
@@ -170,13 +165,12 @@ struct KEpiOmega {
     FIIM_BEPI(2, true, true);
     double *y;
     const double *__restrict__ sv;
-    __device__ double pre(size_t at) const { return __ldg(sv + at); }
+    __device__ double pre(size_t at, long) const { return __ldg(sv + at); }
     __device__ void emit_pre(size_t at, double s, double q, double (&r)[NR]) const {
         y[at] = s;
         r[0] += s * q;
         r[1] += s * s;
     }
-    __device__ void emit(size_t at, double s, double (&r)[NR]) const { emit_pre(at, s, pre(at), r); }
     __device__ void emit2(size_t at, double s0, double s1, double (&ra)[NR], double (&rb)[NR]) const {
         st2(y + at, s0, s1);
         const double2 q = ld2(sv + at);
@@ -191,8 +185,7 @@ struct KEpiInit {
     FIIM_BEPI(1, true, true);
     const double *__restrict__ b;
     double *p, *r0, *r;
-    __device__ double pre(size_t at) const { return b[at]; }
-    __device__ void emit(size_t at, double s, double (&red)[NR]) const { emit_pre(at, s, pre(at), red); }
+    __device__ double pre(size_t at, long) const { return b[at]; }
     __device__ void emit_pre(size_t at, double s, double bi, double (&red)[NR]) const {
         const double pi = __dadd_rn(bi, __dmul_rn(-1.0, s));
         p[at] = pi;
@@ -217,8 +210,7 @@ struct KEpiRestart : KEpiInit {
 struct KEpiResid {
     FIIM_BEPI(2, true, false);
     const double *__restrict__ b;
-    __device__ double pre(size_t at) const { return b[at]; }
-    __device__ void emit(size_t at, double s, double (&red)[NR]) const { emit_pre(at, s, pre(at), red); }
+    __device__ double pre(size_t at, long) const { return b[at]; }
     __device__ void emit_pre(size_t at, double s, double bi, double (&red)[NR]) const {
         const double ri = bi - s;
         red[0] += ri * ri;
@@ -327,7 +319,7 @@ k_spmm(CsrView<V> M, Shape sh, const int *__restrict__ chunk, int nch, const dou
             } else {
 #pragma unroll
                 for (int u = 0; u < VW; ++u)
-                    if (!(Epi::GATED && bs.done[j0 + u])) epi.emit(at + u, s[u], red[u]);
+                    if (!(Epi::GATED && bs.done[j0 + u])) epi.emit_pre(at + u, s[u], epi.pre(at + u, row), red[u]);
             }
         }
     }
@@ -341,8 +333,8 @@ k_spmm(CsrView<V> M, Shape sh, const int *__restrict__ chunk, int nch, const dou
 // broadcast each with the column already times k (three shuffles and a product before); eight
 // entries of one row are added without looking for its end; the next 32 entries are loaded while
 // these are added, and a row's epilogue operand when the row begins. Row sums in storage order, as
-// everywhere. Power-law matrix, n = 200,003, 2.9 M entries, 32 right-hand sides: A X 445 -> 155 us,
-// M X (FP32 factors) 176 -> 144, an iteration 1.53 -> 0.62 ms with the shorter reductions and
+// everywhere. Power-law matrix, n = 200,003, 2.9 M entries, 32 right-hand sides: A X 445 -> 152 us,
+// M X (FP32 factors) 176 -> 133, an iteration 1.53 -> 0.60 ms with the shorter reductions and
 // updates of this file.
 template <typename V, typename Epi>
 static __global__ void __launch_bounds__(kThreads, 4)
@@ -365,7 +357,7 @@ k_spmm_stream(CsrView<V> M, Shape sh, const int *__restrict__ chunk, int nch, co
         int ends = held + lane < r1 ? __ldg(M.rp + held + lane + 1) : 0;
         const int e0 = __ldg(M.rp + r0), e1 = __ldg(M.rp + r1);
         int end = __shfl_sync(full, ends, 0);
-        double s = 0.0, op = out ? epi.pre((size_t)row * sh.k + lane) : 0.0;
+        double s = 0.0, op = out ? epi.pre((size_t)row * sh.k + lane, row) : 0.0;
         auto finish_row = [&] {
             if (out) epi.emit_pre((size_t)row * sh.k + lane, s, op, red[0]);
             s = 0.0;
@@ -374,7 +366,7 @@ k_spmm_stream(CsrView<V> M, Shape sh, const int *__restrict__ chunk, int nch, co
                 ends = held + lane < r1 ? __ldg(M.rp + held + lane + 1) : 0;
             }
             end = __shfl_sync(full, ends, row - held);
-            op = out && row < r1 ? epi.pre((size_t)row * sh.k + lane) : 0.0;
+            op = out && row < r1 ? epi.pre((size_t)row * sh.k + lane, row) : 0.0;
         };
         int c = e0 + lane < e1 ? ldi(M.ci + e0 + lane) : 0;
         V a = e0 + lane < e1 ? ldm(M.v + e0 + lane) : V(0);

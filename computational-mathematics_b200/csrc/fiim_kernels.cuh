@@ -1514,7 +1514,7 @@ k_update_xr(long n, const double *__restrict__ pc, const double *__restrict__ sc
 }
 
 // s = r + (-alpha) v alone, for the solver whose x / r update takes the norms: one read less (x)
-// and no reduction. 128^3 in the body's order: 14.9 us with the norms.
+// and no reduction. 128^3 in the body's order: 14.9 us with the norms, 7.6 without.
 static __global__ void __launch_bounds__(kThreads)
 k_form_s(long n, const double *__restrict__ r, const double *__restrict__ v, double *__restrict__ s, DState *st) {
     pdl_enter();
