@@ -174,20 +174,17 @@ struct BatchSolver : SolverBase {
     int enqueue_iteration(bool cond, cudaGraphConditionalHandle h) {
         const int nb = A.M.nblk;
         FIIM_CUDA(spmv_f(H, p, bt::BEpiScale{tm, IDv}));
-        FIIM_CUDA(spmv_f(G, tm, bt::BEpiNorm{pc}));
-        FIIM_CUDA(finish<1>(G, bt::BEpiNorm{pc}));
-        FIIM_CUDA(spmv(A, A.M.v, pc, bt::BEpiAlpha{v, r0}));
-        FIIM_CUDA(finish<1>(A, bt::BEpiAlpha{v, r0}));
-        FIIM_CUDA(launch_k(bt::k_bupdate_s, sgrid(bt::k_bupdate_s, nb), 0, stream, A.M.rb, A.blk_sys, A.sys_blk,
-                           nb, r, v, x, sv, bs, partials));
-        FIIM_CUDA(finish_rows<2>(bt::BFinS{}));
+        FIIM_CUDA(spmv_f(G, tm, bt::BEpiStore{pc}));
+        FIIM_CUDA(spmv(A, A.M.v, pc, bt::BEpiAlpha{v, r0, pc}));
+        FIIM_CUDA(finish<2>(A, bt::BEpiAlpha{v, r0, pc}));
+        FIIM_CUDA(launch_k(bt::k_bform_s, sgrid(bt::k_bform_s, nb), 0, stream, A.M.rb, A.blk_sys, nb, r, v, sv, bs));
         FIIM_CUDA(spmv_f(H, sv, bt::BEpiScale{tm, IDv}));
         FIIM_CUDA(spmv_f(G, tm, bt::BEpiStore{sc}));
         FIIM_CUDA(spmv(A, A.M.v, sc, bt::BEpiOmega{t, sv}));
         FIIM_CUDA(finish<2>(A, bt::BEpiOmega{t, sv}));
-        FIIM_CUDA(launch_k(bt::k_bupdate_xr, sgrid(bt::k_bupdate_xr, nb), 0, stream, A.M.rb, A.blk_sys, A.sys_blk,
-                           nb, pc, sc, sv, t, r0, x, r, bs, partials));
-        FIIM_CUDA(finish_rows<1>(bt::BFinControl{}));
+        FIIM_CUDA(launch_k(bt::k_bupdate_xr, sgrid(bt::k_bupdate_xr, nb), 0, stream, A.M.rb, A.blk_sys, nb, pc, sc, sv,
+                           t, r0, x, r, bs, partials));
+        FIIM_CUDA(finish_rows<3>(bt::BFinControlN{}));
         FIIM_CUDA(launch_k(bt::k_bupdate_p, sgrid(bt::k_bupdate_p, nb), 0, stream, A.M.rb, A.blk_sys, nb, r, v, p,
                            bs, h, cond ? 1 : 0));
         return FIIM_OK;
@@ -311,10 +308,10 @@ struct BatchSolver : SolverBase {
         FIIM_TRY(build_copy(A, 0, 8, A.M.v));
         FIIM_TRY(build_copy(G, 1, fvb, f16 ? (const void *)G.v16 : f32 ? (const void *)G.v32 : (const void *)G.M.v));
         FIIM_TRY(build_copy(H, 2, fvb, f16 ? (const void *)H.v16 : f32 ? (const void *)H.v32 : (const void *)H.M.v));
-        // Partials of the largest count: per warp of a row block, or per slice (two values each).
+        // Partials of the largest count: per warp of a row block, or per slice (three values each).
         long maxq = std::max({(long)A.M.nblk, (long)G.M.nblk, (long)H.M.nblk, 1L}) * kWarps;
         for (const BMat *B : {&A, &G, &H}) maxq = std::max(maxq, (long)B->M.nsl);
-        FIIM_CUDA(cudaMalloc(&partials, sizeof(double) * 2 * maxq));
+        FIIM_CUDA(cudaMalloc(&partials, sizeof(double) * 3 * maxq));
         // per-system divergence windows (AFIIM/src/bicgstab.cpp:114, ACIFIM/src/bicgstab.cpp:132)
         std::vector<int> mm(nsys);
         for (int k = 0; k < nsys; ++k) {
@@ -430,8 +427,8 @@ struct BatchSolver : SolverBase {
         FIIM_CUDA(cudaMemcpyAsync(b, b_in, sizeof(double) * N, kin, stream));
         FIIM_CUDA(cudaMemcpyAsync(x, x_io, sizeof(double) * N, kin, stream));
         FIIM_TRY(reset_state(tol, nmax));
-        FIIM_CUDA(spmv(A, A.M.v, x, bt::BEpiInit{b, p, r0, r}));
-        FIIM_CUDA(finish<1>(A, bt::BEpiInit{b, p, r0, r}));
+        FIIM_CUDA(spmv(A, A.M.v, x, bt::BEpiInit{b, p, r0, r, x}));
+        FIIM_CUDA(finish<2>(A, bt::BEpiInit{b, p, r0, r, x}));
         FIIM_TRY(run_loop(nmax));
         FIIM_CUDA(spmv(A, A.M.v, x, bt::BEpiResid{b}));
         FIIM_CUDA((finish<2, false>(A, bt::BEpiResid{b})));
@@ -449,8 +446,8 @@ struct BatchSolver : SolverBase {
             if (hg->active == 0) break;
             ++rounds;
             extra += 4;
-            FIIM_CUDA(spmv(A, A.M.v, x, bt::BEpiRestart{{b, p, r0, r}}));
-            FIIM_CUDA(finish<1>(A, bt::BEpiRestart{{b, p, r0, r}}));
+            FIIM_CUDA(spmv(A, A.M.v, x, bt::BEpiRestart{{b, p, r0, r, x}}));
+            FIIM_CUDA(finish<2>(A, bt::BEpiRestart{{b, p, r0, r, x}}));
             FIIM_TRY(run_loop(nmax));
             FIIM_CUDA(spmv(A, A.M.v, x, bt::BEpiResid{b}));
             FIIM_CUDA((finish<2, false>(A, bt::BEpiResid{b})));
@@ -490,7 +487,7 @@ struct BatchSolver : SolverBase {
             summary->true_relres = worst_rel;
             summary->refine_steps = rounds;
             summary->device_ms = ms;
-            summary->launches = 4 + extra + (hg->loops_total + hg->loops) * 14;
+            summary->launches = 4 + extra + (hg->loops_total + hg->loops) * 12;
         }
         return FIIM_OK;
     }

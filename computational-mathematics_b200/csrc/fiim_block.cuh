@@ -159,7 +159,7 @@ struct KEpiAlpha {
         ra[0] += q.x * s0;
         rb[0] += q.y * s1;
     }
-    __device__ void finish(BState &bs, int j, const double *t) const { bt::BEpiAlpha{}.finish(bs, j, t); }
+    __device__ void finish(BState &bs, int j, const double *t) const { bt::BFinAlpha{}.finish(bs, j, t); }
 };
 struct KEpiOmega {
     FIIM_BEPI(2, true, true);

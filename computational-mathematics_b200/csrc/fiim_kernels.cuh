@@ -4,13 +4,14 @@
 // launches, each one pass over HBM with the BLAS-1 work and the scalar recurrences
 // fused in:
 //   K1 tm = IDv o (H p)                 spmv, scale epilogue        (:172-173)
-//   K2 pc = G tm,  sum pc^2             spmv, norm epilogue         (:175, :201)
+//   K2 pc = G tm,  CTA sums of pc^2     spmv, norm epilogue         (:175, :201)
 //   K3 v = A pc,   alpha = m1/(r0.v)    spmv, dot epilogue          (:178, :181)
-//   K4 s = r - alpha v, sum r^2, x^2    stream                      (:184-185, :201, :216)
+//   K4 s = r - alpha v                  stream                      (:184-185)
 //   K5 tm = IDv o (H s)                 spmv, scale epilogue        (:189-190)
 //   K6 sc = G tm                        spmv                        (:192)
 //   K7 t = A sc,   omega = t.s / t.t    spmv, 2-dot epilogue        (:195, :198)
-//   K8 x += alpha pc + omega sc, r = s - omega t, m1 = r0.r, tests  (:207-267)
+//   K8 x += alpha pc + omega sc, r = s - omega t, m1 = r0.r, tests  (:207-267);
+//      the next iteration's sum r^2, x^2                            (:201, :216)
 //   K9 p = r + beta (p - omega v)                                   (:270-271)
 //
 // Rounding: every vector the reference computes is computed here with the same

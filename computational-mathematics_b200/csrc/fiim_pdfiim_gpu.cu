@@ -13,9 +13,10 @@
 //   * kept entries are sorted by index through their ranks.
 // One pass over the rows leaves every row's entries and D^{-1} in the next free places; running
 // totals of the counts and a transpose, all on the device, put them in order, and the second call
-// copies them from there into the caller's arrays. A row whose pattern outgrows the warp's shared memory (CAP members in a solve, 4 CAP in the set; 2048 at the
-// largest CAP) is listed and built again with a larger CAP; past the largest CAP the call
-// returns FIIM_EARG and the host construction serves.
+// copies them from there into the caller's arrays. A row whose pattern outgrows the warp's shared
+// memory (CAP members in a solve, 4 CAP in the set; 2048 at the largest CAP) is listed and built
+// again with a larger CAP; past the largest CAP the call returns FIIM_EARG and the host
+// construction serves.
 
 #include <cuda_runtime.h>
 
