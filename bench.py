@@ -807,9 +807,11 @@ def run_ours(args):
     achieved = h_bytes / (h_ms / 1000.0) / 1e9
     h_alone = next(m for k, m, _ in ktimes if k == "H_spmv_scale")
     # The bytes H's product reads in the form it is served in (the formula above counts 4-byte
-    # column indices and row offsets; the sliced-diagonal form reads neither), and the
+    # column indices and row offsets; the sliced-diagonal form reads neither, and the values of
+    # equal slices once), and the
     # iteration's bytes on the same count.
-    form_names = {0: "CSR stream", 1: "CSR stream (bulk copies)", 2: "CSR stream (warp blocks)", 3: "sliced-diagonal"}
+    form_names = {0: "CSR stream", 1: "CSR stream (bulk copies)", 2: "CSR stream (warp blocks)", 3: "sliced-diagonal",
+                  4: "packed slices"}
     nvb = 8.0 * n
     h_form = S.matrix_bytes(2) + 3 * nvb
     it_form = 2 * sum(S.matrix_bytes(w) for w in range(3)) + 32 * nvb
@@ -825,8 +827,9 @@ def run_ours(args):
                 "per_kernel_in_sequence": [{"kernel": k, "ms": round(m, 5)} for k, m, _ in seq],
                 "form": form_names.get(S.spmv_shape(2)[1], "?"),
                 "bytes_note": ("achieved/frac use the survey's formula S(M) = 12 nnz + 4 (n + 1), which counts "
-                               "4-byte column indices and row offsets; the sliced-diagonal form reads neither, "
-                               "so frac can exceed 1: frac_on_form_bytes and traffic give what it reads"),
+                               "4-byte column indices, row offsets and every value; the sliced-diagonal form reads no "
+                               "indices, and equal slices' values once, so frac can exceed 1: "
+                               "frac_on_form_bytes and traffic give what it reads"),
                 "form_bytes_per_launch": h_form,
                 "achieved_on_form_bytes": round(h_form / (h_ms / 1000) / 1e9, 1),
                 "frac_on_form_bytes": round(h_form / (h_ms / 1000) / 1e9 / peak, 4),
@@ -979,9 +982,9 @@ def main():
     ap.add_argument("--no-small", action="store_true", help="skip the small plain case (Poisson 128^2)")
     ap.add_argument("--cpu-solves", type=int, default=3, help="timed full solves of the CPU baseline leg")
     # DRAM bytes per launch of the dominant kernel (H's SpMV) from an ncu capture of the
-    # 128^3 workload (dram__bytes_read.sum + dram__bytes_write.sum, mean of three H launches:
-    # 0.817 x its algorithmic bytes, the column stream being stored as 16-bit offsets).
-    ap.add_argument("--ncu-traffic", type=float, default=220.0e6,
+    # 128^3 workload (dram__bytes_read.sum + dram__bytes_write.sum: the gathered vector and the
+    # D^-1 operand; the shared blocks and the output stay in cache).
+    ap.add_argument("--ncu-traffic", type=float, default=33.8e6,
                     help="dram bytes per launch of the dominant kernel from an ncu capture")
     ap.add_argument("--dry-run", action="store_true",
                     help="no GPU: check the rank launcher and max-over-ranks timing over gloo (solves nothing)")

@@ -1299,10 +1299,11 @@ k_spmv_vec(CsrView<double> M, const double *__restrict__ x, Epi epi, DState *st,
 // entries at a time, leaves the rounded products in its part of shared memory, and lane l adds row
 // l's products left to right, from tile to tile, so every sum is the reference's bit for bit.
 // FILL 0 uses every entry; 1 keeps col >= row and 2 keeps col <= row (MKL's TRIANGULAR
-// descriptors), told apart by the columns kept beside the products. rpw comes from the entry count read on the device: 32 rows while they hold about
-// two tiles, fewer for longer rows, and (while they hold more than 64) fewer while some warps of
-// the grid would have no rows.
-// The next rows' offsets are loaded while these are summed.
+// descriptors), told apart by the columns kept beside the products. rpw comes from the entry count
+// read on the device: 32 rows while they hold about two tiles, fewer for longer rows, and (while
+// they hold more than 64) fewer while some warps of the grid would have no rows.
+// The next rows' offsets are loaded while these are summed. Loading the next tile's entries then,
+// too, made products of short rows 4% faster and those of uneven or long rows 12 to 50% slower.
 constexpr int kStream = 256;
 template <typename Epi, int FILL>
 static __global__ void __launch_bounds__(kThreads, 4)

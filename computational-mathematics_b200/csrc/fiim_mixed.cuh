@@ -3,9 +3,9 @@
 // (AFIIM/src/bicgstab.cpp:168-275), on FP32 vectors and FP32 (or BF16) matrix values.
 //
 // Inner iteration = the nine launches of the FP64 path, on 4-byte vectors:
-//   tm = D^{-1} o (H p); pc = G tm (+||pc||^2); v = A32 pc, alpha; s = r - alpha v (+||r||^2,
-//   ||e||^2); tm = D^{-1} o (H s); sc = G tm; t = A32 sc, omega; e += alpha pc + omega sc,
-//   r = s - omega t, m1 = r0.r, tests, beta; p = r + beta (p - omega v).
+//   tm = D^{-1} o (H p); pc = G tm (+ partial ||pc||^2); v = A32 pc, alpha; s = r - alpha v;
+//   tm = D^{-1} o (H s); sc = G tm; t = A32 sc, omega; e += alpha pc + omega sc, r = s - omega t,
+//   m1 = r0.r, the next ||r||^2 and ||e||^2, tests, beta; p = r + beta (p - omega v).
 // Matrix products accumulate in FP32 (rows summed in storage order from shared memory);
 // every dot product and norm accumulates FP32 products in FP64, and the recurrence scalars
 // (alpha, omega, beta, rho) are FP64 in DState.

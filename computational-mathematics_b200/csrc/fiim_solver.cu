@@ -1380,9 +1380,10 @@ double Solver::iteration_bytes() const {
 }
 
 // ------------------------------------------------------------------ kernel-level API
-// One set-up-free product on s (k_spmv_stream). after_ours: the launch before it on s is ours and waited for all before itself, so this one may
-// read its matrix while that one finishes (programmatic dependent launch); otherwise the launch
-// before it may be the caller's, still writing the matrix.
+// One set-up-free product on s (k_spmv_stream). after_ours: the launch before it on s is ours and
+// waited for all before itself, so this one may read its matrix while that one finishes
+// (programmatic dependent launch); otherwise the launch before it may be the caller's, still
+// writing the matrix.
 template <int FILL, typename Epi>
 static cudaError_t launch_stream(cudaStream_t s, const CsrView<double> &M, const double *x, const Epi &epi, bool after_ours) {
     auto kern = k_spmv_stream<Epi, FILL>;
