@@ -817,13 +817,15 @@ int build_gpu(int n, const int *Ai, const int *Aj, const double *Av, const Param
             FIIM_CUDA(cudaMemcpyAsync(&no, novf, sizeof(int), cudaMemcpyDeviceToHost, st));
             FIIM_CUDA(cudaStreamSynchronize(st));
             if (no == 0) break;
-            std::vector<int> left(no);
-            FIIM_CUDA(cudaMemcpy(left.data(), ovf, sizeof(int) * no, cudaMemcpyDeviceToHost));
+            std::vector<int> left(no);   // on st, as the kernel that reads rows2: no stream orders another's copies
+            FIIM_CUDA(cudaMemcpyAsync(left.data(), ovf, sizeof(int) * no, cudaMemcpyDeviceToHost, st));
+            FIIM_CUDA(cudaStreamSynchronize(st));
             std::sort(left.begin(), left.end());
             if (c == 2)
                 return set_error(FIIM_EARG, "row %d's pattern outgrows %d members; use the host construction "
                                             "(fiim_pdfiim_build) or a warpsize cap", left[0], kCaps[2]);
-            FIIM_CUDA(cudaMemcpy(rows2, left.data(), sizeof(int) * no, cudaMemcpyHostToDevice));
+            FIIM_CUDA(cudaMemcpyAsync(rows2, left.data(), sizeof(int) * no, cudaMemcpyHostToDevice, st));
+            FIIM_CUDA(cudaStreamSynchronize(st));   // before the host rows go
             rows = rows2;
             nrows = no;
         }

@@ -48,3 +48,9 @@ def test_small(n):
 @pytest.mark.parametrize("norm", ["I", "1", "2"])
 def test_large_arrays(norm):
     same(FB.gen_convdiff3d(72, 0.4), 0.05, 2, 2, 1, -1, norm)
+
+
+def test_many_rows_outgrow_both_smaller_capacities():
+    """Five fill levels of the 7-point stencil reach up to 115 members: most of 21,952 rows are listed
+    and built again at 64 and then at 128."""
+    same(FB.gen_convdiff3d(28, 0.4), 0.02, 5, 1, 1)
