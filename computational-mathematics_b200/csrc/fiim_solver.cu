@@ -591,17 +591,19 @@ int check_fill_launch(DevCsr &M, int fill, cudaStream_t s, unsigned long long *d
     return FIIM_OK;
 }
 
-// After the stream has synchronized: compact M to its triangle if the check found entries
-// outside it.
-int check_fill_finish(DevCsr &M, int fill, unsigned long long outside) {
+// After the stream s has synchronized: compact M to its triangle if the check found entries
+// outside it. The copies run on s, which orders them before the kernels that read M next (s waits
+// for no other stream), and are done when this returns.
+int check_fill_finish(DevCsr &M, int fill, unsigned long long outside, cudaStream_t s) {
     if (fill == 0 || outside == 0) return FIIM_OK;
     const int n = (int)M.n;
     const long nnz = M.nnz;
     std::vector<int> crp(n + 1), cci(nnz);
     std::vector<double> cv(nnz);
-    FIIM_CUDA(cudaMemcpy(crp.data(), M.rp, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost));
-    FIIM_CUDA(cudaMemcpy(cci.data(), M.ci, sizeof(int) * nnz, cudaMemcpyDeviceToHost));
-    FIIM_CUDA(cudaMemcpy(cv.data(), M.v, sizeof(double) * nnz, cudaMemcpyDeviceToHost));
+    FIIM_CUDA(cudaMemcpyAsync(crp.data(), M.rp, sizeof(int) * (n + 1), cudaMemcpyDeviceToHost, s));
+    FIIM_CUDA(cudaMemcpyAsync(cci.data(), M.ci, sizeof(int) * nnz, cudaMemcpyDeviceToHost, s));
+    FIIM_CUDA(cudaMemcpyAsync(cv.data(), M.v, sizeof(double) * nnz, cudaMemcpyDeviceToHost, s));
+    FIIM_CUDA(cudaStreamSynchronize(s));
     long c = 0;
     std::vector<int> nrp(n + 1, 0);
     for (int i = 0; i < n; ++i) {
@@ -616,11 +618,12 @@ int check_fill_finish(DevCsr &M, int fill, unsigned long long outside) {
         nrp[i + 1] = (int)c;
     }
     M.nnz = c;
-    FIIM_CUDA(cudaMemcpy(M.rp, nrp.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice));
+    FIIM_CUDA(cudaMemcpyAsync(M.rp, nrp.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice, s));
     if (c > 0) {
-        FIIM_CUDA(cudaMemcpy(M.ci, cci.data(), sizeof(int) * c, cudaMemcpyHostToDevice));
-        FIIM_CUDA(cudaMemcpy(M.v, cv.data(), sizeof(double) * c, cudaMemcpyHostToDevice));
+        FIIM_CUDA(cudaMemcpyAsync(M.ci, cci.data(), sizeof(int) * c, cudaMemcpyHostToDevice, s));
+        FIIM_CUDA(cudaMemcpyAsync(M.v, cv.data(), sizeof(double) * c, cudaMemcpyHostToDevice, s));
     }
+    FIIM_CUDA(cudaStreamSynchronize(s));   // before the host arrays go
     M.hrp.swap(nrp);
     M.rows_same = false;   // the stored offsets are the filtered ones
     signature(M, M.hrp.data());
@@ -633,7 +636,7 @@ int upload_csr(DevCsr &M, long nnz_cap, int n, const int *rp, const int *ci, con
     if (fill == 0 || M.nnz == 0) return FIIM_OK;
     FIIM_TRY(check_fill_launch(M, fill, s, d_count, h_count));
     FIIM_CUDA(cudaStreamSynchronize(s));
-    return check_fill_finish(M, fill, *h_count);
+    return check_fill_finish(M, fill, *h_count, s);
 }
 
 // Uploads of the solver's matrices: every copy and triangle check issued, then one sync.
@@ -647,7 +650,7 @@ static int upload_all(DevCsr *const *mats, const long *caps, const int *const *r
     }
     for (int k = 0; k < count; ++k) FIIM_TRY(check_fill_launch(*mats[k], fills[k], s, d_count + k, h_count + k));
     FIIM_CUDA(cudaStreamSynchronize(s));
-    for (int k = 0; k < count; ++k) FIIM_TRY(check_fill_finish(*mats[k], fills[k], h_count[k]));
+    for (int k = 0; k < count; ++k) FIIM_TRY(check_fill_finish(*mats[k], fills[k], h_count[k], s));
     return FIIM_OK;
 }
 

@@ -159,3 +159,32 @@ def test_batch_with_and_without_shared_blocks(monkeypatch, precision):
     assert np.array_equal(out["1"][0]["info"], out["0"][0]["info"]) and not out["1"][0]["info"].any()
     assert np.all(np.abs(out["1"][0]["iter"] - out["0"][0]["iter"]) <= 2)
     assert np.linalg.norm(out["1"][1] - out["0"][1]) <= 1e-7 * np.linalg.norm(out["0"][1])
+
+
+def test_entries_outside_the_triangles_of_a_large_system():
+    """G with entries below its diagonal and H with entries above: the solver reads the triangles only,
+    through the sliced copies laid out of what is left, bit for bit as if they were given alone."""
+    side = 48
+    A = FB.gen_convdiff3d(side, 0.5)
+    n = side ** 3
+    F = FB.pdfiim_build(A, 0.05, 2, 2, 1)
+
+    def widened(rp, ci, v, upper):
+        rows = np.repeat(np.arange(n), np.diff(rp))
+        other = np.arange(side, n) if upper else np.arange(n - side)      # one entry on the other side
+        r = np.concatenate([rows, other])
+        c = np.concatenate([ci, other - side if upper else other + side])
+        w = np.concatenate([v, np.full(len(other), 3.0)])
+        order = np.lexsort((c, r))
+        ptr = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]).astype(np.int32)
+        return ptr, c[order].astype(np.int32), w[order]
+
+    G, H = widened(F["Gi"], F["Gj"], F["Gv"], True), widened(F["Hi"], F["Hj"], F["Hv"], False)
+    W = dict(F, Gi=G[0], Gj=G[1], Gv=G[2], Hi=H[0], Hj=H[1], Hv=H[2])
+    b, out = FB.rand_normal(n, 9), []
+    for f in (F, W):
+        with FB.Solver(A, f, variant="pdfiim") as S:
+            x = np.zeros(n)
+            r = S.solve(b, x, tol=1e-10, nmax=300)
+            out.append((r["iter"], x, S.spmv_shape(1)[1], S.spmv_shape(2)[1]))
+    assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1]) and out[0][2:] == out[1][2:] == (3, 3)
