@@ -104,6 +104,19 @@ struct DevCsr {
 // total at most tile; a row with more than tile entries forms a block by itself.
 void build_row_blocks(const std::vector<int> &rp, int tile, int max_rows, std::vector<int> &rb);
 
+// A run of entries [b, e) of a CSR matrix, walked a step at a time. Positions are unsigned and the end is told
+// by what is left, so nothing wraps, however close the end is to the last entry an int can count.
+struct EntryRun {
+    unsigned at, left;
+    __host__ __device__ EntryRun(int b, int e) : at((unsigned)b), left(e > b ? (unsigned)(e - b) : 0u) {}
+    __host__ __device__ bool more() const { return left > 0; }
+    __host__ __device__ bool has(int k) const { return (unsigned)k < left; }   // entry k of the step
+    __host__ __device__ void next(int step) {
+        at += (unsigned)step;
+        left = left > (unsigned)step ? left - (unsigned)step : 0u;
+    }
+};
+
 // Host CSR (owning), used for symmetric expansion and transposes.
 struct HostCsr {
     int n = 0;

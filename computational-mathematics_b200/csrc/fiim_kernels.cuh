@@ -37,6 +37,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <climits>
+
 #include "fiim_internal.h"
 
 namespace fiim {
@@ -1319,18 +1321,19 @@ k_spmv_stream(CsrView<double> M, const double *__restrict__ x, Epi epi) {
     int *col = col_all[FILL ? w : 0];
     const long nw = (long)gridDim.x * kWarps;
     const long nnz = __ldg(M.rp + M.n);
-    int rpw = 32;
+    // the tiles' int positions have to end below INT_MAX: past that a warp a row, whose walk does not wrap
+    int rpw = nnz > INT_MAX - 2 * kStream ? 1 : 32;
     while (rpw > 1 && (rpw * nnz > 2L * kStream * M.n || (M.n < nw * rpw && rpw * nnz > 64L * M.n))) rpw >>= 1;
     if (rpw == 1) {   // long rows: a warp each, its products passed to the sum lane by lane
         pdl_enter();
         for (long row = (long)blockIdx.x * kWarps + w; row < M.n; row += nw) {
-            const int e1 = __ldg(M.rp + row + 1);
             double s = 0.0;
-            for (int t0 = __ldg(M.rp + row); t0 < e1; t0 += 32) {
-                const int e = t0 + lane, c = e < e1 ? ldi(M.ci + e) : 0;
+            for (EntryRun t(__ldg(M.rp + row), __ldg(M.rp + row + 1)); t.more(); t.next(32)) {
+                const bool in = t.has(lane);
+                const int c = in ? ldi(M.ci + t.at + lane) : 0;
                 // what is not added is a zero: a sum that starts at +0 is never -0, so +0 leaves it as it is
-                const bool keep = e < e1 && (FILL == 0 || (FILL == 1 ? c >= row : c <= row));
-                const double p = keep ? __dmul_rn(ldm(M.v + e), ldx(x + c)) : 0.0;
+                const bool keep = in && (FILL == 0 || (FILL == 1 ? c >= row : c <= row));
+                const double p = keep ? __dmul_rn(ldm(M.v + t.at + lane), ldx(x + c)) : 0.0;
 #pragma unroll
                 for (int j = 0; j < 32; ++j) s = __dadd_rn(s, __shfl_sync(full, p, j));
             }
