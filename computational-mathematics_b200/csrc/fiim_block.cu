@@ -71,8 +71,9 @@ struct BlockSolver {
                                                                           M.nblk, X, epi, bs, partials);
             return cudaGetLastError();
         };
-        if constexpr (L == 32 && VW == 1) return go(bk::k_spmm_stream<V, Epi>);
-        else return go(bk::k_spmm<L, VW, V, Epi>);
+        if constexpr (L == 32 && VW == 1)
+            if (bk::streams(M.nnz)) return go(bk::k_spmm_stream<V, Epi>);
+        return go(bk::k_spmm<L, VW, V, Epi>);
     }
 
     // Chunks of consecutive rows of about equal work (M.rb, M.nblk of them), whole steps of a warp

@@ -336,6 +336,11 @@ k_spmm(CsrView<V> M, Shape sh, const int *__restrict__ chunk, int nch, const dou
 // everywhere. Power-law matrix, n = 200,003, 2.9 M entries, 32 right-hand sides: A X 445 -> 152 us,
 // M X (FP32 factors) 176 -> 133, an iteration 1.53 -> 0.60 ms with the shorter reductions and
 // updates of this file.
+// Its int positions run up to two tiles past a run's end, so a matrix whose entries come that close to 2^31
+// keeps k_spmm, whose positions start at a row. (Positions compared by what is left, here, took 1.2% more:
+// 6.68 -> 6.76 ms for the ten iterations of the system above.)
+inline bool streams(long nnz) { return nnz <= INT_MAX - 64; }
+
 template <typename V, typename Epi>
 static __global__ void __launch_bounds__(kThreads, 4)
 k_spmm_stream(CsrView<V> M, Shape sh, const int *__restrict__ chunk, int nch, const double *__restrict__ X, Epi epi, BState bs,
