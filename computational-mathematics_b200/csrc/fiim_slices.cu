@@ -261,8 +261,11 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
         return !st.refused && !st.pad && st.max_m <= kDiaMaxDiags && dia < csr && 32.0 * R * (double)st.ndiag < 2147483648.0;
     };
     // Shared when at most half of the slices differ; otherwise the class numbers cost a load in
-    // front of every block and most blocks are read once.
-    auto sharing = [&](int nsl) { return share_on && 2L * st.uniq <= nsl; };
+    // front of every block and most blocks are read once. k_spmv_cls counts the blocks' values, whole quads of
+    // diagonals, in ints.
+    auto sharing = [&](int R, int nsl) {
+        return share_on && 2L * st.uniq <= nsl && 32L * R * (long)st.uniq_ndiag < (1L << 31);
+    };
     // FP64 slices that share take two rows a lane (k_spmv_cls). The others take two when their
     // 32-row slices average more diagonals than one chunk of the kernel holds (H at 128^3: 11
     // diagonals, 32.9 against 41.6 us a product; A and G, 7 diagonals, were slower with two).
@@ -278,12 +281,12 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
         nsl = slices(R);
         FIIM_TRY(scan(R, nsl));
         const bool two = smaller(R, nsl);
-        if (!two || !sharing(nsl)) {
+        if (!two || !sharing(R, nsl)) {
             R = 1;
             nsl = slices(R);
             FIIM_TRY(scan(R, nsl, kPackMax));
             dia = smaller(R, nsl);
-            if (dia && two && !sharing(nsl) && (long)st.ndiag > 8L * nsl) {
+            if (dia && two && !sharing(R, nsl) && (long)st.ndiag > 8L * nsl) {
                 R = 2;
                 nsl = slices(R);
                 FIIM_TRY(scan(R, nsl));
@@ -303,7 +306,7 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
         return build_pack(M, s, vals, nsl, st, m, id, k0);
     }
     const int sh = 32 * R, rs = record_ints();
-    for (bool share = sharing(nsl);; share = false) {
+    for (bool share = sharing(R, nsl);; share = false) {
         const int ncls = share ? st.uniq : nsl;
         const long ndiag = share ? (long)st.uniq_ndiag : (long)st.ndiag;
         const size_t b_rec = Arena::need(sizeof(int) * (size_t)rs * ncls),
