@@ -94,7 +94,9 @@ int oneshot(int variant, int issym, char mode, int nr, int n, const double *Av, 
     o.verbose = verbose;
     o.memory = FIIM_MEM_HOST;
     const bool combined = (variant == FIIM_ACIFIM && mode == 'C' && nr > 1);
-    std::vector<long> key = {variant, issym, (long)mode, combined ? nr : 1, n, Ai[n], Gi[n],
+    int dev = -1;   // a failure is reported by the set-up
+    if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError();
+    std::vector<long> key = {dev, variant, issym, (long)mode, combined ? nr : 1, n, Ai[n], Gi[n],
                              (!issym && Hi) ? Hi[n] : -1, (combined && Li) ? Li[n] : -1,
                              (combined && Ui) ? Ui[n] : -1};
     // The arrays of the call in stamping order: address and size, and the content hash when asked.
@@ -142,7 +144,7 @@ int oneshot(int variant, int issym, char mode, int nr, int n, const double *Av, 
         FIIM_TRY(g_one.s->solve_finish(nullptr, nullptr));
     }
     g_one.stamps.clear();
-    int rc = FIIM_OK, dev = -1;
+    int rc = FIIM_OK;
     if (g_one.s && g_one.key == key && !issym) {
         g_one.s->opt.verbose = verbose;
         rc = g_one.s->stage_inputs(b, x);   // ahead of the matrix copies
@@ -150,12 +152,13 @@ int oneshot(int variant, int issym, char mode, int nr, int n, const double *Av, 
         if (rc != FIIM_OK) g_one.s->inputs_staged = false;
     } else {
         // Another shape: set the thread's solver up again, in the memory, stream and events it has
-        // (on the device it was made on; a thread that moved gets a new one).
+        // (on the device it was made on; a thread that moved gets a new one on its present device).
         g_one.key.clear();
-        if (g_one.s && (cudaGetDevice(&dev) != cudaSuccess || dev != g_one.s->device)) {
-            g_one.s->destroy();
+        if (g_one.s && dev != g_one.s->device) {
+            g_one.s->destroy();   // leaves its device current
             delete g_one.s;
             g_one.s = nullptr;
+            if (dev >= 0) FIIM_CUDA(cudaSetDevice(dev));
         }
         auto *s = g_one.s ? g_one.s : new fiim::Solver;
         rc = s->create(n, Ai, Aj, Av, Gi, Gj, Gv, IDv, Hi, Hj, Hv, Li, Lj, Lv, Ui, Uj, Uv, o);

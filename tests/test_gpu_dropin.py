@@ -71,3 +71,21 @@ def test_threads():
     for t in threads:
         t.join()
     assert not errors, errors
+
+
+def test_a_thread_that_moves_to_another_device():
+    """The same shape again after the thread's current device changed: solved there, and left current."""
+    import torch
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two GPUs")
+    s = system((33, 3))
+    try:
+        for dev in (0, 1, 0):
+            torch.cuda.set_device(dev)
+            before = torch.cuda.mem_get_info(dev)[0]
+            check([s])
+            assert torch.cuda.current_device() == dev
+            if dev == 1:
+                assert torch.cuda.mem_get_info(dev)[0] < before
+    finally:
+        torch.cuda.set_device(0)
