@@ -239,8 +239,9 @@ int grid_for(K kernel, long units_per_block, long units) {
     return (int)std::min<long>(need, (long)occupancy(kernel) * num_sms());
 }
 
-// CTAs of k_spmv_dia with one row a lane (four per SM, at most one 32-row slice a warp when the
-// matrix is small): the grid whose summation tree the sliced forms share.
+// The grid of the sliced-diagonal products whose sums steer the iteration, for one row a lane (four
+// CTAs per SM, at most one 32-row slice a warp when the matrix is small). A property of the sums'
+// tree, not of a kernel's occupancy: such products are launched on it whatever that is.
 inline int dia_grid(long n) {
     return (int)std::min<long>((n + 32 * 8 - 1) / (32 * 8), 4L * num_sms());
 }

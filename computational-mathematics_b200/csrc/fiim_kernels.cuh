@@ -285,9 +285,14 @@ struct FinInit {   // ro = ||r0||, m1 = ro^2, rc = ro (AFIIM/src/bicgstab.cpp:16
     static constexpr bool REDUCES = reduces;      \
     static constexpr bool GATED = gated
 
-// An epilogue whose sums steer the iteration (r0, alpha, omega) declares STEERS: their summation
-// tree is the same in the sliced forms with and without shared blocks (k_spmv_cls), so a solve's
-// iterates do not depend on which of them serves A.
+// An epilogue whose sums steer the iteration (r0, alpha, omega) declares STEERS: k_spmv_cls, with one
+// and two rows a lane, adds them in the tree of k_spmv_dia with one row a lane on dia_grid CTAs, so
+// there a solve's iterates do not depend on whether A's slices share blocks. Slices with their own
+// blocks and more than eight diagonals on average take two rows a lane, and k_spmv_dia then adds a
+// lane's neighbouring rows first: another tree. (In the one tree, half as many warps for the same
+// rows, A's products took up to 12% more at 12 diagonals and 20% at 27: 31.1 -> 34.8 us at 10^6 rows,
+// 53.2 -> 64.6 at 100^3.) Which form serves is a function of the matrix alone, after a reload as
+// after a set-up (fiim_slices.cu).
 template <typename E, typename = void>
 struct Steers : std::false_type {};
 template <typename E>
@@ -1075,8 +1080,8 @@ __device__ __forceinline__ void cls_slice(const DiaView<V> &M, const T *__restri
 // arithmetic: G 17.1 / 14.0 against 21.7 / 17.9 us with one, A 20.3 / 18.1 against 24.5 / 22.4,
 // and every slice reading its own block 26.2 / 23.7 and 34.2 / 30.5 (H 21.3 against 39.0), all at
 // 128^3 in the body's order, constant coefficients.
-// An epilogue that steers the iteration sums as k_spmv_dia with one row a lane would: vgrid is
-// that kernel's grid, and warp g takes the slices of its warps 2 g (rows first + lane) and
+// An epilogue that steers the iteration sums as k_spmv_dia with one row a lane does: vgrid is
+// that kernel's grid (dia_grid), which one row a lane takes itself; with two, warp g takes the slices of its warps 2 g (rows first + lane) and
 // 2 g + 1 (rows first + 32 + lane), each with its own running sums.
 template <typename Epi, int R>
 constexpr bool kClsPairs = Steers<Epi>::value && R == 2;
@@ -1118,7 +1123,7 @@ cudaError_t spmv_cls(cudaStream_t s, const M &m, const DiaView<V> &view, const T
                      double *partials) {
     auto go = [&](auto kern, bool pairs) {
         const int vgrid = dia_grid(m.n);
-        const int grid = pairs ? (vgrid + 1) / 2 : grid_for(kern, kWarps, m.nsl);
+        const int grid = pairs ? (vgrid + 1) / 2 : Steers<Epi>::value ? vgrid : grid_for(kern, kWarps, m.nsl);
         return launch_k(kern, grid, 0, s, view, x, epi, st, partials, vgrid);
     };
     if constexpr (sizeof(V) == 8) {

@@ -208,9 +208,12 @@ static cudaError_t spmv_dia(cudaStream_t s, const DevCsr &M, const double *x, co
                             double *partials) {
     if (M.dseg) return cudaErrorInvalidValue;   // k_spmv_dia takes slices of one segment
     const DiaView<double> view = dia_view<double>(M);
-    auto go = [&](auto kern) { return launch_k(kern, grid_for(kern, kWarps, M.nsl), 0, s, view, x, epi, st, partials); };
+    auto go = [&](auto kern, int grid) { return launch_k(kern, grid, 0, s, view, x, epi, st, partials); };
+    auto full = [&](auto kern) { return grid_for(kern, kWarps, M.nsl); };
     if (M.dcls) return spmv_cls<double, double>(s, M, view, x, epi, st, partials);
-    return M.dsh == 64 ? go(k_spmv_dia<double, double, 2, Epi>) : go(k_spmv_dia<double, double, 1, Epi>);
+    if (M.dsh == 64) return go(k_spmv_dia<double, double, 2, Epi>, full(k_spmv_dia<double, double, 2, Epi>));
+    auto kern = k_spmv_dia<double, double, 1, Epi>;
+    return go(kern, Steers<Epi>::value ? dia_grid(M.n) : full(kern));
 }
 
 // Solver SpMV: the sliced-diagonal copy where the matrix has one, else CSR-stream over the

@@ -188,3 +188,69 @@ def test_entries_outside_the_triangles_of_a_large_system():
             r = S.solve(b, x, tol=1e-10, nmax=300)
             out.append((r["iter"], x, S.spmv_shape(1)[1], S.spmv_shape(2)[1]))
     assert out[0][0] == out[1][0] and np.array_equal(out[0][1], out[1][1]) and out[0][2:] == out[1][2:] == (3, 3)
+
+
+def stencil(sides, points, kind):
+    """The 7-, 19- or 27-point stencil on a box, with constant or varying entries."""
+    nx, ny, nz = sides
+    n = nx * ny * nz
+    i = np.arange(n)
+    at = (i // (nx * ny), i // nx % ny, i % nx)
+    steps = [(a, b, c) for a in (-1, 0, 1) for b in (-1, 0, 1) for c in (-1, 0, 1)
+             if abs(a) + abs(b) + abs(c) <= {7: 1, 19: 2, 27: 3}[points]]
+    inside = np.stack([np.all([(0 <= q + d) & (q + d < m) for q, d, m in zip(at, s, (nz, ny, nx))], axis=0)
+                       for s in steps], axis=1)
+    cols = np.stack([i + (s[0] * ny + s[1]) * nx + s[2] for s in steps], axis=1)
+    v = np.stack([np.where(s == (0, 0, 0), 30.0, -1.0 / (1 + sum(map(abs, s)))) + 0.0 * i for s in steps], axis=1)
+    if kind == "varying":
+        v *= 1.0 + 0.1 * np.sin(0.7 * np.arange(n))[:, None]
+    rp = np.concatenate([[0], np.cumsum(inside.sum(1))]).astype(np.int32)
+    return rp, cols[inside].astype(np.int32), v[inside]
+
+
+# the last box: several slices a warp of the products' grid
+BOXES = [(37, 41, 23), (33, 32, 32), (67, 64, 63)]
+
+
+def solves(monkeypatch, A, envs):
+    """(iterations, x) of one solve with A served as each environment says."""
+    n = len(A[0]) - 1
+    b, out = FB.rand_normal(n, 5), []
+    for env in envs:
+        for k, v in env.items():
+            monkeypatch.setenv(k, v)
+        x = np.full(n, 0.25)
+        with FB.Solver(A, identity_factors(n)) as S:
+            r = S.solve(b, x, tol=1e-11, nmax=100)
+            assert S.spmv_shape(0)[1] == 3 and S.mode() < 2, env
+        for k in env:
+            monkeypatch.delenv(k)
+        assert r["info"] == 0
+        out.append((r["iter"], x))
+    return b, out
+
+
+@pytest.mark.parametrize("kind", ["constant", "varying"])
+@pytest.mark.parametrize("sides", BOXES, ids=lambda s: "x".join(map(str, s)))
+def test_sharing_leaves_the_iterates_alone(monkeypatch, sides, kind):
+    """Seven diagonals: with shared blocks (one and two rows a lane) and with a block a slice, the sums that
+    steer the solve have one tree, so x is the same bit for bit."""
+    envs = ({}, {"FIIM_DIA_SHARE": "0"}, {"FIIM_DIA_R": "1"}, {"FIIM_DIA_SHARE": "0", "FIIM_DIA_R": "1"})
+    _, out = solves(monkeypatch, stencil(sides, 7, kind), envs)
+    for env, (its, x) in zip(envs[1:], out[1:]):
+        assert its == out[0][0] and np.array_equal(x, out[0][1]), env
+
+
+@pytest.mark.parametrize("points", [19, 27])
+@pytest.mark.parametrize("sides", BOXES, ids=lambda s: "x".join(map(str, s)))
+def test_wide_stencils_with_and_without_sharing(monkeypatch, sides, points):
+    """More than eight diagonals: a block a slice means two rows a lane and another tree. Both solutions
+    leave a residual below 1e-11 of the start's, and the symmetric A has 30 on its diagonal and at most 9
+    beside it, so its inverse is at most 1 / 21: they differ by no more than twice that. One row a lane has
+    the shared blocks' tree."""
+    A = stencil(sides, points, "constant")
+    n = len(A[0]) - 1
+    b, out = solves(monkeypatch, A, ({}, {"FIIM_DIA_SHARE": "0"}, {"FIIM_DIA_SHARE": "0", "FIIM_DIA_R": "1"}))
+    r0 = np.linalg.norm(b - O.csr_mv(*A, np.full(n, 0.25)))
+    assert np.linalg.norm(out[0][1] - out[1][1]) <= 2 * 1e-11 * r0 / 21 + 1e-13 * np.linalg.norm(out[0][1])
+    assert out[2][0] == out[0][0] and np.array_equal(out[2][1], out[0][1])
