@@ -91,6 +91,9 @@ struct DevCsr {
     int4 *khdr = nullptr;        // per slice: first record, records, first value
     int2 *krec = nullptr;        // offset and row mask of each slice's diagonals (ndiag of them)
     bool dia_tried = false;      // the copy was considered for the columns hashed in dia_cols
+    int dia_fit = 0;             // R set: for these columns, R rows a lane move fewer bytes than the CSR streams
+    bool dia_pad = false;        // refused for a value that holds the padding pattern
+    void *dscan = nullptr;       // scratch of the class count that a refresh repeats (its own allocation)
     unsigned long long dia_cols = 0;
     unsigned long long *dhash = nullptr;   // device scratch of the column hash (in the arena)
     std::vector<int> hseg_sl;    // first slice of each segment (host), segments + 1 entries
@@ -170,7 +173,8 @@ int build_narrow(DevCsr &M, cudaStream_t s);
 // fewer bytes than the CSR streams; otherwise M keeps the CSR streams. Slices with the same
 // diagonals and values share one record and block (FIIM_DIA_SHARE=0: none do).
 // refresh_dia, after new FP64 values M.v (and possibly new columns) with the same row offsets,
-// keeps or re-places the values where the copy allows it and builds it again otherwise.
+// keeps or re-places the values where the copy allows it and build_dia would choose the same form
+// for them (the slices' classes are counted again), and builds it again otherwise.
 // refresh_dia_async enqueues the same on `aux`, after the copies issued on `copy_s` before the
 // call, so it runs while later copies do; once `aux` is done, *h_bad (pinned) is 0 when the
 // copy holds the new values, else they are not to be used and refresh_dia decides again.

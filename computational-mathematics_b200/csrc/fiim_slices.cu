@@ -42,6 +42,10 @@ int dia_rows_per_lane(int vbytes) {
 
 void release_dia(DevCsr &M) {
     if (M.dia_mem) cudaFree(M.dia_mem);
+    if (M.dscan) cudaFree(M.dscan);
+    M.dscan = nullptr;
+    M.dia_fit = 0;
+    M.dia_pad = false;
     M.dia_mem = nullptr;
     M.dia_bytes = 0;
     M.drec = M.dcls = nullptr;
@@ -258,14 +262,12 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
     auto smaller = [&](int R, int nsl) {
         const double dia = (double)vbytes * 32 * R * (double)st.ndiag + 4.0 * record_ints() * nsl;
         const double csr = (double)nnz * (vbytes + (M.narrow ? 2 : 4)) + 4.0 * (n + 1);
-        return !st.refused && !st.pad && st.max_m <= kDiaMaxDiags && dia < csr && 32.0 * R * (double)st.ndiag < 2147483648.0;
+        const bool fits = !st.refused && st.max_m <= kDiaMaxDiags && dia < csr && 32.0 * R * (double)st.ndiag < 2147483648.0;
+        if (fits) M.dia_fit |= R;
+        if (st.pad) M.dia_pad = true;
+        return fits && !st.pad;
     };
-    // Shared when at most half of the slices differ; otherwise the class numbers cost a load in
-    // front of every block and most blocks are read once. k_spmv_cls counts the blocks' values, whole quads of
-    // diagonals, in ints.
-    auto sharing = [&](int R, int nsl) {
-        return share_on && 2L * st.uniq <= nsl && 32L * R * (long)st.uniq_ndiag < (1L << 31);
-    };
+    auto sharing = [&](int R, int nsl) { return share_on && sl::sharing(st, R, nsl); };
     // FP64 slices that share take two rows a lane (k_spmv_cls). The others take two when their
     // 32-row slices average more diagonals than one chunk of the kernel holds (H at 128^3: 11
     // diagonals, 32.9 against 41.6 us a product; A and G, 7 diagonals, were slower with two).
@@ -360,13 +362,45 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
 
 // Enqueues the check that the copy still holds M's matrix with the values `vals`, and, for a
 // copy whose slices have their own blocks, the new values; stats.bad tells afterwards whether
-// it does (a copy with shared blocks holds only the very same values).
-static int enqueue_refresh(DevCsr &M, const void *vals, cudaStream_t s) {
-    const sl::Args a = copy_args(M, vals);
+// it does (a copy with shared blocks holds only the very same values) and build_dia would choose
+// this form for them: where shared blocks fit the columns, the different slices are counted again,
+// which reads the matrix once for each number of rows a lane that fits. ok = false: not enqueued,
+// the form has to be chosen anew.
+static int enqueue_refresh(DevCsr &M, const void *vals, cudaStream_t s, bool *ok) {
+    const bool recount = !M.dcls && M.dia_fit && M.dvbytes == 8 && !M.dseg && share_wanted();
+    const int nsl[2] = {(int)((M.n + 31) / 32), (int)((M.n + 63) / 64)};
+    unsigned table = 64;
+    while (table < 2U * (unsigned)nsl[0]) table <<= 1;
+    const size_t b_st = Arena::need(2 * sizeof(sl::Stats)), b_keys = Arena::need(8UL * table);
+    *ok = !M.dia_pad;
+    if (recount && !M.dscan && cudaMalloc(&M.dscan, b_st + 2 * b_keys) != cudaSuccess) {
+        cudaGetLastError();
+        M.dscan = nullptr;
+        *ok = false;
+    }
+    if (!*ok) return FIIM_OK;
+    sl::Args a = copy_args(M, vals);
     FIIM_CUDA(cudaMemsetAsync(M.dstat, 0, sizeof(sl::Stats), s));
     if (M.pack) FIIM_CUDA(pack(true, a, M.khdr, M.krec, s));
     else if (M.dcls) FIIM_CUDA((walk<sl::kVerify, true>(M.dsh / 32, M.dvbytes, a, s)));
     else FIIM_CUDA((walk<sl::kPlace, false>(M.dsh / 32, M.dvbytes, a, s)));
+    if (!recount) return FIIM_OK;
+    FIIM_CUDA(cudaMemsetAsync(M.dscan, 0, b_st + 2 * b_keys, s));
+    char *mem = static_cast<char *>(M.dscan);
+    sl::Stats *count = reinterpret_cast<sl::Stats *>(mem);
+    a.most = kDiaMaxDiags;
+    a.mask = table - 1;
+    a.cls = nullptr;
+    for (int R = 1; R <= 2; ++R) {
+        if (!(M.dia_fit & R)) continue;
+        a.nsl = nsl[R - 1];
+        a.stats = count + (R - 1);
+        a.keys = reinterpret_cast<unsigned long long *>(mem + b_st + (R - 1) * b_keys);
+        FIIM_CUDA((walk<sl::kCount, true>(R, 8, a, s)));
+    }
+    sl::k_recheck<<<1, 1, 0, s>>>(make_int2(M.dia_fit & 1 ? nsl[0] : 0, M.dia_fit & 2 ? nsl[1] : 0), count,
+                                  reinterpret_cast<sl::Stats *>(M.dstat));
+    FIIM_CUDA(cudaGetLastError());
     return FIIM_OK;
 }
 
@@ -375,10 +409,12 @@ int refresh_dia(DevCsr &M, cudaStream_t s) {
     if (!M.dia && !M.pack) {   // not built for the previous columns: decide again only if they changed
         unsigned long long h = 0;
         FIIM_TRY(col_hash(M, s, &h));
-        if (M.dia_tried && h == M.dia_cols) return FIIM_OK;
+        if (M.dia_tried && h == M.dia_cols && !M.dia_fit) return FIIM_OK;   // whatever the values
         return build_dia(M, s, 8, M.v);
     }
-    FIIM_TRY(enqueue_refresh(M, M.v, s));
+    bool ok = false;
+    FIIM_TRY(enqueue_refresh(M, M.v, s, &ok));
+    if (!ok) return build_dia(M, s, 8, M.v);
     sl::Stats st{};
     FIIM_CUDA(cudaMemcpyAsync(&st, M.dstat, sizeof st, cudaMemcpyDeviceToHost, s));
     FIIM_CUDA(cudaStreamSynchronize(s));
@@ -389,7 +425,10 @@ int refresh_dia(DevCsr &M, cudaStream_t s) {
 int refresh_dia_async(DevCsr &M, cudaStream_t copy_s, cudaStream_t aux, cudaEvent_t done, int *h_bad) {
     FIIM_CUDA(cudaEventRecord(done, copy_s));
     FIIM_CUDA(cudaStreamWaitEvent(aux, done, 0));
-    FIIM_TRY(enqueue_refresh(M, M.v, aux));
+    bool ok = false;
+    *h_bad = 1;
+    FIIM_TRY(enqueue_refresh(M, M.v, aux, &ok));
+    if (!ok) return FIIM_OK;
     FIIM_CUDA(cudaMemcpyAsync(h_bad, &reinterpret_cast<sl::Stats *>(M.dstat)->bad, sizeof(int), cudaMemcpyDeviceToHost, aux));
     return FIIM_OK;
 }

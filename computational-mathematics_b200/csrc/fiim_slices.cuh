@@ -26,6 +26,13 @@ struct Stats {
     int bad;                         // verify / place: the copy does not hold these values
 };
 
+// Shared blocks serve slices of which at most half differ: otherwise the class numbers cost a load
+// in front of every block and most blocks are read once. k_spmv_cls counts the blocks' values, whole
+// quads of diagonals, in ints.
+__host__ __device__ inline bool sharing(const Stats &st, int R, int nsl) {
+    return 2L * st.uniq <= nsl && 32L * R * (long)st.uniq_ndiag < (1L << 31);
+}
+
 struct Args {
     int n, nsl;
     int most;                        // scan: diagonals of one slice at most
@@ -36,6 +43,8 @@ struct Args {
     Stats *stats;
     int *m;                          // scan: diagonals per slice
     unsigned long long *hash;        // scan: hash of a slice's record and values
+    unsigned long long *keys;        // count: table of the hashes met (k_insert), 0 empty
+    unsigned mask;
     // the copy (write, verify, place)
     int *rec;
     int rs;
@@ -45,7 +54,7 @@ struct Args {
     const int *rep;                  // the class's first slice (write; null: every slice writes)
 };
 
-enum { kScan, kWrite, kVerify, kPlace };
+enum { kScan, kCount, kWrite, kVerify, kPlace };   // count: a scan that leaves only the different slices' number
 
 template <typename B>
 __device__ __forceinline__ B pad_bits() {
@@ -54,10 +63,27 @@ __device__ __forceinline__ B pad_bits() {
     else return (B)kDiaPad16;
 }
 
+// The place of hash h in an open-addressing table (0 empty), claimed if nobody did: (claimed, place). The table
+// holds more places than hashes, so an empty or equal one exists.
+struct Claim {
+    bool first;
+    unsigned at;
+};
+__device__ __forceinline__ Claim claim(unsigned long long *keys, unsigned mask, unsigned long long h) {
+    unsigned at = (unsigned)h & mask;
+    for (;;) {
+        const unsigned long long was = atomicCAS(keys + at, 0ULL, h);
+        if (was == 0ULL || was == h) return Claim{was == 0ULL, at};
+        at = (at + 1) & mask;
+    }
+}
+__device__ __forceinline__ int quads(int m) { return (m + kDiaQuad - 1) & -kDiaQuad; }   // shared blocks hold whole quads
+
 // LANES: lane l owns the rows first + l + 32 j (shared blocks), else first + R l + j.
 template <int R, typename B, int MODE, bool LANES>
 static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
     constexpr int SH = 32 * R;
+    constexpr bool SCAN = MODE == kScan || MODE == kCount;
     const unsigned full = 0xffffffffu;
     const int lane = (int)threadIdx.x & 31;
     auto slot_of = [&](int j) { return LANES ? lane + 32 * j : R * lane + j; };   // row - first
@@ -67,7 +93,7 @@ static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
     int max_m = 0;
     for (int s = (int)blockIdx.x * kWarps + ((int)threadIdx.x >> 5); s < a.nsl; s += (int)gridDim.x * kWarps) {
         // refused already: random matrices end at once (one lane's read, so the warp agrees)
-        if (MODE == kScan && __shfl_sync(full, *(volatile int *)&a.stats->refused, 0)) break;
+        if (SCAN && __shfl_sync(full, *(volatile int *)&a.stats->refused, 0)) break;
         const int c = a.cls ? __ldg(a.cls + s) : s;
         if (MODE == kWrite && a.rep && __ldg(a.rep + s) != s) continue;
         int first = s * SH, rows = min(SH, a.n - s * SH);
@@ -76,7 +102,7 @@ static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
             first = q.x;
             rows = q.y;
         }
-        int *rec = MODE == kScan ? nullptr : a.rec + (long)c * a.rs;
+        int *rec = SCAN ? nullptr : a.rec + (long)c * a.rs;
         int k0 = 0, m_have = 0;
         if (MODE == kWrite) k0 = __ldg(a.k0 + s);
         if (MODE == kVerify || MODE == kPlace) {
@@ -103,8 +129,8 @@ static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
             for (int j = 1; j < R; ++j) d = min(d, cur[j]);
             d = __reduce_min_sync(full, d);
             if (d == INT_MAX) break;
-            if (k == (MODE == kScan ? a.most : a.rs - kDiaRecHead) || (MODE >= kVerify && k == m_have)) {
-                if (MODE == kScan) refused = true;
+            if (k == (SCAN ? a.most : a.rs - kDiaRecHead) || (MODE >= kVerify && k == m_have)) {
+                if (SCAN) refused = true;
                 else bad = true;
                 break;
             }
@@ -115,7 +141,7 @@ static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
                 bad = true;
                 break;
             }
-            if (MODE == kScan) h = mix64(h ^ (unsigned)d);
+            if (SCAN) h = mix64(h ^ (unsigned)d);
 #pragma unroll
             for (int j = 0; j < R; ++j) {
                 B o = pad_bits<B>();
@@ -128,7 +154,7 @@ static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
                     cur[j] = nd;
                 }
                 const long slot = (long)(k0 + k) * SH + R * lane + j;
-                if (MODE == kScan) h = mix64(h ^ (unsigned long long)o);
+                if (SCAN) h = mix64(h ^ (unsigned long long)o);
                 if (MODE == kWrite || MODE == kPlace) dv[slot] = o;
                 if (MODE == kVerify && dv[slot] != o) bad = true;
             }
@@ -143,18 +169,25 @@ static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
         refused = __any_sync(full, refused);
         pad = __any_sync(full, pad);
         bad = __any_sync(full, bad);
-        if (MODE == kScan) {
+        if (SCAN) {
             h = mix64(h ^ ((unsigned long long)(lane + 1) << 32));
             for (int o = 16; o > 0; o >>= 1) h += __shfl_xor_sync(full, h, o);
             h = mix64(h ^ (unsigned)(k | clamp));
         }
         if (lane == 0) {
+            if (SCAN) {
+                if (h == 0ULL) h = 1ULL;   // 0 marks an empty slot of the table
+                if (refused) atomicExch(&a.stats->refused, 1);
+            }
             if (MODE == kScan) {
                 a.m[s] = k;
-                a.hash[s] = h ? h : 1ULL;   // 0 marks an empty slot of the table
+                a.hash[s] = h;
                 sum_m += (unsigned)k;
                 max_m = max(max_m, k);
-                if (refused) atomicExch(&a.stats->refused, 1);
+            }
+            if (MODE == kCount && claim(a.keys, a.mask, h).first) {
+                ++max_m;
+                sum_m += (unsigned)quads(k);
             }
             if (MODE == kWrite) {
                 rec[0] = k0;
@@ -168,6 +201,10 @@ static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
     if (MODE == kScan && lane == 0 && max_m) {
         atomicAdd(&a.stats->ndiag, sum_m);
         atomicMax(&a.stats->max_m, max_m);
+    }
+    if (MODE == kCount && lane == 0 && max_m) {   // the slices this warp met first
+        atomicAdd(&a.stats->uniq, max_m);
+        atomicAdd(&a.stats->uniq_ndiag, sum_m);
     }
 }
 
@@ -234,13 +271,7 @@ static __global__ void __launch_bounds__(kThreads)
 k_insert(int nsl, const unsigned long long *__restrict__ hash, unsigned long long *keys, int *first, unsigned mask,
          int *slot) {
     FIIM_FOR_ROWS(s, nsl) {
-        const unsigned long long h = hash[s];
-        unsigned at = (unsigned)h & mask;
-        for (;;) {   // at most nsl < table size keys: an empty or equal slot exists
-            const unsigned long long was = atomicCAS(keys + at, 0ULL, h);
-            if (was == 0ULL || was == h) break;
-            at = (at + 1) & mask;
-        }
+        const unsigned at = claim(keys, mask, hash[s]).at;
         atomicMin(first + at, (int)s);
         slot[s] = (int)at;
     }
@@ -256,7 +287,7 @@ k_reps(int nsl, const int *__restrict__ first, const int *__restrict__ slot, con
         rep[s] = first[slot[s]];
         if (rep[s] == (int)s) {
             ++c;
-            d += (unsigned)((m[s] + kDiaQuad - 1) & -kDiaQuad);   // shared blocks hold whole quads
+            d += (unsigned)quads(m[s]);
         }
     }
     for (int o = 16; o > 0; o >>= 1) {
@@ -269,6 +300,16 @@ k_reps(int nsl, const int *__restrict__ first, const int *__restrict__ slot, con
     }
 }
 
+// Whether a count of the slices in the values a copy with own blocks now holds (for R = 1, 2 where nsl[R - 1]
+// is not 0) finds what would be shared: then the copy is not the form build_dia would choose for them.
+static __global__ void k_recheck(int2 nsl, const Stats *__restrict__ count, Stats *copy) {
+    for (int R = 1; R <= 2; ++R) {
+        const Stats &st = count[R - 1];
+        const int k = R == 1 ? nsl.x : nsl.y;
+        if (k && !st.refused && !st.pad && sharing(st, R, k)) copy->bad = 1;
+    }
+}
+
 // In slice order, over the slices that write (all, or with rep those that are their own
 // representative): id[s] = how many came before, k0[s] = their diagonals. One CTA.
 static __global__ void __launch_bounds__(1024)
@@ -278,7 +319,7 @@ k_offsets(int nsl, const int *__restrict__ m, const int *__restrict__ rep, int *
     int basec = 0, based = 0;
     for (int s0 = 0; s0 < nsl; s0 += 1024) {
         const int s = s0 + t;
-        const int c = s < nsl && (!rep || rep[s] == s), d = c ? (rep ? (m[s] + kDiaQuad - 1) & -kDiaQuad : m[s]) : 0;
+        const int c = s < nsl && (!rep || rep[s] == s), d = c ? (rep ? quads(m[s]) : m[s]) : 0;
         int ic = c, dd = d;
         for (int o = 1; o < 32; o <<= 1) {
             const int uc = __shfl_up_sync(0xffffffffu, ic, o), ud = __shfl_up_sync(0xffffffffu, dd, o);

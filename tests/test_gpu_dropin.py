@@ -89,3 +89,41 @@ def test_a_thread_that_moves_to_another_device():
                 assert torch.cuda.mem_get_info(dev)[0] < before
     finally:
         torch.cuda.set_device(0)
+
+
+PADDING = np.uint64(0xFFF7D1A6B00C5A1D).view(np.float64)   # a NaN: the sliced copies' mark of an empty slot
+
+
+@pytest.mark.parametrize("points", [7, 19, 27])
+def test_reloads_choose_the_form_a_fresh_solver_would(points):
+    """One structure, its entries varying, constant and varying again, with and without an entry that holds
+    the sliced copies' padding pattern: the kept solver takes the new values in the form that a fresh one
+    would choose for them (shared blocks, a block a slice, the CSR streams), whose sums have different trees
+    in part, so x is the fresh solver's bit for bit."""
+    from test_gpu_slices import stencil
+    from test_gpu_solve import identity_factors
+    sides = (41, 37, 33)
+    A = {kind: stencil(sides, points, kind) for kind in ("varying", "constant")}
+    n = len(A["varying"][0]) - 1
+    F, b = identity_factors(n), FB.rand_normal(n, 11)
+    rng = np.random.default_rng(3)
+    for kind in ("varying", "constant"):
+        rp, ci, v = A[kind]
+        v = v.copy()
+        v[rng.integers(len(v))] = PADDING
+        A[kind + " pad"] = (rp, ci, v)
+        A[kind + " other"] = (rp, ci, A[kind][2] * 1.25)
+    order = ["varying", "constant", "varying other", "varying pad", "varying", "constant pad", "constant",
+             "constant other", "varying pad", "constant"]
+    prev = FB.dropin_cache(False)
+    try:
+        for step, kind in enumerate(order):
+            with FB.Solver(A[kind], F, variant="pdfiim") as S:
+                y = np.full(n, 0.25)
+                r1 = S.solve(b, y, tol=1e-9, nmax=60)
+            x = np.full(n, 0.25)
+            r = FB.EPBiCGSTAB_pdfiim(A[kind], b, 1e-9, 60, (F["Gi"], F["Gj"], F["Gv"]), F["IDv"],
+                                     (F["Hi"], F["Hj"], F["Hv"]), x)
+            assert np.array_equal(x, y, equal_nan=True) and r[1] == r1["iter"], (step, kind)
+    finally:
+        FB.dropin_cache(prev)
