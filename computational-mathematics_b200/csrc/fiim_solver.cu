@@ -885,12 +885,12 @@ int Solver::create(int n_, const int *Ai, const int *Aj, const double *Av, const
     bytes += (size_t)(nvec + 1) * Arena::need(sizeof(double) * n);
     const int max_blocks = num_sms() * 32;
     bytes += Arena::need(sizeof(DState)) + Arena::need(sizeof(double) * 4 * max_blocks) + Arena::need(16) + 1024;
-    FIIM_TRY(arena.reserve(bytes));
     inputs_staged = false;
-    for (DevCsr *M : {&A, &G, &H, &L, &U}) {   // a solver set up before: nothing of it is kept but the memory
-        release_dia(*M);
+    for (DevCsr *M : {&A, &G, &H, &L, &U}) {   // a solver set up before: nothing of it is kept but the arena
+        release_dia(*M);                       // before that grows: the two systems need not fit together
         *M = DevCsr{};
     }
+    FIIM_TRY(arena.reserve(bytes));
     FIIM_TRY(carve_csr(arena, A, n, nA));
     FIIM_TRY(carve_csr(arena, G, n, nG));
     FIIM_TRY(carve_csr(arena, H, n, nH));
