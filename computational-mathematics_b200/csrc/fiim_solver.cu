@@ -890,6 +890,10 @@ int Solver::create(int n_, const int *Ai, const int *Aj, const double *Av, const
         release_dia(*M);                       // before that grows: the two systems need not fit together
         *M = DevCsr{};
     }
+    // An arena much larger than this system's goes back to the device; up to kArenaSlack more is kept, which
+    // spares calls over systems of about one size an allocation each.
+    constexpr size_t kArenaSlack = size_t(64) << 20;
+    if (arena.cap > bytes + kArenaSlack) arena.release();
     FIIM_TRY(arena.reserve(bytes));
     FIIM_TRY(carve_csr(arena, A, n, nA));
     FIIM_TRY(carve_csr(arena, G, n, nG));

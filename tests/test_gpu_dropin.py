@@ -127,3 +127,16 @@ def test_reloads_choose_the_form_a_fresh_solver_would(points):
             assert np.array_equal(x, y, equal_nan=True) and r[1] == r1["iter"], (step, kind)
     finally:
         FB.dropin_cache(prev)
+
+
+def test_a_smaller_system_gives_the_larger_ones_memory_back():
+    """After a large system, a small one leaves no more on the device than 64 MB beyond its own."""
+    import torch
+    small, large = system((12, 1)), system((72, 2))
+    free = []
+    for s in (small, large, small):
+        check([s])
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[1] > 100 << 20          # the large one's arena
+    assert free[0] - free[2] <= 68 << 20
