@@ -155,6 +155,7 @@ struct Stager {
     ~Stager() { release(); }
 };
 Stager &thread_stager(int device);
+void copy_parallel(void *to, const void *from, size_t len);   // memcpy by all host threads
 
 int upload_csr_async(DevCsr &M, long nnz_cap, int n, const int *rp, const int *ci, const double *v, bool device_src,
                      cudaStream_t s, Stager *stager = nullptr);

@@ -23,6 +23,9 @@
 #include <algorithm>
 #include <climits>
 #include <cstring>
+#include <memory>
+#include <new>
+#include <type_traits>
 #include <vector>
 
 #include "fiim_b200.h"
@@ -675,7 +678,7 @@ int launch_rows(int n, const int *rows, int nrows, const CsrD &A, const CsrD &At
 // One device allocation carved into pieces.
 struct Slab {
     char *p = nullptr;
-    size_t used = 0;
+    size_t used = 0, size = 0;
     Slab() = default;
     Slab(const Slab &) = delete;
     Slab &operator=(const Slab &) = delete;
@@ -683,11 +686,13 @@ struct Slab {
     void release() {
         if (p) cudaFree(p);
         p = nullptr;
-        used = 0;
+        used = size = 0;
     }
     int reserve(size_t bytes) {
         release();
+        size = bytes;
         if (cudaMalloc(&p, bytes) == cudaSuccess) return FIIM_OK;
+        size = 0;
         cudaGetLastError();
         p = nullptr;
         return set_error(FIIM_ENOMEM, "device allocation of %zu bytes for the factor construction failed", bytes);
@@ -704,18 +709,40 @@ struct Slab {
     }
 };
 
-// Factors built by the thread's last first call, on the device until the second call copies them
-// out (or another first call replaces them).
+// Factors built by the thread's last first call, until the second call copies them out (or another
+// first call replaces them, or the thread ends): on the device up to kHeldMost bytes, which a caller that
+// only asks for the sizes leaves there; larger ones in host memory, device = -1.
+constexpr size_t kHeldMost = size_t(512) << 20;
 struct BuiltGpu {
     int n = 0, device = -1;
     long nG = 0, nH = 0;
     Slab mem;
+    std::unique_ptr<char[]> host;
     int *Gi = nullptr, *Gj = nullptr, *Hi = nullptr, *Hj = nullptr;
     double *Gv = nullptr, *Hv = nullptr, *D = nullptr;
     void clear() {
         mem.release();
+        host.reset();
         n = 0;
     }
+    // The arrays' places in one piece of memory that starts at p; its size.
+    size_t carve(char *p, int rows) {
+        size_t used = 0;
+        auto take = [&](auto *&at, size_t count) {
+            using T = std::remove_reference_t<decltype(*at)>;
+            at = reinterpret_cast<T *>(p + used);
+            used += Slab::need<T>(count);
+        };
+        take(Gi, (size_t)rows + 1);
+        take(Hi, (size_t)rows + 1);
+        take(D, (size_t)rows);
+        take(Gj, (size_t)nG);
+        take(Gv, (size_t)nG);
+        take(Hj, (size_t)nH);
+        take(Hv, (size_t)nH);
+        return used;
+    }
+    int to_host(int dev);
 };
 thread_local BuiltGpu g_built_gpu;
 
@@ -835,27 +862,15 @@ int build_gpu(int n, const int *Ai, const int *Aj, const double *Av, const Param
         room = asked;
     }
     // H: the tasks' h lists one after another; G: the tasks' g lists, columns, turned into rows.
-    const size_t cap = (size_t)asked;   // entries of G and H together
-    if (cap > 2UL * 0x7fffffffUL) return set_error(FIIM_EARG, "factors too large for int32 CSR");
-    FIIM_TRY(out.mem.reserve(2 * Slab::need<int>(n + 1) + Slab::need<double>(n) + 2 * (Slab::need<int>(cap) + Slab::need<double>(cap))));
-    out.Gi = out.mem.take<int>(n + 1);
-    out.Hi = out.mem.take<int>(n + 1);
-    out.D = out.mem.take<double>(n);
-    long tot[2] = {0, 0};
-    FIIM_TRY(scan(n, hcnt, sums, out.Hi, nullptr, st));
-    FIIM_CUDA(cudaMemcpyAsync(&tot[1], sums + nb, sizeof(long), cudaMemcpyDeviceToHost, st));
+    if (asked > 2ULL * 0x7fffffffULL) return set_error(FIIM_EARG, "factors too large for int32 CSR");
+    FIIM_TRY(scan(n, hcnt, sums, dTi, nullptr, st));   // A^T is done with
+    FIIM_CUDA(cudaMemcpyAsync(&out.nH, sums + nb, sizeof(long), cudaMemcpyDeviceToHost, st));
     FIIM_CUDA(cudaStreamSynchronize(st));
-    tot[0] = (long)asked - tot[1];
-    if (tot[0] > 0x7fffffffL || tot[1] > 0x7fffffffL) {
-        out.clear();
-        return set_error(FIIM_EARG, "factors too large for int32 CSR");
-    }
-    out.nG = tot[0];
-    out.nH = tot[1];
-    out.Gj = out.mem.take<int>(out.nG);
-    out.Gv = out.mem.take<double>(out.nG);
-    out.Hj = out.mem.take<int>(out.nH);
-    out.Hv = out.mem.take<double>(out.nH);
+    out.nG = (long)asked - out.nH;
+    if (out.nG > 0x7fffffffL || out.nH > 0x7fffffffL) return set_error(FIIM_EARG, "factors too large for int32 CSR");
+    FIIM_TRY(out.mem.reserve(out.carve(nullptr, n)));
+    const size_t held = out.carve(out.mem.p, n);
+    FIIM_CUDA(cudaMemcpyAsync(out.Hi, dTi, sizeof(int) * (n + 1), cudaMemcpyDeviceToDevice, st));
     k_h_rows<<<grid_for(k_h_rows, kWarps, n), kThreads, 0, st>>>(n, o, out.Hi, out.Hj, out.Hv);
     FIIM_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * n, st));
     k_count_g<<<grid_for(k_count_g, kThreads, n), kThreads, 0, st>>>(n, o, cnt);
@@ -870,15 +885,21 @@ int build_gpu(int n, const int *Ai, const int *Aj, const double *Av, const Param
     FIIM_CUDA(cudaStreamSynchronize(st));
     out.n = n;
     out.device = dev;
+    return held > kHeldMost ? out.to_host(dev) : FIIM_OK;
+}
+
+int BuiltGpu::to_host(int dev) {
+    host.reset(new (std::nothrow) char[mem.size]);
+    if (!host) return set_error(FIIM_ENOMEM, "host allocation of %zu bytes for the factors failed", mem.size);
+    FIIM_TRY(thread_stager(dev).copy_out(host.get(), mem.p, mem.size));
+    carve(host.get(), n);
+    mem.release();
+    device = -1;
     return FIIM_OK;
 }
 
 // The second call: straight into the caller's arrays.
 int copy_out(const BuiltGpu &b, double *Gv, int *Gj, int *Gi, double *D, double *Hv, int *Hj, int *Hi) {
-    int was = -1;
-    FIIM_CUDA(cudaGetDevice(&was));
-    FIIM_CUDA(cudaSetDevice(b.device));
-    Stager &stager = thread_stager(b.device);
     const size_t n = (size_t)b.n, g = (size_t)b.nG, h = (size_t)b.nH;
     const struct {
         void *to;
@@ -887,7 +908,14 @@ int copy_out(const BuiltGpu &b, double *Gv, int *Gj, int *Gi, double *D, double 
     } parts[] = {{Gi, b.Gi, sizeof(int) * (n + 1)}, {Gj, b.Gj, sizeof(int) * g}, {Gv, b.Gv, sizeof(double) * g},
                  {Hi, b.Hi, sizeof(int) * (n + 1)}, {Hj, b.Hj, sizeof(int) * h}, {Hv, b.Hv, sizeof(double) * h},
                  {D, b.D, sizeof(double) * n}};
-    int rc = FIIM_OK;
+    if (b.device < 0) {
+        for (const auto &p : parts) copy_parallel(p.to, p.from, p.bytes);
+        return FIIM_OK;
+    }
+    int was = -1, rc = FIIM_OK;
+    FIIM_CUDA(cudaGetDevice(&was));
+    FIIM_CUDA(cudaSetDevice(b.device));
+    Stager &stager = thread_stager(b.device);
     for (const auto &p : parts)
         if (rc == FIIM_OK) rc = stager.copy_out(p.to, p.from, p.bytes);
     cudaSetDevice(was);

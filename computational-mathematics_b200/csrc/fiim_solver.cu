@@ -454,7 +454,7 @@ static bool pageable(const void *p) {
     return yes;
 }
 
-static void copy_parallel(void *to, const void *from, size_t len) {
+void copy_parallel(void *to, const void *from, size_t len) {
     const long parts = (long)((len + (size_t(1) << 19) - 1) >> 19);
 #pragma omp parallel for schedule(static)
     for (long q = 0; q < parts; ++q) {

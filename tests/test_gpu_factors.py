@@ -54,3 +54,31 @@ def test_many_rows_outgrow_both_smaller_capacities():
     """Five fill levels of the 7-point stencil reach up to 115 members: most of 21,952 rows are listed
     and built again at 64 and then at 128."""
     same(FB.gen_convdiff3d(28, 0.4), 0.02, 5, 1, 1)
+
+
+def test_large_factors_do_not_stay_on_the_device():
+    """Between the two calls: factors past 512 MB wait in host memory, smaller ones on the device, and the
+    second call copies either out as the host construction has them."""
+    import ctypes as C
+
+    import torch
+
+    def sizes_only(A):
+        ng, nh = C.c_int(0), C.c_int(0)
+        FB._check(FB.lib().fiim_pdfiim_build_gpu(
+            C.c_int(len(A[0]) - 1), FB._ptr(A[0]), FB._ptr(A[1]), FB._ptr(A[2]), C.c_int(1), C.c_int(1), C.c_int(1),
+            C.c_double(0.05), C.c_int(-1), C.c_char(b"I"), C.c_char(b"B"), C.byref(ng), C.byref(nh),
+            None, None, None, None, None, None, None))
+        return 12 * (ng.value + nh.value)
+
+    FB.pdfiim_build(FB.gen_poisson2d(40, 37), 0.05, 1, 1, 1, gpu=True)   # modules and pinned buffers
+    for side, large in ((64, False), (184, True)):
+        A = FB.gen_convdiff3d(side, 0.5)
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        held = sizes_only(A)
+        after = torch.cuda.mem_get_info()[0]
+        assert (held > 512 << 20) == large
+        assert before - after <= (4 << 20 if large else held + (32 << 20))
+        same(A, 0.05, 1, 1, 1)
+        assert before - torch.cuda.mem_get_info()[0] <= 4 << 20
