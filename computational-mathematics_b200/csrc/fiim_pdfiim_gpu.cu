@@ -688,13 +688,17 @@ struct Slab {
         p = nullptr;
         used = size = 0;
     }
-    int reserve(size_t bytes) {
+    bool fits(size_t bytes) {
         release();
         size = bytes;
-        if (cudaMalloc(&p, bytes) == cudaSuccess) return FIIM_OK;
+        if (cudaMalloc(&p, bytes) == cudaSuccess) return true;
         size = 0;
         cudaGetLastError();
         p = nullptr;
+        return false;
+    }
+    int reserve(size_t bytes) {
+        if (fits(bytes)) return FIIM_OK;
         return set_error(FIIM_ENOMEM, "device allocation of %zu bytes for the factor construction failed", bytes);
     }
     template <typename T>
@@ -743,6 +747,7 @@ struct BuiltGpu {
         return used;
     }
     int to_host(int dev);
+    int order_on_host(const Out &o, int rows, cudaStream_t st);
 };
 thread_local BuiltGpu g_built_gpu;
 
@@ -790,17 +795,26 @@ int build_gpu(int n, const int *Ai, const int *Aj, const double *Av, const Param
     Slab mem, entries;
     StreamGuard guard{st};   // after the slabs: synchronized before they go
     const int nb = (n + kScan - 1) / kScan;
-    FIIM_TRY(mem.reserve(2 * Slab::need<int>(n + 1) + 4 * Slab::need<int>(nnz) + 2 * Slab::need<double>(nnz) +
+    FIIM_TRY(mem.reserve(2 * Slab::need<int>(n + 1) + 2 * Slab::need<int>(nnz) + 2 * Slab::need<double>(nnz) +
                          7 * Slab::need<int>(n) + Slab::need<double>(n) + Slab::need<long>(n) + Slab::need<long>(nb + 1) +
                          3 * Slab::need<long>(1)));
-    int *dAi = mem.take<int>(n + 1), *dTi = mem.take<int>(n + 1), *dAj = mem.take<int>(nnz), *dTj = mem.take<int>(nnz),
-        *key = mem.take<int>(nnz), *row = mem.take<int>(nnz);
+    int *dAi = mem.take<int>(n + 1), *dTi = mem.take<int>(n + 1), *dAj = mem.take<int>(nnz), *dTj = mem.take<int>(nnz);
     double *dAv = mem.take<double>(nnz), *dTv = mem.take<double>(nnz), *dD = mem.take<double>(n);
     int *gcnt = mem.take<int>(n), *hcnt = mem.take<int>(n), *ovf = mem.take<int>(n), *rows2 = mem.take<int>(n),
         *cnt = mem.take<int>(n), *next = mem.take<int>(n), *longs = mem.take<int>(n);
     long *at = mem.take<long>(n), *sums = mem.take<long>(nb + 1);
     unsigned long long *used = mem.take<unsigned long long>(1);
     int *novf = mem.take<int>(1), *nlongs = mem.take<int>(1);
+    // Room for four entries per entry of A and row; a construction that keeps more is counted, given exactly
+    // what it needs, and run again. Where the device has not that much left, the first run only counts.
+    // A^T's lists are made in the same room.
+    auto entry_bytes = [](size_t count) { return Slab::need<int>(count) + Slab::need<double>(count); };
+    unsigned long long room = 4ULL * (unsigned long long)(nnz + n), asked = 0;
+    if (!entries.fits(entry_bytes(room))) {
+        room = (unsigned long long)nnz;
+        FIIM_TRY(entries.reserve(entry_bytes(room)));
+    }
+    int *key = entries.take<int>(nnz), *row = entries.take<int>(nnz);
     Stager &stager = thread_stager(dev);
     FIIM_TRY(stager.copy(dAi, Ai, sizeof(int) * (n + 1), st));
     if (nnz > 0) {
@@ -815,12 +829,10 @@ int build_gpu(int n, const int *Ai, const int *Aj, const double *Av, const Param
     FIIM_TRY(rank_lists(n, Lists{dTi, key, row, nullptr, dAv, dTj, dTv}, longs, nlongs, st));
     const CsrD A{dAi, dAj, dAv}, At{dTi, dTj, dTv};
     // Every row's entries and D^{-1}, in one pass: they go to the next free places, which are then
-    // put in order. Room for four entries per entry of A and row; a construction that keeps more is
-    // counted, given exactly what it needs, and run again.
+    // put in order.
     Out o{gcnt, hcnt, dD, at, nullptr, nullptr, used, 0, ovf, novf};
-    unsigned long long room = 4ULL * (unsigned long long)(nnz + n), asked = 0;
     for (;;) {
-        FIIM_TRY(entries.reserve(Slab::need<int>(room) + Slab::need<double>(room)));
+        entries.used = 0;
         o.ej = entries.take<int>(room);
         o.ev = entries.take<double>(room);
         o.room = room;
@@ -860,6 +872,7 @@ int build_gpu(int n, const int *Ai, const int *Aj, const double *Av, const Param
         FIIM_CUDA(cudaStreamSynchronize(st));
         if (asked <= room) break;
         room = asked;
+        FIIM_TRY(entries.reserve(entry_bytes(room)));
     }
     // H: the tasks' h lists one after another; G: the tasks' g lists, columns, turned into rows.
     if (asked > 2ULL * 0x7fffffffULL) return set_error(FIIM_EARG, "factors too large for int32 CSR");
@@ -868,15 +881,17 @@ int build_gpu(int n, const int *Ai, const int *Aj, const double *Av, const Param
     FIIM_CUDA(cudaStreamSynchronize(st));
     out.nG = (long)asked - out.nH;
     if (out.nG > 0x7fffffffL || out.nH > 0x7fffffffL) return set_error(FIIM_EARG, "factors too large for int32 CSR");
-    FIIM_TRY(out.mem.reserve(out.carve(nullptr, n)));
+    Slab lists;
+    if (!out.mem.fits(out.carve(nullptr, n)) || !lists.fits(Slab::need<int>(out.nG) + Slab::need<double>(out.nG))) {
+        out.mem.release();
+        return out.order_on_host(o, n, st);   // A, A^T and the entries are all the device has to hold
+    }
     const size_t held = out.carve(out.mem.p, n);
     FIIM_CUDA(cudaMemcpyAsync(out.Hi, dTi, sizeof(int) * (n + 1), cudaMemcpyDeviceToDevice, st));
     k_h_rows<<<grid_for(k_h_rows, kWarps, n), kThreads, 0, st>>>(n, o, out.Hi, out.Hj, out.Hv);
     FIIM_CUDA(cudaMemsetAsync(cnt, 0, sizeof(int) * n, st));
     k_count_g<<<grid_for(k_count_g, kThreads, n), kThreads, 0, st>>>(n, o, cnt);
     FIIM_TRY(scan(n, cnt, sums, out.Gi, next, st));
-    Slab lists;
-    FIIM_TRY(lists.reserve(Slab::need<int>(out.nG) + Slab::need<double>(out.nG)));
     int *gkey = lists.take<int>(out.nG);
     double *gval = lists.take<double>(out.nG);
     k_g_to_rows<<<grid_for(k_g_to_rows, kThreads, n), kThreads, 0, st>>>(n, o, next, gkey, gval);
@@ -894,6 +909,46 @@ int BuiltGpu::to_host(int dev) {
     FIIM_TRY(thread_stager(dev).copy_out(host.get(), mem.p, mem.size));
     carve(host.get(), n);
     mem.release();
+    device = -1;
+    return FIIM_OK;
+}
+
+// The tasks' lists put in order in host memory, by counting sorts; o's arrays are on the device, st is done.
+int BuiltGpu::order_on_host(const Out &o, int rows, cudaStream_t st) {
+    const size_t count = (size_t)(nG + nH);
+    std::unique_ptr<int[]> cg(new (std::nothrow) int[rows]), ch(new (std::nothrow) int[rows]), ej(new (std::nothrow) int[count]);
+    std::unique_ptr<long[]> at(new (std::nothrow) long[rows]);
+    std::unique_ptr<double[]> ev(new (std::nothrow) double[count]);
+    const size_t bytes = carve(nullptr, rows);
+    host.reset(new (std::nothrow) char[bytes]);
+    if (!cg || !ch || !ej || !at || !ev || !host)
+        return set_error(FIIM_ENOMEM, "host allocation of %zu bytes for the factors failed", bytes + 12 * count);
+    carve(host.get(), rows);
+    FIIM_CUDA(cudaMemcpyAsync(cg.get(), o.gcnt, sizeof(int) * rows, cudaMemcpyDeviceToHost, st));
+    FIIM_CUDA(cudaMemcpyAsync(ch.get(), o.hcnt, sizeof(int) * rows, cudaMemcpyDeviceToHost, st));
+    FIIM_CUDA(cudaMemcpyAsync(at.get(), o.at, sizeof(long) * rows, cudaMemcpyDeviceToHost, st));
+    FIIM_CUDA(cudaMemcpyAsync(ej.get(), o.ej, sizeof(int) * count, cudaMemcpyDeviceToHost, st));
+    FIIM_CUDA(cudaMemcpyAsync(ev.get(), o.ev, sizeof(double) * count, cudaMemcpyDeviceToHost, st));
+    FIIM_CUDA(cudaMemcpyAsync(D, o.D, sizeof(double) * rows, cudaMemcpyDeviceToHost, st));
+    FIIM_CUDA(cudaStreamSynchronize(st));
+    std::fill(Gi, Gi + rows + 1, 0);
+    Hi[0] = 0;
+    for (int i = 0; i < rows; ++i) {
+        for (long q = at[i]; q < at[i] + cg[i]; ++q) Gi[ej[q] + 1]++;
+        Hi[i + 1] = Hi[i] + ch[i];
+        std::copy_n(ej.get() + at[i] + cg[i], ch[i], Hj + Hi[i]);
+        std::copy_n(ev.get() + at[i] + cg[i], ch[i], Hv + Hi[i]);
+    }
+    for (int i = 0; i < rows; ++i) Gi[i + 1] += Gi[i];
+    for (int i = 0; i < rows; ++i)   // Gi[r]: row r's next place, until all are shifted back by one row
+        for (long q = at[i]; q < at[i] + cg[i]; ++q) {
+            const int place = Gi[ej[q]]++;
+            Gj[place] = i;
+            Gv[place] = ev[q];
+        }
+    for (int r = rows; r > 0; --r) Gi[r] = Gi[r - 1];
+    Gi[0] = 0;
+    n = rows;
     device = -1;
     return FIIM_OK;
 }

@@ -82,3 +82,28 @@ def test_large_factors_do_not_stay_on_the_device():
         assert before - after <= (4 << 20 if large else held + (32 << 20))
         same(A, 0.05, 1, 1, 1)
         assert before - torch.cuda.mem_get_info()[0] <= 4 << 20
+
+
+def test_little_device_memory():
+    """With the rest of the device taken: where only A, A^T and the entries fit, the first run counts, the
+    second fills and the host orders, to the same arrays; where those do not fit, an error."""
+    import torch
+    A = FB.gen_convdiff3d(72, 0.4)
+    n, nnz = 72 ** 3, len(A[1])
+    host = same(A, 0.05, 2, 2, 1)
+    entries = 12 * (len(host["Gj"]) + len(host["Hj"]))
+    matrices = 24 * nnz + 60 * n
+    assert 12 * 4 * (nnz + n) > entries + (16 << 20)     # the first room does not fit below
+    for keep in (matrices + entries + (16 << 20), matrices // 2):
+        torch.cuda.synchronize()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - keep, dtype=torch.uint8, device="cuda")
+        try:
+            if keep > matrices:
+                gpu = FB.pdfiim_build(A, 0.05, 2, 2, 1, gpu=True)
+                assert all(np.array_equal(host[k], gpu[k]) for k in host)
+            else:
+                with pytest.raises(FB.FiimError, match="allocation"):
+                    FB.pdfiim_build(A, 0.05, 2, 2, 1, gpu=True)
+        finally:
+            del hog
+            torch.cuda.empty_cache()
