@@ -1,6 +1,8 @@
 """The GPU factor construction's ordering on the device against the host construction, array for
 array: rows and columns with lists past one warp's, more entries than the first room, one row, and
 arrays large enough for the staged copies."""
+import time
+
 import numpy as np
 import pytest
 
@@ -107,3 +109,35 @@ def test_little_device_memory():
         finally:
             del hog
             torch.cuda.empty_cache()
+
+
+def band(n, dense_column):
+    """A band of four diagonals, with or without a first column that every row has."""
+    i = np.arange(n)
+    cols = np.stack([np.zeros(n, np.int64) if dense_column else i - 2, i - 1, i, i + 2], axis=1)
+    keep = np.stack([i > 1, i > 0, i >= 0, i + 2 < n], axis=1)
+    v = np.where(cols == i[:, None], 6.0, 0.4)
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+    return rp, cols[keep].astype(np.int32), v[keep]
+
+
+def test_a_list_of_many_thousand_entries():
+    """Keys of three bytes, sorted in as many passes."""
+    A = band(70001, True)
+    assert np.bincount(A[1])[0] == 70001 and len(A[1]) > 1 << 16
+    same(A, 0.001, 1, 1, 1)
+
+
+def test_a_dense_column_costs_what_its_entries_do():
+    """1.5 M rows: the ordering of one list with an entry a row is linear, so the construction takes no
+    more than a few times what the band takes without that column (comparing all pairs: 40 times)."""
+    times = {}
+    for dense in (False, True):
+        A = band(1_500_000, dense)
+        t = []
+        for _ in range(4):
+            t0 = time.perf_counter()
+            FB.pdfiim_build(A, 0.001, 1, 1, 1, gpu=True)
+            t.append(time.perf_counter() - t0)
+        times[dense] = min(t)
+    assert times[True] < 8 * times[False], times
