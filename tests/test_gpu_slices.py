@@ -254,3 +254,21 @@ def test_wide_stencils_with_and_without_sharing(monkeypatch, sides, points):
     r0 = np.linalg.norm(b - O.csr_mv(*A, np.full(n, 0.25)))
     assert np.linalg.norm(out[0][1] - out[1][1]) <= 2 * 1e-11 * r0 / 21 + 1e-13 * np.linalg.norm(out[0][1])
     assert out[2][0] == out[0][0] and np.array_equal(out[2][1], out[0][1])
+
+
+@pytest.mark.parametrize("kind", sorted(KINDS))
+@pytest.mark.parametrize("n", [1000, 4097])
+def test_banded_matrices_are_served_by_the_sliced_copy(monkeypatch, kind, n):
+    """Nine diagonals over full rows: form 3, with shared blocks (fewer bytes than the values) where every
+    row is alike and a block a slice where none are; the CSR streams only where they are asked for."""
+    A = banded(n, (-100, -33, -8, -1, 0, 1, 8, 32, 101), KINDS[kind])
+    with FB.Solver(A, identity_factors(n)) as S:
+        assert S.spmv_shape(0)[1] == 3
+        if kind != "layers":
+            assert (S.matrix_bytes(0) < 8 * len(A[1])) == (kind == "constant")
+    for env in ("FIIM_DIA_SHARE", "FIIM_DIA"):
+        monkeypatch.setenv(env, "0")
+        with FB.Solver(A, identity_factors(n)) as S:
+            assert S.spmv_shape(0)[1] == (3 if env == "FIIM_DIA_SHARE" else 0)
+            assert S.matrix_bytes(0) >= 8 * len(A[1])
+        monkeypatch.delenv(env)
