@@ -764,7 +764,7 @@ k_narrow_cols(const int *__restrict__ ci, const int *__restrict__ eb, int nblk, 
 // that agree in all of this share one record and block (SHARED: cls names a slice's record).
 // Bytes per entry: the value's width and the padding, plus 2 or 4 per R rows for the records,
 // against the width plus 2 or 4 per entry and 4 per row for the CSR streams; shared, 4 per
-// slice, and the blocks stay in L1.
+// slice, and the blocks, which stay in L1 or L2 (fiim_slices.cu).
 constexpr unsigned long long kDiaPad = 0xFFF7D1A6B00C5A1DULL;   // FP64 padding; FP32 and BF16 below
 constexpr unsigned kDiaPad32 = 0xFFD1A6B5u;
 constexpr unsigned short kDiaPad16 = 0xFFD1u;

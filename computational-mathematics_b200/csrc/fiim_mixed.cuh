@@ -214,8 +214,9 @@ k_inner_init(long n, const double *__restrict__ r64, const DState *sto, float *_
     grid_reduce<1>(red, partials, st, FinStart{});
 }
 
-// s = r - alpha v. With the norms moved to the x / r update and ||pc||^2 left to it, a solve of
-// 881,730 rows (FP32 factors, 104 iterations) went from 11.49 to 10.95 ms.
+// s = r - alpha v. The norms are taken by the x / r update, which writes their vectors, and ||pc||^2 is
+// added up there: this launch reads a third less. The solve gained too little to tell from one run to
+// another (881,730 rows, FP32 factors, 104 iterations: 11.49 to 10.95 ms, repeated 11.87 to 11.25).
 static __global__ void __launch_bounds__(kThreads)
 k_update_s_f(long n, const float *__restrict__ r, const float *__restrict__ v, float *__restrict__ s, DState *st) {
     pdl_enter();

@@ -1,8 +1,11 @@
 // Building and refreshing the sliced-diagonal copy of a matrix (fiim_kernels.cuh, k_spmv_dia)
 // on the device. The copy holds one record and one block of values per DIFFERENT slice: a
-// stencil with constant coefficients has a few dozen (128^3 convection-diffusion: A 27, G 58,
-// H 32 of 65,536 slices of 32 rows), and its products then read the vectors and little else,
-// since the blocks stay in L1. Slices count as the same when their diagonals, their values bit
+// stencil with constant coefficients has a few dozen where the grid's lines are whole or simple
+// fractions of slices (128^3 convection-diffusion: A 18, G 40, H 22 of 32,768 slices of 64 rows,
+// 0.07 to 0.12 MB of blocks, which stay in L1), and hundreds where they are not (97^3: 403, 638 and
+// 481 of 14,261, 1.7 to 2.7 MB, which come from L2). Its products then read the vectors and
+// little else: an iteration at 96, 97, 100, 127 and 128 a side takes 89, 95, 91, 78 and 74 ps a row,
+// against 131, 133, 133, 114 and 114 with a block a slice. Slices count as the same when their diagonals, their values bit
 // for bit (padding included) and their clamp flag agree; equality is found by a 64-bit hash
 // and then checked on every slice, so a hash collision costs the sharing, never a product.
 
