@@ -79,6 +79,7 @@ struct DevCsr {
     long ndiag = 0;              // diagonals over the blocks held (dsh slots each)
     int *drec = nullptr;         // dncls records
     int *dcls = nullptr;         // the record of each slice (null: its own)
+    int *dfirst = nullptr;       // the first slice of each record (with dcls)
     int2 *dpos = nullptr;        // first row and rows of each slice (several segments only)
     char *dstat = nullptr;       // device counters of the check (fiim_slices.cuh, Stats)
     void *dvals = nullptr;       // dsh * ndiag values of dvbytes bytes each (FP64, FP32 or BF16)

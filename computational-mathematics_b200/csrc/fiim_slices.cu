@@ -51,7 +51,7 @@ void release_dia(DevCsr &M) {
     M.dia_pad = false;
     M.dia_mem = nullptr;
     M.dia_bytes = 0;
-    M.drec = M.dcls = nullptr;
+    M.drec = M.dcls = M.dfirst = nullptr;
     M.dpos = nullptr;
     M.dstat = nullptr;
     M.dvals = nullptr;
@@ -315,9 +315,9 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
         const int ncls = share ? st.uniq : nsl;
         const long ndiag = share ? (long)st.uniq_ndiag : (long)st.ndiag;
         const size_t b_rec = Arena::need(sizeof(int) * (size_t)rs * ncls),
-                     b_cls = share ? Arena::need(sizeof(int) * nsl) : 0,
+                     b_cls = share ? Arena::need(sizeof(int) * nsl) : 0, b_first = share ? Arena::need(sizeof(int) * ncls) : 0,
                      b_pos = segmented ? Arena::need(sizeof(int2) * nsl) : 0, b_st = Arena::need(sizeof(sl::Stats)),
-                     b_v = Arena::need((size_t)vbytes * sh * ndiag), all = b_rec + b_cls + b_pos + b_st + b_v;
+                     b_v = Arena::need((size_t)vbytes * sh * ndiag), all = b_rec + b_cls + b_pos + b_st + b_v + b_first;
         char *mem = nullptr;
         if (cudaMalloc(&mem, all) != cudaSuccess) {
             cudaGetLastError();
@@ -330,6 +330,7 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
         M.dpos = segmented ? reinterpret_cast<int2 *>(mem + b_rec + b_cls) : nullptr;
         M.dstat = mem + b_rec + b_cls + b_pos;
         M.dvals = mem + b_rec + b_cls + b_pos + b_st;
+        M.dfirst = share ? reinterpret_cast<int *>(mem + b_rec + b_cls + b_pos + b_st + b_v) : nullptr;
         M.dvbytes = vbytes;
         M.dsh = sh;
         M.nsl = nsl;
@@ -344,7 +345,7 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
         sl::k_offsets<<<1, 1024, 0, s>>>(nsl, m, share ? rep : nullptr, id, k0);
         FIIM_CUDA(cudaGetLastError());
         if (share) {
-            sl::k_classes<<<grid_for(sl::k_classes, kThreads, nsl), kThreads, 0, s>>>(nsl, rep, id, M.dcls);
+            sl::k_classes<<<grid_for(sl::k_classes, kThreads, nsl), kThreads, 0, s>>>(nsl, rep, id, M.dcls, M.dfirst);
             FIIM_CUDA(cudaGetLastError());
         }
         sl::Args a = copy_args(M, vals);
@@ -363,14 +364,18 @@ int build_dia(DevCsr &M, cudaStream_t s, int vbytes, const void *vals, const std
     return FIIM_OK;
 }
 
-// Enqueues the check that the copy still holds M's matrix with the values `vals`, and, for a
-// copy whose slices have their own blocks, the new values; stats.bad tells afterwards whether
-// it does (a copy with shared blocks holds only the very same values) and build_dia would choose
-// this form for them: where shared blocks fit the columns, the different slices are counted again,
-// which reads the matrix once for each number of rows a lane that fits. ok = false: not enqueued,
-// the form has to be chosen anew.
+// Enqueues the new values `vals` of M's matrix into the copy, and the check that it then holds them;
+// stats.bad tells afterwards whether it does and build_dia would choose this form for them. Shared
+// blocks take the values of their first slices, and every slice is checked against its block (slices
+// that were alike and are alike still share; laying the copy out again for new constant coefficients
+// made a drop-in call at 110^3 with five iterations 13.8 ms, this way it takes 10.0). For slices with
+// their own blocks whose columns would allow shared ones, the different slices are counted again, which
+// reads the matrix once for each number of rows a lane that fits. ok = false: not enqueued, the form
+// has to be chosen anew.
 static int enqueue_refresh(DevCsr &M, const void *vals, cudaStream_t s, bool *ok) {
-    const bool recount = !M.dcls && M.dia_fit && M.dvbytes == 8 && !M.dseg && share_wanted();
+    // which numbers of rows a lane, sharing, would be chosen before what the copy is now
+    const int better = M.dia_fit & (!M.dcls ? 3 : M.dsh == 32 ? 2 : 0);
+    const bool recount = better && M.dvbytes == 8 && !M.dseg && share_wanted();
     const int nsl[2] = {(int)((M.n + 31) / 32), (int)((M.n + 63) / 64)};
     unsigned table = 64;
     while (table < 2U * (unsigned)nsl[0]) table <<= 1;
@@ -384,9 +389,17 @@ static int enqueue_refresh(DevCsr &M, const void *vals, cudaStream_t s, bool *ok
     if (!*ok) return FIIM_OK;
     sl::Args a = copy_args(M, vals);
     FIIM_CUDA(cudaMemsetAsync(M.dstat, 0, sizeof(sl::Stats), s));
-    if (M.pack) FIIM_CUDA(pack(true, a, M.khdr, M.krec, s));
-    else if (M.dcls) FIIM_CUDA((walk<sl::kVerify, true>(M.dsh / 32, M.dvbytes, a, s)));
-    else FIIM_CUDA((walk<sl::kPlace, false>(M.dsh / 32, M.dvbytes, a, s)));
+    if (M.pack) {
+        FIIM_CUDA(pack(true, a, M.khdr, M.krec, s));
+    } else if (M.dcls) {
+        sl::Args first = a;
+        first.nsl = M.dncls;
+        first.list = M.dfirst;
+        FIIM_CUDA((walk<sl::kPlace, true>(M.dsh / 32, M.dvbytes, first, s)));
+        FIIM_CUDA((walk<sl::kVerify, true>(M.dsh / 32, M.dvbytes, a, s)));
+    } else {
+        FIIM_CUDA((walk<sl::kPlace, false>(M.dsh / 32, M.dvbytes, a, s)));
+    }
     if (!recount) return FIIM_OK;
     FIIM_CUDA(cudaMemsetAsync(M.dscan, 0, b_st + 2 * b_keys, s));
     char *mem = static_cast<char *>(M.dscan);
@@ -395,13 +408,13 @@ static int enqueue_refresh(DevCsr &M, const void *vals, cudaStream_t s, bool *ok
     a.mask = table - 1;
     a.cls = nullptr;
     for (int R = 1; R <= 2; ++R) {
-        if (!(M.dia_fit & R)) continue;
+        if (!(better & R)) continue;
         a.nsl = nsl[R - 1];
         a.stats = count + (R - 1);
         a.keys = reinterpret_cast<unsigned long long *>(mem + b_st + (R - 1) * b_keys);
         FIIM_CUDA((walk<sl::kCount, true>(R, 8, a, s)));
     }
-    sl::k_recheck<<<1, 1, 0, s>>>(make_int2(M.dia_fit & 1 ? nsl[0] : 0, M.dia_fit & 2 ? nsl[1] : 0), count,
+    sl::k_recheck<<<1, 1, 0, s>>>(make_int2(better & 1 ? nsl[0] : 0, better & 2 ? nsl[1] : 0), count,
                                   reinterpret_cast<sl::Stats *>(M.dstat));
     FIIM_CUDA(cudaGetLastError());
     return FIIM_OK;

@@ -52,6 +52,7 @@ struct Args {
     const int *cls;                  // class of each slice (null: its own index)
     const int *k0;                   // first diagonal of each class's block (write)
     const int *rep;                  // the class's first slice (write; null: every slice writes)
+    const int *list;                 // place: the slices to walk, nsl of them (null: all)
 };
 
 enum { kScan, kCount, kWrite, kVerify, kPlace };   // count: a scan that leaves only the different slices' number
@@ -91,7 +92,8 @@ static __global__ void __launch_bounds__(kThreads) k_walk(Args a) {
     B *dv = static_cast<B *>(a.dv);
     unsigned long long sum_m = 0;
     int max_m = 0;
-    for (int s = (int)blockIdx.x * kWarps + ((int)threadIdx.x >> 5); s < a.nsl; s += (int)gridDim.x * kWarps) {
+    for (int at = (int)blockIdx.x * kWarps + ((int)threadIdx.x >> 5); at < a.nsl; at += (int)gridDim.x * kWarps) {
+        const int s = MODE == kPlace && a.list ? __ldg(a.list + at) : at;
         // refused already: random matrices end at once (one lane's read, so the warp agrees)
         if (SCAN && __shfl_sync(full, *(volatile int *)&a.stats->refused, 0)) break;
         const int c = a.cls ? __ldg(a.cls + s) : s;
@@ -360,9 +362,13 @@ k_offsets(int nsl, const int *__restrict__ m, const int *__restrict__ rep, int *
     }
 }
 
+// The class of each slice, and each class's first slice.
 static __global__ void __launch_bounds__(kThreads)
-k_classes(int nsl, const int *__restrict__ rep, const int *__restrict__ id, int *__restrict__ cls) {
-    FIIM_FOR_ROWS(s, nsl) { cls[s] = id[rep[s]]; }
+k_classes(int nsl, const int *__restrict__ rep, const int *__restrict__ id, int *__restrict__ cls, int *__restrict__ first) {
+    FIIM_FOR_ROWS(s, nsl) {
+        cls[s] = id[rep[s]];
+        if (rep[s] == (int)s) first[id[s]] = (int)s;
+    }
 }
 
 }  // namespace sl

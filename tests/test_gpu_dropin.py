@@ -140,3 +140,33 @@ def test_a_smaller_system_gives_the_larger_ones_memory_back():
         free.append(torch.cuda.mem_get_info()[0])
     assert free[0] - free[1] > 100 << 20          # the large one's arena
     assert free[0] - free[2] <= 68 << 20
+
+
+@pytest.mark.parametrize("points", [7, 27])
+def test_reloads_into_shared_blocks(points):
+    """Constant and layered entries, scaled, split into more kinds of slices and merged again: shared blocks
+    take new values where the slices that share them stay alike, and are laid out again where not; x is a
+    fresh solver's bit for bit."""
+    from test_gpu_slices import stencil
+    from test_gpu_solve import identity_factors
+    A0 = stencil((41, 37, 33), points, "constant")
+    n = len(A0[0]) - 1
+    rows = np.repeat(np.arange(n), np.diff(A0[0]))
+    layer = lambda k: 1.0 + (rows // (n // k + 1)) % 2   # noqa: E731
+    values = [A0[2], A0[2] * 1.25, A0[2] * layer(5), A0[2] * layer(5) * 0.75, A0[2], A0[2] * layer(9),
+              A0[2] * np.where(rows == 20011, 1.5, 1.0), A0[2] * 1.5]
+    F, b = identity_factors(n), FB.rand_normal(n, 12)
+    prev = FB.dropin_cache(False)
+    try:
+        for step, v in enumerate(values):
+            A = (A0[0], A0[1], v)
+            with FB.Solver(A, F, variant="pdfiim") as S:
+                y = np.full(n, 0.25)
+                r1 = S.solve(b, y, tol=1e-9, nmax=100)
+                assert S.spmv_shape(0)[1] == 3 and S.matrix_bytes(0) < 8 * len(v)
+            x = np.full(n, 0.25)
+            r = FB.EPBiCGSTAB_pdfiim(A, b, 1e-9, 100, (F["Gi"], F["Gj"], F["Gv"]), F["IDv"],
+                                     (F["Hi"], F["Hj"], F["Hv"]), x)
+            assert r1["info"] == 0 and np.array_equal(x, y) and r[1] == r1["iter"], step
+    finally:
+        FB.dropin_cache(prev)
