@@ -62,26 +62,37 @@ struct BlockSolver {
     cudaGraphExec_t exec = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
 
+    bool deal[3] = {};               // A, G, H: rows dealt out to the warps (set_chunks)
+
     bk::Shape shape() const { return bk::Shape{n, k}; }
 
     template <int L, int VW, typename V, typename Epi>
-    cudaError_t spmm_lv(const DevCsr &M, const V *vals, const double *X, const Epi &epi) {
-        auto go = [&](auto kern) {
-            kern<<<grid_for(kern, kWarps, M.nblk), kThreads, 0, stream>>>(CsrView<V>{M.rp, M.ci, vals, n}, shape(), M.rb,
-                                                                          M.nblk, X, epi, bs, partials);
+    cudaError_t spmm_lv(int which, const DevCsr &M, const V *vals, const double *X, const Epi &epi) {
+        auto go = [&](auto kern, const int *chunk, int nch) {
+            kern<<<grid_for(kern, kWarps, nch), kThreads, 0, stream>>>(CsrView<V>{M.rp, M.ci, vals, n}, shape(), chunk, nch,
+                                                                       X, epi, bs, partials);
             return cudaGetLastError();
         };
         if constexpr (L == 32 && VW == 1)
-            if (bk::streams(M.nnz)) return go(bk::k_spmm_stream<V, Epi>);
-        return go(bk::k_spmm<L, VW, V, Epi>);
+            if (bk::streams(M.nnz)) return go(bk::k_spmm_stream<V, Epi>, M.rb, M.nblk);
+        constexpr int step = 32 / L;
+        if (deal[which]) return go(bk::k_spmm<L, VW, V, Epi, true>, nullptr, (n + step - 1) / step);
+        return go(bk::k_spmm<L, VW, V, Epi, false>, M.rb, M.nblk);
     }
 
-    // Chunks of consecutive rows of about equal work (M.rb, M.nblk of them), whole steps of a warp
-    // (32 / kp rows) each, one for every warp that the product's kernel keeps on the chip. A step
-    // costs what its longest row does: its entries, and two more for the row's own reads and writes
-    // (4 and 8 more measured 2 and 7% slower). Every chunk ends at the step nearest its share.
-    int set_chunks(DevCsr &M) {
+    // How M's rows reach the warps: dealt out one step of a warp (32 / kp rows) after another, or chunks of
+    // consecutive rows of about equal work (M.rb, M.nblk of them), one for every warp that the product's
+    // kernel keeps on the chip. A step costs what its longest row does: its entries, and two more for the
+    // row's own reads and writes (4 and 8 more measured 2 and 7% slower). Every chunk ends at the step
+    // nearest its share. Rows are dealt out where no warp then gets more than kUneven times the mean:
+    // warps that run together read neighbouring rows of X, and eight CTAs an SM hide more latency. Chunks
+    // against dealt rows (us): stencils of 7 points, at most 1.45 times the mean, 64^3 with 16 right-hand
+    // sides A X 95 against 89, 100^3 365 against 276 and M X 754 against 481; factors of power-law
+    // matrices, 1.1 to 2.3 times, 800,003 rows with 8 M X 237 against 202; power-law rows, 3.2 times and
+    // more, 200,003 rows with 8 A X 137 against 236, 800,003 with 16 532 against 807.
+    int set_chunks(DevCsr &M, bool &dealt) {
         constexpr long kRowCost = 2;
+        constexpr double kUneven = 2.5;
         const long warps = (long)(kp == 32 ? 4 : 6) * kWarps * num_sms();   // k_spmm_stream, k_spmm
         const int step = 32 / kp;
         auto cost = [&](int i) {
@@ -89,9 +100,16 @@ struct BlockSolver {
             for (int e = std::min(n, i + step); i < e; ++i) len = std::max(len, M.hrp[i + 1] - M.hrp[i]);
             return len + kRowCost;
         };
+        const long steps = (n + step - 1) / step;
+        std::vector<long> share(std::min<long>(steps, 8L * kWarps * num_sms()), 0);
         long total = 0, sum = 0;
-        for (int i = 0; i < n; i += step) total += cost(i);
-        const long nch = std::min<long>((n + step - 1) / step, warps);
+        for (long q = 0; q < steps; ++q) {
+            const long w = cost((int)(q * step));
+            share[q % share.size()] += w;
+            total += w;
+        }
+        dealt = (double)*std::max_element(share.begin(), share.end()) * (double)share.size() <= kUneven * (double)total;
+        const long nch = std::min<long>(steps, warps);
         std::vector<int> rb(1, 0);
         for (int i = 0; i < n; i += step) {
             const long w = cost(i), at = (long)rb.size() * total / nch;   // where the open one should end
@@ -111,16 +129,16 @@ struct BlockSolver {
     cudaError_t spmm(int which, const DevCsr &M, const V *vals, const double *X, const Epi &epi) {
         const SpmmShape s = shp[which];
         switch (s.per_lane * 64 + s.lanes) {
-            case 64 + 4: return spmm_lv<4, 1>(M, vals, X, epi);
-            case 64 + 8: return spmm_lv<8, 1>(M, vals, X, epi);
-            case 64 + 16: return spmm_lv<16, 1>(M, vals, X, epi);
-            case 64 + 32: return spmm_lv<32, 1>(M, vals, X, epi);
-            case 128 + 4: return spmm_lv<4, 2>(M, vals, X, epi);
-            case 128 + 8: return spmm_lv<8, 2>(M, vals, X, epi);
-            case 128 + 16: return spmm_lv<16, 2>(M, vals, X, epi);
-            case 256 + 2: return spmm_lv<2, 4>(M, vals, X, epi);
-            case 256 + 4: return spmm_lv<4, 4>(M, vals, X, epi);
-            case 256 + 8: return spmm_lv<8, 4>(M, vals, X, epi);
+            case 64 + 4: return spmm_lv<4, 1>(which, M, vals, X, epi);
+            case 64 + 8: return spmm_lv<8, 1>(which, M, vals, X, epi);
+            case 64 + 16: return spmm_lv<16, 1>(which, M, vals, X, epi);
+            case 64 + 32: return spmm_lv<32, 1>(which, M, vals, X, epi);
+            case 128 + 4: return spmm_lv<4, 2>(which, M, vals, X, epi);
+            case 128 + 8: return spmm_lv<8, 2>(which, M, vals, X, epi);
+            case 128 + 16: return spmm_lv<16, 2>(which, M, vals, X, epi);
+            case 256 + 2: return spmm_lv<2, 4>(which, M, vals, X, epi);
+            case 256 + 4: return spmm_lv<4, 4>(which, M, vals, X, epi);
+            case 256 + 8: return spmm_lv<8, 4>(which, M, vals, X, epi);
             default: return cudaErrorInvalidValue;
         }
     }
@@ -293,7 +311,8 @@ struct BlockSolver {
         std::vector<int> mmv(32, mm);
         FIIM_CUDA(cudaMemcpyAsync(bs.maxmsteps, mmv.data(), sizeof(int) * 32, cudaMemcpyHostToDevice, stream));
         FIIM_CUDA(cudaStreamSynchronize(stream));
-        for (DevCsr *M : {&A, &G, &H}) FIIM_TRY(set_chunks(*M));
+        DevCsr *const mats[] = {&A, &G, &H};
+        for (int q = 0; q < 3; ++q) FIIM_TRY(set_chunks(*mats[q], deal[q]));
         FIIM_TRY(choose_shapes());
         return build_graph();
     }

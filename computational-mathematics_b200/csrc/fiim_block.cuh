@@ -238,7 +238,8 @@ __device__ __forceinline__ double wide(float v) { return (double)v; }
 // as the chip holds of the one-value-a-lane kernels (4 CTAs an SM below, 6 in k_spmm), so that each
 // warp has one run of consecutive rows and all end together. Rows dealt one by one left the warps
 // with the long rows of a power-law matrix running on alone, and two or four chunks a warp were
-// 5 to 40% slower than one.
+// 5 to 40% slower than one. k_spmm with DEAL takes matrices of even rows: a chunk is one step of the
+// warp, and they are dealt out in order.
 #define FIIM_CHUNKS(ch)                                                                       \
     for (int ch = (int)(((long)blockIdx.x * kThreads + threadIdx.x) >> 5); ch < nch;          \
          ch += (int)(((long)gridDim.x * kThreads) >> 5))
@@ -259,8 +260,8 @@ __device__ __forceinline__ void gather(const double *__restrict__ p, double (&x)
     }
 }
 
-template <int L, int VW, typename V, typename Epi>
-static __global__ void __launch_bounds__(kThreads, VW == 1 ? 6 : 1)
+template <int L, int VW, typename V, typename Epi, bool DEAL>
+static __global__ void __launch_bounds__(kThreads, VW == 1 ? (DEAL ? 8 : 6) : 1)
 k_spmm(CsrView<V> M, Shape sh, const int *__restrict__ chunk, int nch, const double *__restrict__ X, Epi epi, BState bs,
        double *__restrict__ partials) {
     if (Epi::GATED && bs.g->active <= 0) return;
@@ -271,7 +272,8 @@ k_spmm(CsrView<V> M, Shape sh, const int *__restrict__ chunk, int nch, const dou
         for (int q = 0; q < Epi::NR; ++q) red[u][q] = 0.0;
     const int lane_ = threadIdx.x & 31, j_ = lane_ % L, grp_ = lane_ / L;
     FIIM_CHUNKS(ch)
-    for (long base = __ldg(chunk + ch), last_ = __ldg(chunk + ch + 1); base < last_; base += 32 / L) {
+    for (long base = DEAL ? ch * (32L / L) : __ldg(chunk + ch),
+              last_ = DEAL ? min(base + 32 / L, (long)M.n) : __ldg(chunk + ch + 1); base < last_; base += 32 / L) {
         const long row = base + grp_;
         const bool live = row < last_;
         const int j0 = j_ * VW;            // this lane's first right-hand side

@@ -58,3 +58,26 @@ def test_block_reductions_cover_every_row(n, k):
         rel = np.linalg.norm(b - O.csr_mv(rp, ci, v, np.ascontiguousarray(X[:, j]))) / np.linalg.norm(b)
         assert res["info"][j] == 0 and rel < 1e-5
         assert abs(res["true_relres"][j] - rel) <= 1e-9 * rel + 1e-15
+
+
+@pytest.mark.parametrize("shape", [None, "8,4", "16,2"])
+@pytest.mark.parametrize("n,k", [(1, 4), (33, 1), (900, 16), (6011, 4), (6011, 9), (6012, 16), (70001, 3), (6011, 32)])
+def test_rows_dealt_out_to_the_warps(monkeypatch, shape, n, k):
+    """Matrices of even rows (one step of a warp after another, the last one partly filled) beside an
+    uneven one (chunks): the same products, in every shape that serves k."""
+    if shape:
+        if k % int(shape.split(",")[1]):
+            pytest.skip("the shape's vector width does not divide k")
+        monkeypatch.setenv("FIIM_BLOCK_SHAPE", shape)
+    r = np.random.default_rng(n + k)
+    even = np.full(n, 7)
+    A, G, H = rows_of(even, n, 1), rows_of(even, n, 2), rows_of(LENGTHS["uneven"](n, r), n, 3)
+    F = {"Gi": G[0], "Gj": G[1], "Gv": G[2], "IDv": r.standard_normal(n), "Hi": H[0], "Hj": H[1], "Hv": H[2]}
+    X = r.standard_normal((n, k))
+    for precision in ("fp64", "fp32"):
+        S = FB.BlockSolver(A, F, k, precision=precision)
+        Fr = rounded(F, precision)
+        for op, ref in (("A", lambda u: O.csr_mv(*A, u)), ("M", lambda u: O.prec_apply(Fr, u))):
+            want = np.stack([ref(np.ascontiguousarray(X[:, j])) for j in range(k)], axis=1)
+            assert np.array_equal(S.apply(X, np.full((n, k), 7.0), op=op), want), (precision, op)
+        S.close()
